@@ -71,7 +71,16 @@ struct SolverParams {
   // AVBD_CONTACT_MATERIALS (the WebGPU engine's contact extensions) when 1
   int contactModel;
   double restitutionThreshold, contactPersistence;
+  // f32 copies for the solve (a conversion there runs on the FP64 pipe)
+  float dtF, dt2F, alphaF, betaLinF, penaltyMaxF, stickThresholdF;
 };
+
+// A parameter in the solve's scalar: the f32 copy or the f64 value.
+template <class T>
+__host__ __device__ inline T pick(double d, float f) {
+  if constexpr (sizeof(T) == 4) return f;
+  else return d;
+}
 
 // Device scalars shared by all kernels of a step.
 struct Control {
@@ -80,7 +89,7 @@ struct Control {
   unsigned barrierGen;
   int numCandidates;
   int numColors;
-  int colorChanged;
+  unsigned solveArrivals;  // arrivals at the solve's grid barrier this step
   int liveManifolds;
   int liveContacts;
   int fp64Bodies;

@@ -988,7 +988,9 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
                      P.neighbor_wait_limit > 0 ? (long long)P.neighbor_wait_limit
                                                : (P.wait_limit > 0 ? (long long)P.wait_limit : 4000000LL),
                      P.tail_div, P.contact_model == AVBD_CONTACT_MATERIALS ? 1 : 0,
-                     P.restitution_threshold, P.contact_persistence};
+                     P.restitution_threshold, P.contact_persistence,
+                     (float)P.dt, (float)(P.dt * P.dt), (float)P.alpha, (float)P.beta_lin, (float)P.penalty_max,
+                     (float)P.stick_threshold};
   int rc = 0;
   D4 *sizeP, *massDP;
   float4 *massFP;

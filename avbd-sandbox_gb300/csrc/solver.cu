@@ -77,6 +77,40 @@ __device__ bool grid_barrier(Control *ctl, long long limit) {
   return ok != 0;
 }
 
+// The solve's grid barrier: arrivals of the step are counted in one word
+// (zeroed with the step's counters), and phase k of `blocks` blocks is over
+// when it reaches k * blocks. Waiters poll the word the arrivals go to, and
+// the timeout flag in the same round trip: the generation word of
+// grid_barrier, its second fence and its closing flag read are three more
+// memory round trips a phase (3,800 cycles a barrier of one busy block with
+// grid_barrier, 2,200 with this). Gives up as grid_barrier does.
+__device__ __forceinline__ bool solve_barrier(Control *ctl, unsigned target, long long limit) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->solveArrivals) : "memory");
+    int good = 1;
+    long long spins = 0;
+    for (;;) {
+      const unsigned f = *((volatile unsigned *)&ctl->flags);  // in flight together with the count
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->solveArrivals) : "memory");
+      if (f & kOvfTimeout) good = 0;
+      if ((int)(v - target) >= 0 || !good) break;
+      if (++spins > limit) {
+        atomicOr(&ctl->flags, kOvfTimeout);
+        good = 0;
+        break;
+      }
+      __nanosleep(20);
+    }
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
 // ---------------------------------------------------------------------------
 // Preparation
 // ---------------------------------------------------------------------------
@@ -753,6 +787,36 @@ __device__ __forceinline__ void group_reduce(Sys<T> &s, unsigned mask, int G) {
   }
 }
 
+// The same butterfly for a whole warp of groups of at most 16 lanes (maxG the
+// largest), every lane taking part: with a mask per group the groups of a
+// warp run this one after the other (in f64, 50 bodies of a hanging chain:
+// 51,000 cycles an update, the solve 8.9 ms; this form 4.7 ms; in f32, a
+// pile of 200 boxes, 0.34 ms and 0.30). Groups narrower than a level's
+// distance sit that level out.
+template <class T>
+__device__ __forceinline__ void warp_reduce(Sys<T> &s, int G, int maxG) {
+  __syncwarp();
+  auto level = [&](int m, bool on) {
+    auto add = [&](T &v) {
+      const T o = __shfl_xor_sync(0xffffffffu, v, m);
+      v = on ? v + o : v;
+    };
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      add(s.l[k]);
+      add(s.a[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++) add(s.c[k]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      add(s.bl[k]);
+      add(s.ba[k]);
+    }
+  };
+  for (int m = maxG >> 1; m > 0; m >>= 1) level(m, m < G);
+}
+
 // For groups of 32 lanes: the same sums by reduce-scatter (xor distances 16,
 // 8, 4, 2, 1, the butterfly's own pairing, so every total is bitwise the
 // butterfly's) and an all-gather: 31 + 27 shuffles instead of 5 x 27.
@@ -1108,7 +1172,8 @@ template <class T>
 __device__ __forceinline__ void contact_dual(const World &w, const ContactData<T> &d, const BState<T> &self, T alpha) {
   const BState<T> &A = d.side ? d.o : self;
   const BState<T> &B = d.side ? self : d.o;
-  const T beta = (T)w.p.betaLin, kmax = (T)w.p.penaltyMax, thr = (T)w.p.stickThreshold;
+  const T beta = pick<T>(w.p.betaLin, w.p.betaLinF), kmax = pick<T>(w.p.penaltyMax, w.p.penaltyMaxF);
+  const T thr = pick<T>(w.p.stickThreshold, w.p.stickThresholdF);
   const ContactEval<T> e = eval_contact(d.n, d.mu, d.cA, d.cB, d.cK, d.cL, A, B, alpha, d.x);
   float4 cK = d.cK;
   float stick = d.cL.w;
@@ -1510,7 +1575,7 @@ __device__ __noinline__ void extra_dual(const World &w, int i, int cb, int nm, i
 template <class T>
 __device__ __forceinline__ void inertial_core(const SolverParams &P, T m, T I0, T I1, T I2, float4 y, float4 qy,
                                               const BState<T> &self, bool selfSphere, Sys<T> &s) {
-  const T dt2 = (T)(P.dt * P.dt);
+  const T dt2 = pick<T>(P.dt * P.dt, P.dt2F);
   const T ml = m / dt2;
   s.l[0] = ml; s.l[2] = ml; s.l[5] = ml;
   const V3<T> dy = self.dp - V3<T>{(T)y.x, (T)y.y, (T)y.z};
@@ -1562,20 +1627,24 @@ __device__ inline void st_release(int *p, int v) {
 // Reduce the group's partial systems, solve the 6x6 system (maths.js:660-725),
 // integrate (maths.js:568-592) and publish the new iterate; on the last main
 // iteration also the BDF1 velocity (solver.js:476-488).
+// maxG > 0: the whole warp is here, its widest group of maxG lanes (an idle
+// lane: G = 1, lane = 1); 0: this group alone.
 // publish: lane 0 releases *publish = pubValue once the body's new state is
 // stored (what a later body of the tail segment reads of it), before the
 // velocity and the dual updates.
 template <class T>
 __device__ __forceinline__ void finish_body(const World &w, int i, int lane, int G, unsigned mask, bool velocity,
-                                            float4 qt, Sys<T> &s, BState<T> &self, int *publish = nullptr,
+                                            float4 qt, Sys<T> &s, BState<T> &self, int maxG, int *publish = nullptr,
                                             int pubValue = 0) {
-  const T dt = (T)w.p.dt;
+  const T dt = pick<T>(w.p.dt, w.p.dtF);
   if constexpr (sizeof(T) == 4) {
     if (G == 32) group_reduce32(s);
     else if (G > 32) group_reduce_warps(s, G);
+    else if (maxG) warp_reduce(s, G, maxG);
     else group_reduce(s, mask, G);
   } else {
-    group_reduce(s, mask, G);
+    if (maxG) warp_reduce(s, G, maxG);
+    else group_reduce(s, mask, G);
   }
   V3<T> xl, xa;
   ldlt_solve(s, -s.bl[0], -s.bl[1], -s.bl[2], -s.ba[0], -s.ba[1], -s.ba[2], xl, xa);
@@ -1609,12 +1678,13 @@ __device__ __forceinline__ void finish_body(const World &w, int i, int lane, int
 // constraints it owns, and on the last main iteration its BDF1 velocity.
 // Register form: the FP64 path.
 template <class T, bool E>
-__device__ void solve_body(const World &w, int4 rec, int lane, int G, unsigned mask, T alpha, bool dual, bool velocity) {
+__device__ void solve_body(const World &w, int4 rec, int lane, int G, unsigned mask, T alpha, bool dual, bool velocity,
+                           int maxG, bool act) {
   const int i = rec.x, cb = rec.y, nm = rec.z - rec.y;
   // one round of loads: own state, constraint ranges and this lane's first contact
   BState<T> self = load_state<T>(w, i);
   const int cStart = ld(&w.g.cStart[i]), cEnd = ld(&w.g.cStart[i + 1]);
-  const int total = nm + (cEnd - cStart);
+  const int total = act ? nm + (cEnd - cStart) : 0;
   const bool selfSphere = (ld(&w.b.flags0[i]) & kBodySphere) != 0;
   const bool has0 = lane < nm;
   ContactData<T> d0;
@@ -1626,7 +1696,7 @@ __device__ void solve_body(const World &w, int4 rec, int lane, int G, unsigned m
   if (has0) contact_primal<T>(d0, self, alpha, s);
   if (extra) extra_primal<T, E>(w, i, cb, nm, cStart, total, lane, G, self, alpha, s);
   if (lane == 0 && ld(&w.grab->body) == i) s = grab_primal<T>(w, i, self, s);
-  finish_body<T>(w, i, lane, G, mask, velocity, ld(&w.b.quatT[i]), s, self);
+  finish_body<T>(w, i, lane, G, mask, velocity, ld(&w.b.quatT[i]), s, self, maxG);
   if (!dual) return;
   // dual updates of the constraints this body owns (it has the larger colour)
   if (has0 && d0.owned) contact_dual<T>(w, d0, self, alpha);
@@ -1798,10 +1868,12 @@ __device__ __noinline__ void tail_wait_extra(const World &w, int nm, int cStart,
   }
 }
 
-// `tw`: the tail waits of this body (null outside the tail segment).
+// `tw`: the tail waits of this body (null outside the tail segment). maxG:
+// see finish_body; `act` is false on the idle lanes of a whole warp.
 template <bool E>
 __device__ void solve_body_staged(const World &w, int4 rec, int lane, int G, unsigned mask, float alpha, bool dual,
-                                  bool velocity, float4 *stage, const TailWait *tw = nullptr) {
+                                  bool velocity, float4 *stage, const TailWait *tw = nullptr, int maxG = 0,
+                                  bool act = true) {
   using T = float;
   const int i = rec.x, cb = rec.y, nm = rec.z - rec.y;
   const int nk = lane < nm ? (nm - lane + G - 1) / G : 0;  // this lane's contacts
@@ -1821,7 +1893,7 @@ __device__ void solve_body_staged(const World &w, int4 rec, int lane, int G, uns
   self.dp = V3<T>{d0.x, d0.y, d0.z};
   self.q = Q4<T>{q0.x, q0.y, q0.z, q0.w};
   self.dang = qsub(self.q, Q4<T>{qt.x, qt.y, qt.z, qt.w});
-  const int total = nm + (cEnd - cStart);
+  const int total = act ? nm + (cEnd - cStart) : 0;
   Sys<T> s;
   zero(s);
   if (lane == 0) inertial_core<T>(w.p, mf.x, mf.y, mf.z, mf.w, y, qy, self, sphere, s);
@@ -1842,7 +1914,8 @@ __device__ void solve_body_staged(const World &w, int4 rec, int lane, int G, uns
   // in the tail segment the body's progress is published as soon as its state is stored: the
   // bodies waiting for it (higher colours) own every constraint they share with it, so they
   // read nothing its dual updates write
-  finish_body<T>(w, i, lane, G, mask, velocity, qt, s, self, tw ? &w.b.progress[i] : nullptr, tw ? tw->need : 0);
+  finish_body<T>(w, i, lane, G, mask, velocity, qt, s, self, maxG, tw ? &w.b.progress[i] : nullptr,
+                 tw ? tw->need : 0);
   if (!dual) return;
   if (nk <= kStageSlots) {
     // every contact of this lane is still staged; the owner alone writes a
@@ -1868,8 +1941,8 @@ __device__ void solve_body_staged(const World &w, int4 rec, int lane, int G, uns
 // instead of lowering the occupancy of the FP32 path.
 template <bool E>
 __device__ __noinline__ void solve_body_f64(const World &w, int4 rec, int lane, int G, unsigned mask, double alpha,
-                                            bool dual, bool velocity) {
-  solve_body<double, E>(w, rec, lane, G, mask, alpha, dual, velocity);
+                                            bool dual, bool velocity, int maxG = 0, bool act = true) {
+  solve_body<double, E>(w, rec, lane, G, mask, alpha, dual, velocity, maxG, act);
 }
 
 // The neighbours come from the body's manifold list (one entry per touching
@@ -1950,6 +2023,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
   const int numColors = *((volatile int *)&ctl->numColors);
   const int warpLane = threadIdx.x & 31;
   const int total = P.iterations + (P.postStabilize ? 1 : 0);
+  unsigned arrivals = 0;  // of all active blocks at the next barrier's end
   const int kb = P.solveBlocksPerSm > 0 ? P.solveBlocksPerSm : 1, S = gridDim.x / kb;
   const int jb = S * kb == (int)gridDim.x ? ((int)blockIdx.x % kb) * S + (int)blockIdx.x / kb : (int)blockIdx.x;
   // colour chunk bounds, constant through the solve: the first kChunkCache + 1
@@ -1967,23 +2041,41 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
     const int tailDiv = P.tailDiv > 0 ? P.tailDiv : kTailDiv;
     while (tail > 0 && chunkAt(tail) - chunkAt(tail - 1) <= (int)gridDim.x / tailDiv) tail--;
   }
+  // the blocks that any phase gives work; the others leave, so that a small
+  // scene's barriers wait for few
+  int active = tail < numColors ? (int)gridDim.x : 1;
+  for (int c = 0; c < tail && active < (int)gridDim.x; c++)
+    active = min((int)gridDim.x, max(active, chunkAt(c + 1) - chunkAt(c)));
+  if (jb >= active) return;
   for (int it = 0; it < total; it++) {
     const double alpha = P.postStabilize ? (it < P.iterations ? 1.0 : 0.0) : P.alpha;
+    const float alphaF = P.postStabilize ? (it < P.iterations ? 1.f : 0.f) : P.alphaF;
     const bool dual = it < P.iterations;
     const bool vel = it == P.iterations - 1;
     for (int c = 0; c < tail; c++) {
       const int q0 = chunkAt(c), q1 = chunkAt(c + 1);
-      for (int q = q0 + jb; q < q1; q += gridDim.x) {
+      for (int q = q0 + jb; q < q1; q += active) {
+        // whole warps: a lane past the colour's last group, or of a body of
+        // the other precision, goes along idle
         const int e = ld(&w.a.laneTab[(size_t)q * kLaneMaxGroup + threadIdx.x]);
-        if (e < 0) continue;
-        const int G = 1 << (e & 7);
-        const int lane = threadIdx.x & (G - 1);
-        const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << G) - 1u) << (warpLane & ~(G - 1)));
-        const int4 rec = ld(&w.a.colorRec[e >> 4]);
-        if (e & 8) solve_body_f64<E>(w, rec, lane, G, mask, alpha, dual, vel);
-        else solve_body_staged<E>(w, rec, lane, G, mask, (float)alpha, dual, vel, stage);
+        const int4 rec0 = e >= 0 ? ld(&w.a.colorRec[e >> 4]) : make_int4(0, 0, 0, 0);
+        const bool f32 = e >= 0 && !(e & 8), f64 = e >= 0 && (e & 8);
+        const unsigned any32 = __ballot_sync(0xffffffffu, f32), any64 = __ballot_sync(0xffffffffu, f64);
+        if (any32) {
+          const int G = f32 ? 1 << (e & 7) : 1;
+          const int maxG = __shfl_sync(0xffffffffu, G, __ffs(any32) - 1);  // groups come in decreasing size
+          solve_body_staged<E>(w, f32 ? rec0 : make_int4(0, 0, 0, 0), f32 ? threadIdx.x & (G - 1) : 1, G, 0u, alphaF,
+                               dual, vel, stage, nullptr, maxG, f32);
+        }
+        if (any64) {
+          const int G = f64 ? 1 << (e & 7) : 1;
+          const int maxG = __shfl_sync(0xffffffffu, G, __ffs(any64) - 1);
+          solve_body_f64<E>(w, f64 ? rec0 : make_int4(0, 0, 0, 0), f64 ? warpLane & (G - 1) : 1, G, 0u, alpha, dual,
+                            vel, maxG, f64);
+        }
       }
-      if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+      arrivals += active;
+      if (!solve_barrier(ctl, arrivals, w.p.barrierLimit)) return;
     }
     if (tail < numColors) {  // the tail segment of iteration it
       int c = tail;
@@ -2007,10 +2099,11 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
           if (lane == 0) st_release(&w.b.progress[rec.x], it + 1);
         } else {
           const TailWait tw{tail, c, it + 1};  // publishes the body's progress itself
-          solve_body_staged<E>(w, rec, lane, G, mask, (float)alpha, dual, vel, stage, &tw);
+          solve_body_staged<E>(w, rec, lane, G, mask, alphaF, dual, vel, stage, &tw);
         }
       }
-      if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+      arrivals += active;
+      if (!solve_barrier(ctl, arrivals, w.p.barrierLimit)) return;
     }
   }
 }
