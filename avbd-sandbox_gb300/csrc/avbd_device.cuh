@@ -71,6 +71,7 @@ struct SolverParams {
   // AVBD_CONTACT_MATERIALS (the WebGPU engine's contact extensions) when 1
   int contactModel;
   double restitutionThreshold, contactPersistence;
+  int mayFp64;   // a body may be an FP64 body (adj_sort_kernel's test, bounded at pack)
   // f32 copies for the solve (a conversion there runs on the FP64 pipe)
   float dtF, dt2F, alphaF, betaLinF, penaltyMaxF, stickThresholdF;
 };

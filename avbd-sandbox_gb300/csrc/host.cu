@@ -980,6 +980,27 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   World &w = ctx->w;
   w = World{};
   const avbd_params &P = ctx->params;
+  // whether a body's stiffest joint or spring can ever make it an FP64 body:
+  // the penalties adj_sort_kernel compares stay below the stiffness and the
+  // cap (a hard joint counts as the cap); 1e-6 covers their f32 rounding
+  bool mayFp64 = false;
+  if (P.fp64_ratio_threshold > 0) {
+    auto stiff = [&](double k, int i) {
+      if (i >= 0 && B.mass[i] > 0 &&
+          !(k * (1.0 + 1e-6) <= P.fp64_ratio_threshold * (B.mass[i] / (P.dt * P.dt))))
+        mayFp64 = true;
+    };
+    for (int j = 0; j < ctx->nj; j++) {
+      // a penalty below the floor is raised to it before the stiffness caps it
+      const double k = std::isinf(J.stiffness_lin[j]) ? std::max(P.penalty_max, P.penalty_min) : J.stiffness_lin[j];
+      stiff(k, J.body_a[j]);
+      stiff(k, J.body_b[j]);
+    }
+    for (int s = 0; s < ctx->ns; s++) {
+      stiff(SP.stiffness[s], SP.body_a[s]);
+      stiff(SP.stiffness[s], SP.body_b[s]);
+    }
+  }
   w.p = SolverParams{P.dt, P.gravity, P.iterations, P.post_stabilize, P.beta_lin, P.beta_ang, P.alpha, P.gamma,
                      P.penalty_min, P.penalty_max, P.collision_margin, P.stick_threshold, P.rotated_inertia,
                      P.spring_stiffness_ramp, P.spring_geometric_stiffness, P.cached_contact_jacobians,
@@ -988,7 +1009,7 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
                      P.neighbor_wait_limit > 0 ? (long long)P.neighbor_wait_limit
                                                : (P.wait_limit > 0 ? (long long)P.wait_limit : 4000000LL),
                      P.tail_div, P.contact_model == AVBD_CONTACT_MATERIALS ? 1 : 0,
-                     P.restitution_threshold, P.contact_persistence,
+                     P.restitution_threshold, P.contact_persistence, mayFp64 ? 1 : 0,
                      (float)P.dt, (float)(P.dt * P.dt), (float)P.alpha, (float)P.beta_lin, (float)P.penalty_max,
                      (float)P.stick_threshold};
   int rc = 0;

@@ -2013,7 +2013,7 @@ __device__ __forceinline__ void group_sync(int G, unsigned mask) {
 constexpr int kTailDiv = 8;  // default of SolverParams::tailDiv
 constexpr int kTailMinColors = 16;  // automatic: steps of fewer colours have no tail segment
 constexpr int kChunkCache = 64;  // colours whose chunk bounds the solve keeps in shared memory
-template <bool E>
+template <bool E, bool F64>
 __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
   if (step_skipped(w)) return;
   extern __shared__ float4 stageSm[];
@@ -2067,7 +2067,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
           solve_body_staged<E>(w, f32 ? rec0 : make_int4(0, 0, 0, 0), f32 ? threadIdx.x & (G - 1) : 1, G, 0u, alphaF,
                                dual, vel, stage, nullptr, maxG, f32);
         }
-        if (any64) {
+        if (F64 && any64) {
           const int G = f64 ? 1 << (e & 7) : 1;
           const int maxG = __shfl_sync(0xffffffffu, G, __ffs(any64) - 1);
           solve_body_f64<E>(w, f64 ? rec0 : make_int4(0, 0, 0, 0), f64 ? warpLane & (G - 1) : 1, G, 0u, alpha, dual,
@@ -2088,7 +2088,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
         const int lane = threadIdx.x & (G - 1);
         const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << G) - 1u) << (warpLane & ~(G - 1)));
         const int4 rec = ld(&w.a.colorRec[e >> 4]);
-        if (e & 8) {
+        if (F64 && (e & 8)) {
           // a wait that gave up has set the timeout flag: the body is not
           // solved on stale data, and the kernel ends at the next grid barrier
           if (wait_neighbors(w, rec.x, it, lane, G, mask, tail)) {
@@ -2120,7 +2120,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
 
 
 
-template <bool E>
+template <bool E, bool F64>
 __global__ void __launch_bounds__(kSolveBlock, 3) wave_kernel(World w, int G) {
   if (step_skipped(w)) return;
   extern __shared__ float4 stageSm[];
@@ -2147,7 +2147,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) wave_kernel(World w, int G) {
         const int i = rec.x;
         if (!wait_neighbors(w, i, it, lane, G, mask)) return;
         __syncwarp(mask);  // orders every lane's reads after the acquires of the others
-        if (ld(&w.b.flags[i]) & kBodyFp64) solve_body_f64<E>(w, rec, lane, G, mask, alpha, dual, vel);
+        if (F64 && (ld(&w.b.flags[i]) & kBodyFp64)) solve_body_f64<E>(w, rec, lane, G, mask, alpha, dual, vel);
         else solve_body_staged<E>(w, rec, lane, G, mask, (float)alpha, dual, vel, stage);
         // the warp barrier orders every lane's writes before lane 0's release,
         // which makes them visible at gpu scope to whoever acquires the flag
@@ -2319,15 +2319,30 @@ cudaError_t launch_joint_anchor(const World &w, int joint, double x, double y, d
   return cudaGetLastError();
 }
 
+// The solve's instantiations: the contact extensions
+// (AVBD_CONTACT_MATERIALS) and the FP64 bodies each in kernels of their own,
+// so that the others carry none of their registers. The FP64 path's calls
+// cost the kernel a 1.4 KB stack frame and 260 bytes of spills, which every
+// grid barrier's acquire throws out of L1; without it there are none (148 registers;
+// solve of piles of 200 / 8,192 bodies 0.30 -> 0.27 / 0.60 -> 0.55 ms, the
+// crushed 36-layer pyramid 4.96 -> 4.58).
+static const void *solve_instance(bool wave, bool ext, bool fp64) {
+  if (wave) {
+    if (ext) return fp64 ? (const void *)wave_kernel<true, true> : (const void *)wave_kernel<true, false>;
+    return fp64 ? (const void *)wave_kernel<false, true> : (const void *)wave_kernel<false, false>;
+  }
+  if (ext) return fp64 ? (const void *)solve_kernel<true, true> : (const void *)solve_kernel<true, false>;
+  return fp64 ? (const void *)solve_kernel<false, true> : (const void *)solve_kernel<false, false>;
+}
+
 int solve_max_blocks_per_sm(int lanesPerBody) {
   (void)lanesPerBody;
-  const void *kernels[4] = {(const void *)solve_kernel<false>, (const void *)wave_kernel<false>,
-                            (const void *)solve_kernel<true>, (const void *)wave_kernel<true>};
   int best = 1 << 30;
-  for (const void *k : kernels) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem);
+  for (int k = 0; k < 8; k++) {
+    const void *f = solve_instance(k & 1, k & 2, k & 4);
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem);
     int a = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k, kSolveBlock, kSolveSmem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f, kSolveBlock, kSolveSmem);
     best = a < best ? a : best;
   }
   return best;
@@ -2340,14 +2355,10 @@ cudaError_t launch_solve(const World &w, int lanesPerBody, int blocksPerSm, cuda
   int G = lanesPerBody;
   void *args2[] = {&arg, &G};
   void *args1[] = {&arg};
-  // the contact extensions (AVBD_CONTACT_MATERIALS) are a separate
-  // instantiation, so the default kernels carry none of their registers
-  const bool ext = w.p.contactModel != 0;
-  if (w.p.schedule == 1)
-    return cudaLaunchCooperativeKernel(ext ? (const void *)wave_kernel<true> : (const void *)wave_kernel<false>,
-                                       dim3(blocksPerSm * smCount), dim3(kSolveBlock), args2, kSolveSmem, st);
-  return cudaLaunchCooperativeKernel(ext ? (const void *)solve_kernel<true> : (const void *)solve_kernel<false>,
-                                     dim3(blocksPerSm * smCount), dim3(kSolveBlock), args1, kSolveSmem, st);
+  const bool wave = w.p.schedule == 1;
+  return cudaLaunchCooperativeKernel(solve_instance(wave, w.p.contactModel != 0, w.p.mayFp64 != 0),
+                                     dim3(blocksPerSm * smCount), dim3(kSolveBlock), wave ? args2 : args1, kSolveSmem,
+                                     st);
 }
 
 void launch_commit(const World &w, cudaStream_t st, int smCount) { commit_kernel<<<smCount * 4, 256, 0, st>>>(w); }
