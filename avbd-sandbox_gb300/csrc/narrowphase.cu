@@ -435,6 +435,65 @@ __device__ void write_manifold_materials(const World &w, int c, int ia, int ib, 
                                          const D3 *ncA, const D3 *ncB, const uint32_t *feat, int num,
                                          const double *basis);
 
+// Contact i of a box pair's manifold: matched with the previous step's by
+// feature ID, C*(x_t) + margin, warm start.
+__device__ __forceinline__ void write_box_contact(const World &w, int c, int i, int pi, int oldNum, const BodyD &A,
+                                                  const BodyD &B, const NewContactF &nc, const float *bf) {
+  const SolverParams &P = w.p;
+  const Q4<float> qa{(float)A.q.x, (float)A.q.y, (float)A.q.z, (float)A.q.w};
+  const Q4<float> qb{(float)B.q.x, (float)B.q.y, (float)B.q.z, (float)B.q.w};
+  const V3<float> dAB{(float)(B.p.x - A.p.x), (float)(B.p.y - A.p.y), (float)(B.p.z - A.p.z)};
+  const float alpha = (float)P.alpha, gamma = (float)P.gamma;
+  const float kmin = (float)P.penaltyMin, kmax = (float)P.penaltyMax, margin = (float)P.margin;
+  V3<float> rA{nc.ra[0], nc.ra[1], nc.ra[2]};
+  V3<float> rB{nc.rb[0], nc.rb[1], nc.rb[2]};
+  float lam[3] = {0.f, 0.f, 0.f}, pen[3] = {0.f, 0.f, 0.f};
+  bool stick = false;
+  for (int j = 0; j < oldNum; j++) {
+    const int os = pi * kMaxContacts + j;
+    if (nc.feature == w.prev.feat[os]) {
+      const float4 ok = w.prev.cK[os], ol = w.prev.cL[os];
+      lam[0] = ol.x; lam[1] = ol.y; lam[2] = ol.z;
+      pen[0] = ok.x; pen[1] = ok.y; pen[2] = ok.z;
+      stick = ol.w != 0.0f;
+      if (stick) {  // a stuck box contact keeps its anchors (manifold.js:279-282)
+        const float4 oa = w.prev.rA[os], ob = w.prev.rB[os];
+        rA = V3<float>{oa.x, oa.y, oa.z};
+        rB = V3<float>{ob.x, ob.y, ob.z};
+      }
+      break;
+    }
+  }
+  const V3<float> rAw = qrotate(qa, rA), rBw = qrotate(qb, rB);
+  const V3<float> dd{rAw.x - rBw.x - dAB.x, rAw.y - rBw.y - dAB.y, rAw.z - rBw.z - dAB.z};
+  float C0[3];
+  for (int k = 0; k < 3; k++) C0[k] = bf[3 * k] * dd.x + bf[3 * k + 1] * dd.y + bf[3 * k + 2] * dd.z;
+  C0[0] += margin;
+  if (!P.postStabilize)
+    for (int k = 0; k < 3; k++) lam[k] = (lam[k] * alpha) * gamma;
+  for (int k = 0; k < 3; k++) {
+    const float x = pen[k] * gamma;  // clamp(gamma k, kmin, kmax), NaN propagating
+    pen[k] = x != x ? x : fmaxf(kmin, fminf(kmax, x));
+  }
+  const int s = c * kMaxContacts + i;
+  w.cur.feat[s] = nc.feature;
+  w.cur.rA[s] = make_float4(rA.x, rA.y, rA.z, 0.f);
+  w.cur.rB[s] = make_float4(rB.x, rB.y, rB.z, 0.f);
+  w.cur.cA[s] = make_float4(rAw.x, rAw.y, rAw.z, C0[0]);
+  w.cur.cB[s] = make_float4(rBw.x, rBw.y, rBw.z, C0[1]);
+  w.cur.cK[s] = make_float4(pen[0], pen[1], pen[2], C0[2]);
+  w.cur.cL[s] = make_float4(lam[0], lam[1], lam[2], stick ? 1.f : 0.f);
+}
+
+__device__ __forceinline__ void write_box_header(const World &w, int c, int ia, int ib, const double *basis,
+                                                 const float *bf) {
+  const double friction = sqrt(w.b.friction[ia] * w.b.friction[ib]);
+  for (int k = 0; k < 9; k++) w.cur.basisD[c * 9 + k] = basis[k];
+  w.cur.basis0[c] = make_float4(bf[0], bf[1], bf[2], (float)friction);
+  w.cur.basis1[c] = make_float4(bf[3], bf[4], bf[5], 0.f);
+  w.cur.basis2[c] = make_float4(bf[6], bf[7], bf[8], 0.f);
+}
+
 __device__ void write_box_manifold(const World &w, int c, int ia, int ib, const BodyD &A, const BodyD &B,
                                    const NewContactF *nc, int num, const double *basis) {
   const SolverParams &P = w.p;
@@ -453,58 +512,10 @@ __device__ void write_box_manifold(const World &w, int c, int ia, int ib, const 
   if (num == 0) return;
   const int pi = w.g.candPrev[c];
   const int oldNum = pi >= 0 ? w.prev.count[pi] : 0;
-  const Q4<float> qa{(float)A.q.x, (float)A.q.y, (float)A.q.z, (float)A.q.w};
-  const Q4<float> qb{(float)B.q.x, (float)B.q.y, (float)B.q.z, (float)B.q.w};
-  const V3<float> dAB{(float)(B.p.x - A.p.x), (float)(B.p.y - A.p.y), (float)(B.p.z - A.p.z)};
   float bf[9];
   for (int k = 0; k < 9; k++) bf[k] = (float)basis[k];
-  const float alpha = (float)P.alpha, gamma = (float)P.gamma;
-  const float kmin = (float)P.penaltyMin, kmax = (float)P.penaltyMax, margin = (float)P.margin;
-  for (int i = 0; i < num; i++) {
-    V3<float> rA{nc[i].ra[0], nc[i].ra[1], nc[i].ra[2]};
-    V3<float> rB{nc[i].rb[0], nc[i].rb[1], nc[i].rb[2]};
-    float lam[3] = {0.f, 0.f, 0.f}, pen[3] = {0.f, 0.f, 0.f};
-    bool stick = false;
-    for (int j = 0; j < oldNum; j++) {
-      const int os = pi * kMaxContacts + j;
-      if (nc[i].feature == w.prev.feat[os]) {
-        const float4 ok = w.prev.cK[os], ol = w.prev.cL[os];
-        lam[0] = ol.x; lam[1] = ol.y; lam[2] = ol.z;
-        pen[0] = ok.x; pen[1] = ok.y; pen[2] = ok.z;
-        stick = ol.w != 0.0f;
-        if (stick) {  // a stuck box contact keeps its anchors (manifold.js:279-282)
-          const float4 oa = w.prev.rA[os], ob = w.prev.rB[os];
-          rA = V3<float>{oa.x, oa.y, oa.z};
-          rB = V3<float>{ob.x, ob.y, ob.z};
-        }
-        break;
-      }
-    }
-    const V3<float> rAw = qrotate(qa, rA), rBw = qrotate(qb, rB);
-    const V3<float> dd{rAw.x - rBw.x - dAB.x, rAw.y - rBw.y - dAB.y, rAw.z - rBw.z - dAB.z};
-    float C0[3];
-    for (int k = 0; k < 3; k++) C0[k] = bf[3 * k] * dd.x + bf[3 * k + 1] * dd.y + bf[3 * k + 2] * dd.z;
-    C0[0] += margin;
-    if (!P.postStabilize)
-      for (int k = 0; k < 3; k++) lam[k] = (lam[k] * alpha) * gamma;
-    for (int k = 0; k < 3; k++) {
-      const float x = pen[k] * gamma;  // clamp(gamma k, kmin, kmax), NaN propagating
-      pen[k] = x != x ? x : fmaxf(kmin, fminf(kmax, x));
-    }
-    const int s = c * kMaxContacts + i;
-    w.cur.feat[s] = nc[i].feature;
-    w.cur.rA[s] = make_float4(rA.x, rA.y, rA.z, 0.f);
-    w.cur.rB[s] = make_float4(rB.x, rB.y, rB.z, 0.f);
-    w.cur.cA[s] = make_float4(rAw.x, rAw.y, rAw.z, C0[0]);
-    w.cur.cB[s] = make_float4(rBw.x, rBw.y, rBw.z, C0[1]);
-    w.cur.cK[s] = make_float4(pen[0], pen[1], pen[2], C0[2]);
-    w.cur.cL[s] = make_float4(lam[0], lam[1], lam[2], stick ? 1.f : 0.f);
-  }
-  const double friction = sqrt(w.b.friction[ia] * w.b.friction[ib]);
-  for (int k = 0; k < 9; k++) w.cur.basisD[c * 9 + k] = basis[k];
-  w.cur.basis0[c] = make_float4(bf[0], bf[1], bf[2], (float)friction);
-  w.cur.basis1[c] = make_float4(bf[3], bf[4], bf[5], 0.f);
-  w.cur.basis2[c] = make_float4(bf[6], bf[7], bf[8], 0.f);
+  for (int i = 0; i < num; i++) write_box_contact(w, c, i, pi, oldNum, A, B, nc[i], bf);
+  write_box_header(w, c, ia, ib, basis, bf);
 }
 
 // Pairs with a sphere, in f64: the basis-compatibility test and the
@@ -862,30 +873,291 @@ __global__ void __launch_bounds__(128) edge_kernel(World w) {
   }
 }
 
-// 4. Sphere pairs and undecided box pairs: the whole f64 collider.
-__global__ void __launch_bounds__(128) exact_kernel(World w) {
+// ---------------------------------------------------------------------------
+// The exact collider of a box pair on sixteen lanes (collide.js:612-685): an
+// SAT axis a lane, then a polygon vertex a lane. An FP64 warp instruction
+// costs the same for one lane as for 32, and a pair decided by one thread is
+// a chain of some 2,500 of them (150-230 us for a list of ten pairs); here it
+// is about 500 (the list of a 200-box pile: 150 -> 39 us; the narrow phase of
+// a ten-cube stack 233 -> 82 us, of the standing 53-layer pyramid 338 -> 205). Every value is formed by ColliderT's operations in their
+// order, so the contacts are bitwise the serial collider's. Both halves of a
+// warp run in step; `act` is false for a half without a box pair.
+// ---------------------------------------------------------------------------
+constexpr int kGroup = 16;
+
+__device__ __forceinline__ double gshfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src, kGroup); }
+__device__ __forceinline__ D3 gshfl(D3 v, int src) {
+  return D3{gshfl(v.x, src), gshfl(v.y, src), gshfl(v.z, src)};
+}
+__device__ __forceinline__ D3 pick3(bool c, D3 a, D3 b) { return D3{c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z}; }
+
+// The lane of the group with the largest v among those with `on`, the first
+// on ties (-1: none). Compared as integers: a double compare is an FP64 warp
+// instruction. (v + 0 makes -0 equal to +0.)
+__device__ __forceinline__ int group_argmax(double v, bool on) {
+  long long key = __double_as_longlong(v + 0.0);
+  key ^= (key >> 63) & 0x7fffffffffffffffLL;
+  int at = on ? (int)(threadIdx.x & (kGroup - 1)) : kGroup;
+#pragma unroll
+  for (int m = kGroup / 2; m > 0; m >>= 1) {
+    const long long ok = __shfl_xor_sync(0xffffffffu, key, m, kGroup);
+    const int oa = __shfl_xor_sync(0xffffffffu, at, m, kGroup);
+    const bool take = oa < kGroup && (at >= kGroup || ok > key || (ok == key && oa < at));
+    key = take ? ok : key;
+    at = take ? oa : at;
+  }
+  return at < kGroup ? at : -1;
+}
+
+// Returns the contact count; a lane with slot >= 0 holds contact `slot` in nc.
+__device__ int collide_group(const BodyD &A, const BodyD &B, double cd, bool act, D3 *poly, double *basis,
+                             NewContactF &nc, int &slot) {
+  const int gl = threadIdx.x & (kGroup - 1);
+  const unsigned shift = threadIdx.x & (32 - kGroup);
+  auto ballot = [&](bool p) { return (__ballot_sync(0xffffffffu, p) >> shift) & 0xffffu; };
+  slot = -1;
+  // box axes: lanes 0-2 A's, 3-5 B's
+  const bool ofA = gl < 3;
+  const QD q{ofA ? A.q.x : B.q.x, ofA ? A.q.y : B.q.y, ofA ? A.q.z : B.q.z, ofA ? A.q.w : B.q.w};
+  const int ak = ofA ? gl : gl - 3;
+  const D3 mine = rot(q, mk(ak == 0 ? 1.0 : 0.0, ak == 1 ? 1.0 : 0.0, ak == 2 ? 1.0 : 0.0));
+  OBB a, b;
+  a.c = A.p; a.h = A.half;
+  b.c = B.p; b.h = B.half;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    a.ax[i] = gshfl(mine, i);
+    b.ax[i] = gshfl(mine, 3 + i);
+  }
+  const D3 delta = sub(b.c, a.c);
+  // testAxis (collide.js:291-324) of axis gl: faces of A, of B, then the edge pairs
+  const int ek = gl < 6 ? 0 : min(gl - 6, 8);
+  const D3 axis = pick3(gl < 6, mine, crs(gshfl(mine, ek / 3), gshfl(mine, 3 + ek % 3)));
+  const double lenSq = axis.x * axis.x + axis.y * axis.y + axis.z * axis.z;
+  const bool tested = gl < 15 && !(lenSq < geo::kSatEps);
+  const double invLen = 1.0 / sqrt(lenSq);
+  D3 n = scl(axis, invLen);
+  if (dt3(n, delta) < 0) n = neg(n);
+  const double distance = fabs(dt3(delta, n));
+  const double rA = a.h.x * fabs(dt3(n, a.ax[0])) + a.h.y * fabs(dt3(n, a.ax[1])) + a.h.z * fabs(dt3(n, a.ax[2]));
+  const double rB = b.h.x * fabs(dt3(n, b.ax[0])) + b.h.y * fabs(dt3(n, b.ax[1])) + b.h.z * fabs(dt3(n, b.ax[2]));
+  const double sep = distance - (rA + rB);
+  const bool separated = ballot(tested && sep > cd) != 0;
+  const int fBest = group_argmax(sep, tested && gl < 6), eBest = group_argmax(sep, tested && gl >= 6);
+  const double fSep = gshfl(sep, max(fBest, 0)), eSep = gshfl(sep, max(eBest, 0));
+  const bool live = act && !separated && fBest >= 0;
+  if (!__any_sync(0xffffffffu, live)) return 0;
+  const bool edge = eBest >= 0 && 0.95 * eSep > fSep + 0.01;
+  n = gshfl(n, max(edge ? eBest : fBest, 0));
+  {  // orthonormal(basis, -n): the three quotients on three lanes
+    const D3 m = neg(n);
+    const bool xz = fabs(m.x) > fabs(m.z);
+    const D3 t{xz ? -m.y : 0.0, xz ? m.x : -m.z, xz ? 0.0 : m.y};
+    const double len = sqrt(t.x * t.x + t.y * t.y + t.z * t.z);
+    const double part = (gl == 0 ? t.x : gl == 1 ? t.y : t.z) / len;
+    const D3 u{gshfl(part, 0), gshfl(part, 1), gshfl(part, 2)};
+    basis[0] = m.x; basis[1] = m.y; basis[2] = m.z;
+    basis[3] = u.x; basis[4] = u.y; basis[5] = u.z;
+    basis[6] = m.y * u.z - m.z * u.y;
+    basis[7] = m.z * u.x - m.x * u.z;
+    basis[8] = m.x * u.y - m.y * u.x;
+  }
+  int count = 0;
+  if (__any_sync(0xffffffffu, live && !edge)) {  // faceManifold (collide.js:403-472)
+    const bool face = live && !edge;
+    const bool refIsA = fBest < 3;
+    const int refAxis = refIsA ? max(fBest, 0) : fBest - 3;
+    const D3 rc = pick3(refIsA, a.c, b.c), rh = pick3(refIsA, a.h, b.h);
+    const D3 ic = pick3(refIsA, b.c, a.c), ih = pick3(refIsA, b.h, a.h);
+    const int rBase = refIsA ? 0 : 3, iBase = 3 - rBase;
+    const D3 refAx = gshfl(mine, rBase + refAxis);
+    const D3 outward = pick3(refIsA, n, neg(n));
+    const D3 fN = scl(refAx, dt3(outward, refAx) >= 0 ? 1.0 : -1.0);
+    const D3 fC = adds(rc, fN, Collider::hcomp(rh, refAxis));
+    const int u0 = refAxis == 0 ? 1 : 0, v0 = refAxis == 2 ? 1 : 2;
+    const D3 fU = gshfl(mine, rBase + u0), fV = gshfl(mine, rBase + v0);
+    const double fEU = Collider::hcomp(rh, u0), fEV = Collider::hcomp(rh, v0);
+    // the incident face: the axis most parallel to the normal, the first on ties
+    const double dot = dt3(mine, fN);
+    int inc = 0;
+    double best = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double d = fabs(gshfl(dot, iBase + i));
+      if (d > best) {
+        best = d;
+        inc = i;
+      }
+    }
+    const D3 fn = scl(gshfl(mine, iBase + inc), gshfl(dot, iBase + inc) > 0 ? -1.0 : 1.0);
+    const D3 fc = adds(ic, fn, Collider::hcomp(ih, inc));
+    const int u1 = inc == 0 ? 1 : 0, v1 = inc == 2 ? 1 : 2;
+    const D3 u = gshfl(mine, iBase + u1), v = gshfl(mine, iBase + v1);
+    const double eU = Collider::hcomp(ih, u1), eV = Collider::hcomp(ih, v1);
+    const double su = (gl == 0 || gl == 3) ? 1.0 : -1.0, sv = (gl == 0 || gl == 1) ? 1.0 : -1.0;
+    D3 p{fc.x + u.x * (eU * su) + v.x * (eV * sv), fc.y + u.y * (eU * su) + v.y * (eV * sv),
+         fc.z + u.z * (eU * su) + v.z * (eV * sv)};
+    int num = face ? 4 : 0;
+#pragma unroll 1
+    for (int k = 0; k < 4; k++) {  // clipPlane (collide.js:202-247)
+      D3 pn = pick3(k < 2, fU, fV);
+      if (k & 1) pn = neg(pn);
+      const double po = dt3(pn, fC) + (k < 2 ? fEU : fEV);
+      const double db = pn.x * p.x + pn.y * p.y + pn.z * p.z - po;
+      const int prev = gl == 0 ? max(num - 1, 0) : gl - 1;
+      const D3 pa = gshfl(p, prev);
+      const double da = gshfl(db, prev);
+      const bool ai = da <= geo::kPlaneEps, bi = db <= geo::kPlaneEps;
+      const bool cross = gl < num && ai != bi, keep = gl < num && bi;
+      double t = 0;
+      const double denom = da - db;
+      if (fabs(denom) > geo::kSatEps) t = clampd(da / denom, 0, 1);
+      const D3 x{pa.x + (p.x - pa.x) * t, pa.y + (p.y - pa.y) * t, pa.z + (p.z - pa.z) * t};
+      const unsigned m1 = ballot(cross), m2 = ballot(keep), below = (1u << gl) - 1u;
+      const int at = __popc(m1 & below) + __popc(m2 & below);
+      if (cross && at < geo::kPolyCap) poly[at] = x;
+      if (keep && at + (cross ? 1 : 0) < geo::kPolyCap) poly[at + (cross ? 1 : 0)] = p;
+      num = min(__popc(m1) + __popc(m2), geo::kPolyCap);
+      __syncwarp();
+      if (gl < num) p = poly[gl];
+      __syncwarp();
+    }
+    const double dist = dt3(sub(p, fC), fN);
+    const bool kept = gl < num && !(dist > cd + geo::kPlaneEps);
+    const D3 proj = adds(p, fN, -dist);
+    D3 xA = pick3(refIsA, proj, p), xB = pick3(refIsA, p, proj);
+    // addContact (collide.js:254-285): a point within 1 mm of an earlier contact merges into it
+    const D3 m{(xA.x + xB.x) * 0.5, (xA.y + xB.y) * 0.5, (xA.z + xB.z) * 0.5};
+    unsigned close = 0u;
+#pragma unroll 1
+    for (int j = 0; j < geo::kPolyCap - 1; j++) {
+      const D3 mj = gshfl(m, j);
+      const double dx = m.x - mj.x, dy = m.y - mj.y, dz = m.z - mj.z;
+      if (j < gl && dx * dx + dy * dy + dz * dz < geo::kMergeDistSq) close |= 1u << j;
+    }
+    const unsigned keptMask = ballot(kept);
+    unsigned taken = 0u;
+#pragma unroll
+    for (int i = 0; i < geo::kPolyCap; i++) {
+      const unsigned ci = __shfl_sync(0xffffffffu, close, i, kGroup);
+      if (((keptMask >> i) & 1u) && !(ci & taken)) taken |= 1u << i;
+    }
+    count = __popc(taken);
+    uint32_t key = (uint32_t)(refIsA ? geo::kFaceA : geo::kFaceB) << 24;
+    key |= (uint32_t)(refAxis & 0xff) << 16;
+    key |= (uint32_t)(inc & 0xff) << 8;
+    bool own = ((taken >> gl) & 1u) != 0;
+    const bool none = face && num > 0 && count == 0;  // (clipped away whole: no contact)
+    if (__any_sync(0xffffffffu, none)) {  // no vertex deep enough: the support points
+      const D3 sA = Collider::support(a, n), sB = Collider::support(b, neg(n));
+      if (none) {
+        xA = sA;
+        xB = sB;
+        own = gl == 0;
+        count = 1;
+        taken = 1u;
+      }
+    }
+    const D3 ra = rot(conj(A.q), sub(xA, A.p)), rb = rot(conj(B.q), sub(xB, B.p));
+    if (face && own) {
+      slot = __popc(taken & ((1u << gl) - 1u));
+      nc.feature = key | (uint32_t)(gl & 0xff);
+      nc.ra[0] = (float)ra.x; nc.ra[1] = (float)ra.y; nc.ra[2] = (float)ra.z;
+      nc.rb[0] = (float)rb.x; nc.rb[1] = (float)rb.y; nc.rb[2] = (float)rb.z;
+    }
+    if (!face) count = 0;
+  }
+  if (live && edge) {  // the edge contact by the group's first lane
+    count = 1;
+    if (gl == 0) {
+      NewContact e[1];
+      Collider col(A, B, e);
+      col.boxA = a;
+      col.boxB = b;
+      col.cd = cd;
+      count = col.edgeContact((eBest - 6) / 3, (eBest - 6) % 3, n);
+      slot = 0;
+      nc.feature = e[0].feature;
+      nc.ra[0] = (float)e[0].rA.x; nc.ra[1] = (float)e[0].rA.y; nc.ra[2] = (float)e[0].rA.z;
+      nc.rb[0] = (float)e[0].rB.x; nc.rb[1] = (float)e[0].rB.y; nc.rb[2] = (float)e[0].rB.z;
+    }
+  }
+  __syncwarp();
+  return live ? count : 0;
+}
+
+// A lane's pair decided by the serial collider: every sphere pair, and box
+// pairs of long lists.
+__device__ __noinline__ void exact_pair(const World &w, int c) {
+  const uint64_t key = w.g.candKey[c];
+  const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
+  const BodyD A = load_body(w, ia), B = load_body(w, ib);
+  double basis[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  NewContact nc[kMaxContacts];
+  Collider col(A, B, nc);
+  col.cd = pair_skin(w, ia, ib);
+  const int num = col.collide(basis);
+  if (A.sphere || B.sphere) {
+    write_sphere_manifold(w, c, ia, ib, A, B, nc, num, basis);
+    return;
+  }
+  NewContactF ncf[kMaxContacts];
+  for (int k = 0; k < num; k++) {
+    ncf[k].feature = nc[k].feature;
+    ncf[k].ra[0] = (float)nc[k].rA.x; ncf[k].ra[1] = (float)nc[k].rA.y; ncf[k].ra[2] = (float)nc[k].rA.z;
+    ncf[k].rb[0] = (float)nc[k].rB.x; ncf[k].rb[1] = (float)nc[k].rB.y; ncf[k].rb[2] = (float)nc[k].rB.z;
+  }
+  write_box_manifold(w, c, ia, ib, A, B, ncf, num, basis);
+}
+
+// 4. Sphere pairs and undecided box pairs: the whole f64 collider. Lists of up
+//    to kGroupMax pairs: box pairs on sixteen lanes each. Longer ones keep every
+//    sub-partition's FP64 pipe busy either way, and a pair a thread then needs
+//    about half the warp instructions (narrow phase of a batch with 10,257 such
+//    pairs: 0.70 ms on lanes, 0.72 by threads; of a crushed pyramid with 37,825:
+//    1.24 and 0.93).
+constexpr int kGroupMax = 16384;
+__global__ void __launch_bounds__(128) exact_kernel(const __grid_constant__ World w) {
   const int total = *((volatile int *)&w.ctl->npCount[2]);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int c = w.g.npExact[t];
-    const uint64_t key = w.g.candKey[c];
+  if (total > kGroupMax) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x)
+      exact_pair(w, w.g.npExact[t]);
+    return;
+  }
+  __shared__ D3 poly[8][geo::kPolyCap];
+  __shared__ NewContactF held[8][kMaxContacts];
+  const int group = threadIdx.x / kGroup, gl = threadIdx.x & (kGroup - 1);
+  // warps dealt over the blocks first
+  const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (blockDim.x >> 5);
+  for (int t0 = warp * 2; t0 < total; t0 += warps * 2) {
+    const int t = t0 + (group & 1);
+    const int c = t < total ? w.g.npExact[t] : -1;
+    const uint64_t key = w.g.candKey[c >= 0 ? c : w.g.npExact[t0]];
     const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
     const BodyD A = load_body(w, ia), B = load_body(w, ib);
-    double basis[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    NewContact nc[kMaxContacts];
-    Collider col(A, B, nc);
-    col.cd = pair_skin(w, ia, ib);
-    const int num = col.collide(basis);
-    if (A.sphere || B.sphere) {
-      write_sphere_manifold(w, c, ia, ib, A, B, nc, num, basis);
-      continue;
+    const bool sphere = A.sphere || B.sphere, act = c >= 0 && !sphere;
+    if (__any_sync(0xffffffffu, act)) {
+      double basis[9];
+      NewContactF nc;
+      int slot;
+      const int num = collide_group(A, B, pair_skin(w, ia, ib), act, poly[group], basis, nc, slot);
+      if (act && gl == 0) w.cur.count[c] = num;
+      if (w.p.contactModel) {  // the materials merge claims old contacts one after the other
+        if (act && slot >= 0) held[group][slot] = nc;
+        __syncwarp();
+        if (act && num && gl == 0) write_box_manifold(w, c, ia, ib, A, B, held[group], num, basis);
+        __syncwarp();
+      } else if (act && num) {
+        float bf[9];
+        for (int k = 0; k < 9; k++) bf[k] = (float)basis[k];
+        const int pi = w.g.candPrev[c];
+        const int oldNum = pi >= 0 ? w.prev.count[pi] : 0;
+        if (slot >= 0) write_box_contact(w, c, slot, pi, oldNum, A, B, nc, bf);
+        if (gl == 0) write_box_header(w, c, ia, ib, basis, bf);
+      }
     }
-    NewContactF ncf[kMaxContacts];
-    for (int k = 0; k < num; k++) {
-      ncf[k].feature = nc[k].feature;
-      ncf[k].ra[0] = (float)nc[k].rA.x; ncf[k].ra[1] = (float)nc[k].rA.y; ncf[k].ra[2] = (float)nc[k].rA.z;
-      ncf[k].rb[0] = (float)nc[k].rB.x; ncf[k].rb[1] = (float)nc[k].rB.y; ncf[k].rb[2] = (float)nc[k].rB.z;
-    }
-    write_box_manifold(w, c, ia, ib, A, B, ncf, num, basis);
+    if (c >= 0 && sphere && gl == 0) exact_pair(w, c);
+    __syncwarp();
   }
 }
 
