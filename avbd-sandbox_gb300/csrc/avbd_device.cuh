@@ -94,7 +94,7 @@ struct Control {
   int liveManifolds;
   int liveContacts;
   int fp64Bodies;
-  int adjTotal;
+  int gridEntries;  // grid entries handed out this step
   int prevCandidates;  // candidates (= manifold slots) of the previous step
   int npCount[3];      // narrow-phase work lists: face, edge, exact
   int colorBad;        // this step's uploaded colouring has a conflict
@@ -183,14 +183,6 @@ struct Springs {
   D4 *dptD;
 };
 
-// One hash-grid insertion: the body's exact broad-phase inputs travel with
-// it, so the sphere test needs no further loads. b2 = (body << 1) | dynamic;
-// loc = f32 offset of the centre from its cell's corner, w = radius (f32).
-struct __align__(16) Entry {
-  double x, y, z, r;
-  float4 loc;
-  int b2, cx, cy, cz;
-};
 constexpr int kPairScratch = 128;     // partner row of a step's broad phase
 constexpr int kLargeChunk = 1024;     // bodies a block tests against one large body
 constexpr int kStaticPairRow = 64;    // partner row of the allocation-free query
@@ -207,8 +199,14 @@ struct Grid {
   float4 *loc;               // per body: f32 offset from the cell corner, w = radius
   const float *cellF;        // per scene: cell edge (f32 of 1 / invCell)
   unsigned tableMask;
-  int *tableCount, *tableStart, *tableCursor;
-  struct Entry *entries;
+  int2 *table;                   // per hash bucket: its first entry, its bodies
+  int *rank;                     // per body: its place within its bucket
+  int *prevStart;                // n + 1: a body's first manifold slot of the previous step
+  int *rangeSum;                 // partners of each block's run of bodies (pair_ranges)
+  // grid entries, one per regular body: (body << 1) | dynamic and its cell;
+  // f32 offset of the centre from the cell's corner, w = radius (f32)
+  int4 *entryId;
+  float4 *entryLoc;
   int entryCap;
   uint32_t *scratch;  // per body: sorted lower-index partners (kPairScratch each)
   int hasConstraints; // any joint or spring in the world
@@ -408,9 +406,8 @@ __host__ __device__ inline uint32_t color_priority(uint32_t x) {
 }
 
 // Kernel launchers (defined in the .cu files; all asynchronous on `st`).
-size_t broadphase_temp_bytes(int n, int tableSize);
-void launch_broadphase_impl(const World &w, int numLarge, void *temp, size_t tempBytes, cudaStream_t st,
-                            int smCount);
+int pair_ranges_max(int n);  // entries of Grid::rangeSum
+void launch_broadphase_impl(const World &w, int numLarge, cudaStream_t st, int smCount);
 void launch_narrowphase(const World &w, cudaStream_t st, int smCount);
 size_t solver_temp_bytes(int n);
 void launch_prepare(const World &w, void *temp, size_t tempBytes, cudaStream_t st, int smCount);

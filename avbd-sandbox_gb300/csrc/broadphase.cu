@@ -14,14 +14,18 @@
 //      centre; the per-scene cell is at least twice the largest regular
 //      bounding radius, so overlapping regular bodies sit in adjacent cells.
 //      Bodies above twice the scene's 95th-percentile radius are "large" and
-//      are tested against every body of their scene. Counting sort by cell
-//      hash: count, exclusive scan, scatter.
+//      are tested against every body of their scene. Grouped by cell hash:
+//      count (a body's place in its bucket is the count it found), hand each
+//      bucket its run of entries, scatter - no scan over the table, since the
+//      order of the runs is free.
 //   2. per body A (one warp): its 27 neighbour cells, the scene's large
 //      bodies and its old manifolds give the partners B < A; they are sorted
-//      in shared memory and parked in a per-body scratch row with their count
-//   3. exclusive scan of the counts; each body copies its sorted row into its
-//      segment: a globally sorted candidate key array without a global sort
-//   4. per candidate: index of the same pair in the previous step's manifolds
+//      in shared memory and parked in a per-body scratch row with their count;
+//      a block owns a run of bodies and leaves the run's total
+//   3. each block sums the totals of the runs before its own, scans its run
+//      and copies its bodies' sorted rows into their segments: a globally
+//      sorted candidate key array without a global sort
+//   (the narrow phase looks up each candidate's previous manifold)
 #include <cub/cub.cuh>
 
 #include <mutex>
@@ -66,8 +70,7 @@ __device__ __forceinline__ int sphere_f32(int4 ca, float4 la, int cx, int cy, in
 
 // The `visit` predicate of solver.js:316-329 for A = bodies[a], B = bodies[b], b < a.
 __device__ bool accept(const World &w, int a, int b) {
-  const double ma = w.b.massD[a].x, mb = w.b.massD[b].x;
-  if (!(ma > 0 || mb > 0)) return false;
+  if (!((w.b.flags0[a] | w.b.flags0[b]) & kBodyDynamic)) return false;
   const int4 cb = w.g.cellLo[b];
   int t = -1;
   if (cb.w >= 0) t = sphere_f32(w.g.cellLo[a], w.g.loc[a], cb.x, cb.y, cb.z, w.g.loc[b], w.g.cellF[cb.w]);
@@ -111,8 +114,30 @@ __device__ bool centre_cell(const World &w, int i, int4 &c) {
   return ok;
 }
 
+__device__ __forceinline__ uint32_t bucket_of(const World &w, int4 c) {
+  return cell_hash(c.x, c.y, c.z, c.w) & w.g.tableMask;
+}
+
+// Per body: its cell and its place in the cell's bucket, and its first slot
+// among the previous step's manifolds (keys sorted, A-major): a binary search
+// a thread here instead of one by a single lane of each body's warp (with a
+// walk along the body's manifolds after it) and another per candidate later:
+// the broad phase of a 163,000-body batch 0.55 -> 0.42 ms with the fewer
+// launches, of a crushed pyramid 0.54 -> 0.28.
 __global__ void cells_kernel(World w) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.b.n; i += gridDim.x * blockDim.x) {
+  const int prevCount = w.ctl->prevCandidates;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= w.b.n; i += gridDim.x * blockDim.x) {
+    if (prevCount > 0) {
+      const uint64_t lo = (uint64_t)(uint32_t)i << 32;
+      int l = 0, h = i < w.b.n ? prevCount : 0;
+      while (l < h) {
+        const int m = (l + h) >> 1;
+        if (w.prev.key[m] < lo) l = m + 1;
+        else h = m;
+      }
+      w.g.prevStart[i] = i < w.b.n ? l : prevCount;
+    }
+    if (i == w.b.n) break;
     int4 c;
     const bool ok = centre_cell(w, i, c);
     if (ok) {  // f32 offset from the cell corner (cell = 1 / invCell, as the f32 test's cell)
@@ -124,7 +149,34 @@ __global__ void cells_kernel(World w) {
     c.w = ok ? c.w : -1 - c.w;  // scene, negative when the body has no cell
     w.g.cellLo[i] = c;
     if (!ok || is_large(w, i)) continue;
-    atomicAdd(&w.g.tableCount[cell_hash(c.x, c.y, c.z, c.w) & w.g.tableMask], 1);
+    w.g.rank[i] = atomicAdd(&w.g.table[bucket_of(w, c)].y, 1);
+  }
+}
+
+// The first body of each bucket takes the bucket's run of entries: one atomic
+// a warp.
+__global__ void bucket_kernel(World w) {
+  const int lane = threadIdx.x & 31;
+  for (int i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < w.b.n; i0 += gridDim.x * blockDim.x) {
+    const int i = i0 + lane;
+    uint32_t bucket = 0;
+    int count = 0;
+    if (i < w.b.n) {
+      const int4 c = w.g.cellLo[i];
+      if (c.w >= 0 && !is_large(w, i) && w.g.rank[i] == 0) {
+        bucket = bucket_of(w, c);
+        count = w.g.table[bucket].y;
+      }
+    }
+    int incl = count;
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    int base = 0;
+    if (lane == 31 && incl) base = atomicAdd(&w.ctl->gridEntries, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (count) w.g.table[bucket].x = base + incl - count;
   }
 }
 
@@ -132,40 +184,20 @@ __global__ void scatter_kernel(World w) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.b.n; i += gridDim.x * blockDim.x) {
     const int4 c = w.g.cellLo[i];
     if (c.w < 0 || is_large(w, i)) continue;
-    const int at = atomicAdd(&w.g.tableCursor[cell_hash(c.x, c.y, c.z, c.w) & w.g.tableMask], 1);
+    const int at = w.g.table[bucket_of(w, c)].x + w.g.rank[i];
     if (at < w.g.entryCap) {
-      const D4 p = w.b.pos[i];
-      Entry e;
-      e.x = p.x; e.y = p.y; e.z = p.z; e.r = w.b.size[i].w;
-      e.loc = w.g.loc[i];
-      e.b2 = (i << 1) | ((w.b.flags0[i] & kBodyDynamic) ? 1 : 0);
-      e.cx = c.x; e.cy = c.y; e.cz = c.z;
-      w.g.entries[at] = e;
+      w.g.entryId[at] = make_int4((i << 1) | ((w.b.flags0[i] & kBodyDynamic) ? 1 : 0), c.x, c.y, c.z);
+      w.g.entryLoc[at] = w.g.loc[i];
     } else {
       atomicOr(&w.ctl->flags, kOvfCells);
     }
   }
 }
 
-// Range of body a's manifolds in the previous step (keys sorted, A-major).
-__device__ void prev_range(const World &w, int a, int prevCount, int &first, int &last) {
-  const uint64_t lo = (uint64_t)(uint32_t)a << 32;
-  int l = 0, h = prevCount;
-  while (l < h) {
-    const int m = (l + h) >> 1;
-    if (w.prev.key[m] < lo) l = m + 1;
-    else h = m;
-  }
-  first = l;
-  last = l;
-  while (last < prevCount && (int)(w.prev.key[last] >> 32) == a) last++;
-}
-
 // Large bodies: every body b < a of the scene is tested, in chunks of
 // kLargeChunk bodies, one block per (large body, chunk).
-// 1. the accepted count of each chunk
-__global__ void __launch_bounds__(256) large_count_kernel(World w) {
-  const int li = blockIdx.y, ch = blockIdx.x;
+// 1. the accepted count of each chunk (blocks of pairs_kernel's launch)
+__device__ void large_count(const World &w, int li, int ch) {
   const int a = w.g.largeList[li];
   const int s0 = w.g.sceneStart[w.b.scene[a]];
   const int b0 = s0 + ch * kLargeChunk, b1 = min(a, b0 + kLargeChunk);
@@ -177,12 +209,25 @@ __global__ void __launch_bounds__(256) large_count_kernel(World w) {
   if (threadIdx.x == 0) w.g.largeChunk[li * w.g.maxChunks + ch] = b0 < b1 ? total : 0;
 }
 
-// 2. per large body: chunk counts -> chunk offsets, plus the old manifolds the
-//    sphere test rejects (they stay candidates); the body's partner count
-__global__ void large_total_kernel(World w) {
+// Old manifolds of body a that the sphere test rejects (they stay
+// candidates), counted by the block; thread 0 gets the count.
+__device__ int large_rejects(const World &w, int a) {
+  int c = 0;
+  if (w.ctl->prevCandidates > 0)
+    for (int m = w.g.prevStart[a] + threadIdx.x; m < w.g.prevStart[a + 1]; m += blockDim.x)
+      if (w.prev.count[m] > 0 && !accept(w, a, (int)(w.prev.key[m] & 0xffffffffu))) c++;
+  typedef cub::BlockReduce<int, 256> R;
+  __shared__ typename R::TempStorage tmp;
+  return R(tmp).Sum(c);
+}
+
+// 2. per large body: chunk counts -> chunk offsets, plus the rejected old
+//    manifolds; the body's partner count, added to its run's total
+__global__ void __launch_bounds__(256) large_total_kernel(World w, int per) {
   const int li = blockIdx.x;
-  if (threadIdx.x != 0) return;
   const int a = w.g.largeList[li];
+  const int extra = large_rejects(w, a);
+  if (threadIdx.x != 0) return;
   int *cnt = w.g.largeChunk + li * w.g.maxChunks;
   int run = 0;
   for (int ch = 0; ch < w.g.maxChunks; ch++) {
@@ -190,11 +235,8 @@ __global__ void large_total_kernel(World w) {
     cnt[ch] = run;
     run += v;
   }
-  int first, last;
-  prev_range(w, a, w.ctl->prevCandidates, first, last);
-  for (int m = first; m < last; m++)
-    if (w.prev.count[m] > 0 && !accept(w, a, (int)(w.prev.key[m] & 0xffffffffu))) run++;
-  w.g.pairCount[a] = run;
+  w.g.pairCount[a] = run + extra;
+  atomicAdd(&w.g.rangeSum[a / per], run + extra);
 }
 
 __device__ void sort_segment(uint64_t *k, int n) {
@@ -220,23 +262,29 @@ struct BodyA {
 };
 
 // The `visit` predicate (solver.js:316-329) against a grid entry.
-__device__ __forceinline__ bool accept_entry(const World &w, const BodyA &A, const Entry &e) {
-  if (!(A.dyn || (e.b2 & 1))) return false;
-  const int t = sphere_f32(A.c, A.loc, e.cx, e.cy, e.cz, e.loc, A.cell);
+__device__ __forceinline__ bool accept_entry(const World &w, const BodyA &A, int4 id, float4 loc) {
+  if (!(A.dyn || (id.x & 1))) return false;
+  const int t = sphere_f32(A.c, A.loc, id.y, id.z, id.w, loc, A.cell);
   if (t == 0) return false;
+  const int b = id.x >> 1;
   if (t < 0) {
-    const double dx = A.x - e.x, dy = A.y - e.y, dz = A.z - e.z;
-    const double r = A.r + e.r;
+    const D4 pb = w.b.pos[b];
+    const double dx = A.x - pb.x, dy = A.y - pb.y, dz = A.z - pb.z;
+    const double r = A.r + w.b.size[b].w;
     if (!(dx * dx + dy * dy + dz * dz <= r * r)) return false;
   }
-  return !w.g.hasConstraints || accept(w, A.a, e.b2 >> 1);
+  return !w.g.hasConstraints || accept(w, A.a, b);
 }
 
-// Warp-cooperative enumeration of the partners b < a of a non-large body a:
-// lanes take the 27 neighbour cells (and the old manifolds and the scene's
-// large bodies), calling f(b) on the lane that finds b. Each partner is
-// found exactly once: regular bodies live in exactly one cell; old manifolds
-// are added only when the sphere test rejects them.
+// Warp-cooperative enumeration of the partners b < a of a non-large body a
+// (the scene's large bodies, the 27 neighbour cells, the old manifolds),
+// calling f(b) on the lane that finds b. The cells' entries are laid end to
+// end and dealt to the lanes 32 at a time, so that lanes read neighbouring
+// entries and a full cell does not hold up 31 of them (a pile's small boxes
+// lie ten and more to a cell; the batch 0.42 -> 0.29 ms, the crushed pyramid
+// 0.28 -> 0.17, with 32-byte entries in place of 64). Each partner is found exactly once: regular
+// bodies live in exactly one cell; old manifolds are added only when the
+// sphere test rejects them.
 template <class F>
 __device__ void warp_partners(const World &w, const BodyA &A, int prevCount, int lane, F &&f) {
   const int a = A.a, s = A.s;
@@ -245,25 +293,38 @@ __device__ void warp_partners(const World &w, const BodyA &A, int prevCount, int
     const int b = w.g.largeList[k];
     if (b < a && accept(w, a, b)) f(b);
   }
+  int2 run = make_int2(0, 0);  // this lane's cell: first entry, entries
   if (lane < 27) {
-    const int x = A.c.x + lane / 9 - 1, y = A.c.y + (lane / 3) % 3 - 1, z = A.c.z + lane % 3 - 1;
-    const uint32_t bucket = cell_hash(x, y, z, s) & w.g.tableMask;
-    const int beg = w.g.tableStart[bucket];
-    int end = beg + w.g.tableCount[bucket];
-    if (end > w.g.entryCap) end = w.g.entryCap;
-    for (int k = beg; k < end; k++) {
-      const Entry e = w.g.entries[k];
-      const int b = e.b2 >> 1;
-      // entries carry their cell: other cells hashing to this bucket are skipped
-      if (b >= a || e.cx != x || e.cy != y || e.cz != z) continue;
-      if (w.g.numScenes > 1 && w.b.scene[b] != s) continue;  // another scene's cell, same bucket
-      if (accept_entry(w, A, e)) f(b);
-    }
+    run = w.g.table[cell_hash(A.c.x + lane / 9 - 1, A.c.y + (lane / 3) % 3 - 1, A.c.z + lane % 3 - 1, s) &
+                    w.g.tableMask];
+    run.y = min(run.y, w.g.entryCap - run.x);
+    if (run.y < 0) run.y = 0;
   }
-  int first = 0, last = 0;
-  if (lane == 0) prev_range(w, a, prevCount, first, last);
-  first = __shfl_sync(0xffffffffu, first, 0);
-  last = __shfl_sync(0xffffffffu, last, 0);
+  int end = run.y;  // entries of the cells up to this lane's
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, end, d);
+    if (lane >= d) end += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, end, 31);
+  const int skip = run.x - (end - run.y);  // entry index minus place
+  for (int i0 = 0; i0 < total; i0 += 32) {
+    const int i = i0 + lane;
+    int c = 0;  // the cell of place i: the cells that end at or before it
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1)
+      if (__shfl_sync(0xffffffffu, end, c + d - 1) <= i) c += d;
+    const int k = __shfl_sync(0xffffffffu, skip, c) + i;
+    if (i >= total) continue;
+    const int4 id = w.g.entryId[k];
+    const int b = id.x >> 1;
+    // entries carry their cell: other cells hashing to this bucket are skipped
+    if (b >= a || id.y != A.c.x + c / 9 - 1 || id.z != A.c.y + (c / 3) % 3 - 1 || id.w != A.c.z + c % 3 - 1) continue;
+    if (w.g.numScenes > 1 && w.b.scene[b] != s) continue;  // another scene's cell, same bucket
+    if (accept_entry(w, A, id, w.g.entryLoc[k])) f(b);
+  }
+  __syncwarp();
+  if (prevCount <= 0) return;
+  const int first = w.g.prevStart[a], last = w.g.prevStart[a + 1];
   for (int m = first + lane; m < last; m += 32) {
     if (w.prev.count[m] <= 0) continue;
     const int b = (int)(w.prev.key[m] & 0xffffffffu);
@@ -286,18 +347,38 @@ __device__ BodyA body_a(const World &w, int a) {
 }
 
 constexpr int kWarpsPerBlock = 8;
+constexpr int kHeavyRow = 512;  // partners of a body that its warp sorts in shared memory
+
+// The runs of bodies that the blocks of pairs_kernel and copy_kernel own.
+struct PairRanges {
+  int blocks, per;
+};
+PairRanges pair_ranges(int n, int smCount) {
+  const int most = smCount * 32, rows = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  const int per = kWarpsPerBlock * std::max(1, (rows + most - 1) / most);
+  return PairRanges{std::max(1, (n + per - 1) / per), per};
+}
 
 // One pass per non-large body: count its partners and, when they fit, leave
-// them sorted in its scratch row (kRow entries) for the copy after the scan.
+// them sorted in its scratch row (kRow entries) for the copy. Blocks past the
+// runs count the large bodies' chunks.
 template <int kRow>
-__global__ void __launch_bounds__(256) pairs_kernel(World w) {
+__global__ void __launch_bounds__(256) pairs_kernel(World w, int blocks, int per) {
+  if ((int)blockIdx.x >= blocks) {
+    const int k = blockIdx.x - blocks;
+    large_count(w, k / w.g.maxChunks, k % w.g.maxChunks);
+    return;
+  }
   __shared__ uint32_t buf[kWarpsPerBlock][kRow];
   __shared__ int fill[kWarpsPerBlock];
+  __shared__ int sum;
+  if (threadIdx.x == 0) sum = 0;
+  __syncthreads();
   const int prevCount = w.ctl->prevCandidates;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
-  for (int a = warp; a < w.b.n; a += warps) {
-    if (is_large(w, a)) continue;  // large_count_kernel
+  const int b0 = blockIdx.x * per, b1 = min(w.b.n, b0 + per);
+  for (int a = b0 + wib; a < b1; a += kWarpsPerBlock) {
+    if (is_large(w, a)) continue;  // large_count
     const BodyA A = body_a(w, a);
     if (lane == 0) fill[wib] = 0;
     __syncwarp();
@@ -307,7 +388,10 @@ __global__ void __launch_bounds__(256) pairs_kernel(World w) {
     });
     __syncwarp();
     const int n = fill[wib];
-    if (lane == 0) w.g.pairCount[a] = n;
+    if (lane == 0) {
+      w.g.pairCount[a] = n;
+      atomicAdd(&sum, n);
+    }
     if (n <= kRow) {
       // rank sort (partners are distinct): element i goes to #{j : b_j < b_i}
       uint32_t *row = w.g.scratch + (size_t)a * kRow;
@@ -320,23 +404,93 @@ __global__ void __launch_bounds__(256) pairs_kernel(World w) {
     }
     __syncwarp();
   }
+  __syncthreads();
+  if (threadIdx.x == 0) w.g.rangeSum[blockIdx.x] = sum;
 }
 
-// Copy each body's sorted partners into its segment of the key array. The
-// rare bodies with more than kRow partners are enumerated again by their
-// warp straight into the segment, which the warp then sorts in place (odd-even
-// transposition: n rounds of compare-exchange on alternating pairs).
+// Partners before body a: the totals of the runs before its own, and the
+// counts before it in its run. Block-wide; every thread gets it.
+__device__ int pairs_before(const World &w, int a, int per) {
+  int v = 0;
+  const int r = a / per;
+  for (int k = threadIdx.x; k < r; k += blockDim.x) v += w.g.rangeSum[k];
+  for (int i = r * per + threadIdx.x; i < a; i += blockDim.x) v += w.g.pairCount[i];
+  typedef cub::BlockReduce<int, 256> R;
+  __shared__ typename R::TempStorage tmp;
+  __shared__ int total;
+  v = R(tmp).Sum(v);
+  if (threadIdx.x == 0) total = v;
+  __syncthreads();
+  v = total;
+  __syncthreads();
+  return v;
+}
+
+// 3. each chunk writes its accepted partners at its offset, in index order
+//    (blocks of copy_kernel's launch)
+__device__ void large_write(const World &w, int li, int ch, int per) {
+  const int a = w.g.largeList[li];
+  const int s0 = w.g.sceneStart[w.b.scene[a]];
+  const int b0 = s0 + ch * kLargeChunk, b1 = min(a, b0 + kLargeChunk);
+  if (b0 >= b1) return;
+  const int beg = pairs_before(w, a, per);
+  const int n = w.g.pairCount[a];
+  if ((long long)beg + n > w.g.candCap) {
+    if (threadIdx.x == 0) atomicOr(&w.ctl->flags, kOvfPairs);
+    return;
+  }
+  uint64_t *seg = w.g.candKey + beg;
+  const uint64_t hiKey = (uint64_t)(uint32_t)a << 32;
+  typedef cub::BlockScan<int, 256> S;
+  __shared__ typename S::TempStorage tmp;
+  int base = w.g.largeChunk[li * w.g.maxChunks + ch];
+  for (int t0 = b0; t0 < b1; t0 += blockDim.x) {
+    const int b = t0 + threadIdx.x;
+    const int ok = (b < b1 && accept(w, a, b)) ? 1 : 0;
+    int at, tot;
+    S(tmp).ExclusiveSum(ok, at, tot);
+    if (ok && base + at < n) seg[base + at] = hiKey | (uint32_t)b;
+    base += tot;
+    __syncthreads();
+  }
+}
+
+// Each block scans its run's partner counts into the bodies' segment starts
+// and copies their sorted rows into the key array. The rare bodies with more
+// than kRow partners are enumerated again by their warp: up to kHeavyRow are
+// rank-sorted in shared memory, more go straight into the segment, which the
+// warp then sorts in place (odd-even transposition: n rounds of
+// compare-exchange on alternating pairs; 130 us for a crushed pile's 150
+// partners, before the shared-memory form took those).
 template <int kRow>
-__global__ void __launch_bounds__(256) copy_kernel(World w) {
+__global__ void __launch_bounds__(256) copy_kernel(World w, int blocks, int per) {
+  if ((int)blockIdx.x >= blocks) {
+    const int k = blockIdx.x - blocks;
+    large_write(w, k / w.g.maxChunks, k % w.g.maxChunks, per);
+    return;
+  }
   __shared__ int fill[kWarpsPerBlock];
+  __shared__ uint32_t heavy[kWarpsPerBlock][kHeavyRow];
+  typedef cub::BlockScan<int, 256> S;
+  __shared__ typename S::TempStorage tmp;
   const int prevCount = w.ctl->prevCandidates;
   const int cap = w.g.candCap;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
-  for (int a = warp; a < w.b.n; a += warps) {
+  const int b0 = blockIdx.x * per, b1 = min(w.b.n, b0 + per);
+  int base = pairs_before(w, b0, per);
+  for (int i0 = b0; i0 < b1; i0 += blockDim.x) {
+    const int i = i0 + threadIdx.x;
+    int at, tot;
+    S(tmp).ExclusiveSum(i < b1 ? w.g.pairCount[i] : 0, at, tot);
+    if (i < b1) w.g.pairStart[i] = base + at;
+    base += tot;
+    __syncthreads();
+  }
+  if (b1 == w.b.n && threadIdx.x == 0) w.g.pairStart[w.b.n] = base;
+  for (int a = b0 + wib; a < b1; a += kWarpsPerBlock) {
     if (is_large(w, a)) continue;
     const int beg = w.g.pairStart[a];
-    const int n = w.g.pairStart[a + 1] - beg;
+    const int n = w.g.pairCount[a];
     if (n == 0) continue;
     if (beg + n > cap) {
       if (lane == 0) atomicOr(&w.ctl->flags, kOvfPairs);
@@ -354,9 +508,21 @@ __global__ void __launch_bounds__(256) copy_kernel(World w) {
     const BodyA A = body_a(w, a);
     warp_partners(w, A, prevCount, lane, [&](int b) {
       const int at = atomicAdd(&fill[wib], 1);
-      if (at < n) seg[at] = hiKey | (uint32_t)b;
+      if (at >= n) return;
+      if (n <= kHeavyRow) heavy[wib][at] = (uint32_t)b;
+      else seg[at] = hiKey | (uint32_t)b;
     });
     __syncwarp();
+    if (n <= kHeavyRow) {
+      for (int i = lane; i < n; i += 32) {
+        const uint32_t v = heavy[wib][i];
+        int r = 0;
+        for (int j = 0; j < n; j++) r += heavy[wib][j] < v ? 1 : 0;
+        seg[r] = hiKey | v;
+      }
+      __syncwarp();
+      continue;
+    }
     for (int round = 0; round < n; round++) {
       for (int i = 2 * lane + (round & 1); i + 1 < n; i += 64) {
         const uint64_t x = seg[i], y = seg[i + 1];
@@ -370,128 +536,57 @@ __global__ void __launch_bounds__(256) copy_kernel(World w) {
   }
 }
 
-// 3. each chunk writes its accepted partners at its offset, in index order
-__global__ void __launch_bounds__(256) large_write_kernel(World w) {
-  const int li = blockIdx.y, ch = blockIdx.x;
-  const int a = w.g.largeList[li];
-  const int s0 = w.g.sceneStart[w.b.scene[a]];
-  const int b0 = s0 + ch * kLargeChunk, b1 = min(a, b0 + kLargeChunk);
-  if (b0 >= b1) return;
-  const int beg = w.g.pairStart[a];
-  const int n = w.g.pairStart[a + 1] - beg;
-  if ((long long)beg + n > w.g.candCap) {
-    if (threadIdx.x == 0) atomicOr(&w.ctl->flags, kOvfPairs);
-    return;
+// 4. per large body, the old manifolds the sphere test rejected, appended, and
+//    the segment sorted when there are any (rare: a large body's sphere holds
+//    its scene); and the step's candidate count: a step whose candidates
+//    exceed the arena (or that follows a skipped step) is skipped: no candidate
+//    reaches the narrow phase and every later kernel of the step returns at
+//    once (Control::skip).
+__global__ void __launch_bounds__(256) finish_kernel(World w, int numLarge) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int total = w.g.pairStart[w.b.n];
+    w.ctl->wantCandidates = total;
+    if (total > w.g.candCap) {
+      atomicOr(&w.ctl->flags, kOvfPairs);
+      w.ctl->skip = 1;
+    }
+    w.ctl->numCandidates = w.ctl->skip ? 0 : total;
   }
-  uint64_t *seg = w.g.candKey + beg;
-  const uint64_t hiKey = (uint64_t)(uint32_t)a << 32;
-  typedef cub::BlockScan<int, 256> S;
-  __shared__ typename S::TempStorage tmp;
-  __shared__ int base;
-  if (threadIdx.x == 0) base = w.g.largeChunk[li * w.g.maxChunks + ch];
-  __syncthreads();
-  for (int t0 = b0; t0 < b1; t0 += blockDim.x) {
-    const int b = t0 + threadIdx.x;
-    const int ok = (b < b1 && accept(w, a, b)) ? 1 : 0;
-    int at, tot;
-    S(tmp).ExclusiveSum(ok, at, tot);
-    if (ok && base + at < n) seg[base + at] = hiKey | (uint32_t)b;
-    __syncthreads();
-    if (threadIdx.x == 0) base += tot;
-    __syncthreads();
-  }
-}
-
-// 4. the old manifolds the sphere test rejected, appended, and the segment
-//    sorted when there are any (rare: a large body's sphere holds its scene)
-__global__ void large_extra_kernel(World w) {
   const int li = blockIdx.x;
-  if (threadIdx.x != 0) return;
+  if (li >= numLarge) return;
   const int a = w.g.largeList[li];
   const int beg = w.g.pairStart[a];
-  const int n = w.g.pairStart[a + 1] - beg;
+  const int n = w.g.pairCount[a];
   if ((long long)beg + n > w.g.candCap) return;
+  const int extra = large_rejects(w, a);
+  if (threadIdx.x != 0 || extra == 0) return;
   uint64_t *seg = w.g.candKey + beg;
   const uint64_t hiKey = (uint64_t)(uint32_t)a << 32;
-  int first, last;
-  prev_range(w, a, w.ctl->prevCandidates, first, last);
-  int c = n;
-  for (int m = last - 1; m >= first; m--)  // count the extras to find where they start
-    if (w.prev.count[m] > 0 && !accept(w, a, (int)(w.prev.key[m] & 0xffffffffu))) c--;
-  if (c == n) return;
-  for (int m = first; m < last; m++) {
+  int c = n - extra;
+  for (int m = w.g.prevStart[a]; m < w.g.prevStart[a + 1]; m++) {
     const int b = (int)(w.prev.key[m] & 0xffffffffu);
     if (w.prev.count[m] > 0 && !accept(w, a, b)) seg[c++] = hiKey | (uint32_t)b;
   }
   sort_segment(seg, n);
 }
 
-// The step's candidate count; a step whose candidates exceed the arena (or
-// that follows a skipped step) is skipped: no candidate reaches the narrow
-// phase and every later kernel of the step returns at once (Control::skip).
-__global__ void finish_kernel(World w) {
-  const int total = w.g.pairStart[w.b.n];
-  w.ctl->wantCandidates = total;
-  if (total > w.g.candCap) {
-    atomicOr(&w.ctl->flags, kOvfPairs);
-    w.ctl->skip = 1;
-  }
-  w.ctl->numCandidates = w.ctl->skip ? 0 : total;
-}
-
-__global__ void prev_index_kernel(World w) {
-  const int total = w.ctl->numCandidates;
-  const int prevCount = w.ctl->prevCandidates;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
-    const uint64_t k = w.g.candKey[c];
-    int l = 0, h = prevCount;
-    while (l < h) {
-      const int m = (l + h) >> 1;
-      if (w.prev.key[m] < k) l = m + 1;
-      else h = m;
-    }
-    w.g.candPrev[c] = (l < prevCount && w.prev.key[l] == k && w.prev.count[l] > 0) ? l : -1;
-    w.cur.key[c] = k;
-  }
-}
-
 }  // namespace
 
-size_t broadphase_temp_bytes(int n, int tableSize) {
-  size_t a = 0, b = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, a, (int *)nullptr, (int *)nullptr, tableSize);
-  cub::DeviceScan::ExclusiveSum(nullptr, b, (int *)nullptr, (int *)nullptr, n + 1);
-  return a > b ? a : b;
-}
+int pair_ranges_max(int n) { return n / kWarpsPerBlock + 2; }
 
-void launch_broadphase_impl(const World &w, int numLarge, void *temp, size_t tempBytes, cudaStream_t st,
-                            int smCount) {
+void launch_broadphase_impl(const World &w, int numLarge, cudaStream_t st, int smCount) {
   const int T = (int)w.g.tableMask + 1;
-  const int n = w.b.n;
   const int blocks = smCount * 4;
-  cudaMemsetAsync(w.g.tableCount, 0, sizeof(int) * T, st);
+  const PairRanges R = pair_ranges(w.b.n, smCount);
+  const int grid = R.blocks + numLarge * w.g.maxChunks;
+  cudaMemsetAsync(w.g.table, 0, sizeof(int2) * T, st);
   cells_kernel<<<blocks, 256, 0, st>>>(w);
-  size_t tb = tempBytes;
-  cub::DeviceScan::ExclusiveSum(temp, tb, w.g.tableCount, w.g.tableStart, T, st);
-  cudaMemcpyAsync(w.g.tableCursor, w.g.tableStart, sizeof(int) * T, cudaMemcpyDeviceToDevice, st);
+  bucket_kernel<<<blocks, 256, 0, st>>>(w);
   scatter_kernel<<<blocks, 256, 0, st>>>(w);
-  // pairCount[n] = 0 so the scan over n + 1 entries yields the total at [n]
-  cudaMemsetAsync(w.g.pairCount + n, 0, sizeof(int), st);
-  const int warpBlocks = (int)std::min<long long>(((long long)n + 7) / 8, (long long)smCount * 32);
-  pairs_kernel<kPairScratch><<<warpBlocks, 256, 0, st>>>(w);
-  if (numLarge > 0) {
-    large_count_kernel<<<dim3(w.g.maxChunks, numLarge), 256, 0, st>>>(w);
-    large_total_kernel<<<numLarge, 32, 0, st>>>(w);
-  }
-  tb = tempBytes;
-  cub::DeviceScan::ExclusiveSum(temp, tb, w.g.pairCount, w.g.pairStart, n + 1, st);
-  copy_kernel<kPairScratch><<<warpBlocks, 256, 0, st>>>(w);
-  if (numLarge > 0) {
-    large_write_kernel<<<dim3(w.g.maxChunks, numLarge), 256, 0, st>>>(w);
-    large_extra_kernel<<<numLarge, 32, 0, st>>>(w);
-  }
-  finish_kernel<<<1, 1, 0, st>>>(w);
-  prev_index_kernel<<<blocks, 256, 0, st>>>(w);
+  pairs_kernel<kPairScratch><<<grid, 256, 0, st>>>(w, R.blocks, R.per);
+  if (numLarge > 0) large_total_kernel<<<numLarge, 256, 0, st>>>(w, R.per);
+  copy_kernel<kPairScratch><<<grid, 256, 0, st>>>(w, R.blocks, R.per);
+  finish_kernel<<<std::max(numLarge, 1), 256, 0, st>>>(w, numLarge);
 }
 
 }  // namespace avbd
@@ -509,8 +604,8 @@ namespace {
 
 // Where the query's arrays sit in the scratch array, for n bodies.
 struct StaticLayout {
-  size_t pos, size, massD, flags0, scene, cStart, cellLo, loc, cellF, entries, rows, pairCount, pairStart, largeList,
-      largeStart, sceneStart, invCell, tableCount, tableStart, tableCursor, ctl, temp, tempBytes, total;
+  size_t pos, size, massD, flags0, scene, cStart, cellLo, loc, cellF, entryId, entryLoc, rows, pairCount, pairStart, largeList,
+      largeStart, sceneStart, invCell, table, rank, rangeSum, ctl, total;
   int tableSize;
 };
 
@@ -535,7 +630,8 @@ StaticLayout static_layout(int n) {
   L.cellLo = take(m * sizeof(int4));
   L.loc = take(m * sizeof(float4));
   L.cellF = take(sizeof(float));
-  L.entries = take(m * sizeof(Entry));
+  L.entryId = take(m * sizeof(int4));
+  L.entryLoc = take(m * sizeof(float4));
   L.rows = take(m * kStaticPairRow * sizeof(uint32_t));
   L.pairCount = take((m + 1) * sizeof(int));
   L.pairStart = take((m + 1) * sizeof(int));
@@ -543,20 +639,22 @@ StaticLayout static_layout(int n) {
   L.largeStart = take(2 * sizeof(int));
   L.sceneStart = take(2 * sizeof(int));
   L.invCell = take(sizeof(double));
-  L.tableCount = take((size_t)T * sizeof(int));
-  L.tableStart = take((size_t)T * sizeof(int));
-  L.tableCursor = take((size_t)T * sizeof(int));
+  L.table = take((size_t)T * sizeof(int2));
+  L.rank = take(m * sizeof(int));
+  L.rangeSum = take((size_t)pair_ranges_max((int)m) * sizeof(int));
   L.ctl = take(sizeof(Control));
-  L.tempBytes = broadphase_temp_bytes((int)m, T);
-  L.temp = take(L.tempBytes);
   L.total = at;
   return L;
 }
 
-// Caller inputs -> the step's body layout. Bodies whose diameter (padded as
-// the context's pack pads its cell) exceeds the cell are "large".
+// Caller inputs -> the step's body layout, and the scene table's scalars.
+// Bodies whose diameter (padded as the context's pack pads its cell) exceeds
+// the cell are "large", listed in any order (a body's partners are sorted
+// afterwards).
 __global__ void static_stage_kernel(World w, D4 *pos, D4 *size, D4 *massD, int *flags0, int *scene, int *cStart,
-                                    const double *p, const double *radius, const int32_t *dynamic, double cell) {
+                                    int *largeList, int *largeStart, int *sceneStart, double *invCell, float *cellF,
+                                    const double *p, const double *radius, const int32_t *dynamic, double cell,
+                                    double inv) {
   const int n = w.b.n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double r = radius[i];
@@ -568,37 +666,20 @@ __global__ void static_stage_kernel(World w, D4 *pos, D4 *size, D4 *massD, int *
     flags0[i] = (dyn ? kBodyDynamic : 0) | (large ? kBodyLarge : 0);
     scene[i] = 0;
     cStart[i] = 0;
+    if (large) largeList[atomicAdd(&largeStart[1], 1)] = i;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cStart[n] = 0;
-}
-
-// Large bodies in ascending index order (one block).
-__global__ void __launch_bounds__(1024) static_large_list_kernel(World w, int *largeList, int *largeStart) {
-  typedef cub::BlockScan<int, 1024> S;
-  __shared__ typename S::TempStorage tmp;
-  __shared__ int base;
-  if (threadIdx.x == 0) base = 0;
-  __syncthreads();
-  const int n = w.b.n;
-  for (int i0 = 0; i0 < n; i0 += 1024) {
-    const int i = i0 + threadIdx.x;
-    const int f = (i < n && is_large(w, i)) ? 1 : 0;
-    int at, tot;
-    S(tmp).ExclusiveSum(f, at, tot);
-    if (f) largeList[base + at] = i;
-    __syncthreads();
-    if (threadIdx.x == 0) base += tot;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    largeStart[0] = 0;
-    largeStart[1] = base;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    cStart[n] = 0;
+    sceneStart[0] = 0;
+    sceneStart[1] = n;
+    invCell[0] = inv;
+    cellF[0] = (float)(1.0 / inv);
   }
 }
 
-// large_count_kernel / large_write_kernel with the large-body count read on
-// the device and no previous manifolds.
-__global__ void static_large_count_kernel(World w) {
+// The large bodies' counts and segments with the large-body count read on the
+// device and no previous manifolds.
+__global__ void static_large_count_kernel(World w, int per) {
   const int numLarge = w.g.largeStart[1];
   typedef cub::BlockReduce<int, 256> R;
   __shared__ typename R::TempStorage tmp;
@@ -607,7 +688,10 @@ __global__ void static_large_count_kernel(World w) {
     int c = 0;
     for (int b = threadIdx.x; b < a; b += blockDim.x) c += accept(w, a, b) ? 1 : 0;
     const int total = R(tmp).Sum(c);
-    if (threadIdx.x == 0) w.g.pairCount[a] = total;
+    if (threadIdx.x == 0) {
+      w.g.pairCount[a] = total;
+      atomicAdd(&w.g.rangeSum[a / per], total);
+    }
     __syncthreads();
   }
 }
@@ -638,13 +722,6 @@ __global__ void static_large_write_kernel(World w) {
       __syncthreads();
     }
   }
-}
-
-__global__ void static_scalars_kernel(int *sceneStart, double *invCell, float *cellF, int n, double inv) {
-  sceneStart[0] = 0;
-  sceneStart[1] = n;
-  invCell[0] = inv;
-  cellF[0] = (float)(1.0 / inv);
 }
 
 __global__ void static_finish_kernel(World w, int32_t *count) {
@@ -737,10 +814,11 @@ extern "C" int avbd_overlap_pairs_static(int32_t n, const double *pos, const dou
   w.g.loc = (float4 *)(base + L.loc);
   w.g.cellF = (const float *)(base + L.cellF);
   w.g.tableMask = (unsigned)(L.tableSize - 1);
-  w.g.tableCount = (int *)(base + L.tableCount);
-  w.g.tableStart = (int *)(base + L.tableStart);
-  w.g.tableCursor = (int *)(base + L.tableCursor);
-  w.g.entries = (Entry *)(base + L.entries);
+  w.g.table = (int2 *)(base + L.table);
+  w.g.rank = (int *)(base + L.rank);
+  w.g.rangeSum = (int *)(base + L.rangeSum);
+  w.g.entryId = (int4 *)(base + L.entryId);
+  w.g.entryLoc = (float4 *)(base + L.entryLoc);
   w.g.entryCap = n;
   w.g.scratch = (uint32_t *)(base + L.rows);
   w.g.hasConstraints = 0;
@@ -754,31 +832,23 @@ extern "C" int avbd_overlap_pairs_static(int32_t n, const double *pos, const dou
   int smCount = 0;
   e = cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) {
-    // zero what the kernels accumulate into; the scene table and cell size
-    const int sceneStart[2] = {0, n};
-    const double inv = 1.0 / cell_size;
+    // zero what the kernels accumulate into
     cudaMemsetAsync(w.ctl, 0, sizeof(Control), st);
-    cudaMemsetAsync(w.g.tableCount, 0, sizeof(int) * L.tableSize, st);
-    cudaMemsetAsync(w.g.pairCount + n, 0, sizeof(int), st);
+    cudaMemsetAsync(base + L.largeStart, 0, 2 * sizeof(int), st);
+    cudaMemsetAsync(w.g.table, 0, sizeof(int2) * L.tableSize, st);
     const int blocks = smCount * 4;
-    static_stage_kernel<<<blocks, 256, 0, st>>>(w, dPos, dSize, dMass, dFlags, dScene, dCStart, pos, radius,
-                                                dynamic, cell_size);
-    // two scalars and the inverse cell: written by a one-thread kernel so the
-    // call needs no host staging buffer
-    static_scalars_kernel<<<1, 1, 0, st>>>((int *)(base + L.sceneStart), (double *)(base + L.invCell),
-                                           (float *)(base + L.cellF), sceneStart[1], inv);
-    static_large_list_kernel<<<1, 1024, 0, st>>>(w, (int *)(base + L.largeList), (int *)(base + L.largeStart));
+    const PairRanges R = pair_ranges(n, smCount);
+    static_stage_kernel<<<blocks, 256, 0, st>>>(w, dPos, dSize, dMass, dFlags, dScene, dCStart,
+                                                (int *)(base + L.largeList), (int *)(base + L.largeStart),
+                                                (int *)(base + L.sceneStart), (double *)(base + L.invCell),
+                                                (float *)(base + L.cellF), pos, radius, dynamic, cell_size,
+                                                1.0 / cell_size);
     cells_kernel<<<blocks, 256, 0, st>>>(w);
-    size_t tb = L.tempBytes;
-    cub::DeviceScan::ExclusiveSum(base + L.temp, tb, w.g.tableCount, w.g.tableStart, L.tableSize, st);
-    cudaMemcpyAsync(w.g.tableCursor, w.g.tableStart, sizeof(int) * L.tableSize, cudaMemcpyDeviceToDevice, st);
+    bucket_kernel<<<blocks, 256, 0, st>>>(w);
     scatter_kernel<<<blocks, 256, 0, st>>>(w);
-    const int warpBlocks = (int)std::min<long long>(((long long)n + 7) / 8, (long long)smCount * 32);
-    pairs_kernel<kStaticPairRow><<<warpBlocks, 256, 0, st>>>(w);
-    static_large_count_kernel<<<smCount, 256, 0, st>>>(w);
-    tb = L.tempBytes;
-    cub::DeviceScan::ExclusiveSum(base + L.temp, tb, w.g.pairCount, w.g.pairStart, n + 1, st);
-    copy_kernel<kStaticPairRow><<<warpBlocks, 256, 0, st>>>(w);
+    pairs_kernel<kStaticPairRow><<<R.blocks, 256, 0, st>>>(w, R.blocks, R.per);
+    static_large_count_kernel<<<smCount, 256, 0, st>>>(w, R.per);
+    copy_kernel<kStaticPairRow><<<R.blocks, 256, 0, st>>>(w, R.blocks, R.per);
     static_large_write_kernel<<<smCount, 256, 0, st>>>(w);
     static_finish_kernel<<<1, 1, 0, st>>>(w, count);
     e = cudaGetLastError();

@@ -57,8 +57,8 @@ struct avbd_ctx {
   int n = 0, nj = 0, ns = 0, numScenes = 1, numLarge = 0;
   int candCap = 0, entryCap = 0, tableSize = 0, adjCap = 0, colorBlocks = 0;
   int lanes = 8, blocksPerSm = 1;
-  size_t bpTempBytes = 0, svTempBytes = 0;
-  void *bpTemp = nullptr, *svTemp = nullptr;
+  size_t svTempBytes = 0;
+  void *svTemp = nullptr;
   double *statsOut = nullptr;
   World w{};
   Manifolds mA{}, mB{};
@@ -492,11 +492,11 @@ void invalidate_graphs(avbd_ctx *ctx) {
 int enqueue_step(avbd_ctx *ctx) {
   World &w = ctx->w;
   cudaStream_t st = ctx->stream;
-  // per-step counters: numCandidates .. adjTotal
+  // per-step counters: numCandidates .. gridEntries
   CK(cudaMemsetAsync(&w.ctl->numCandidates, 0, sizeof(int) * 7, st));
   int rc;
   if ((rc = record(ctx, 0))) return rc;
-  launch_broadphase_impl(w, ctx->numLarge, ctx->bpTemp, ctx->bpTempBytes, st, ctx->smCount);
+  launch_broadphase_impl(w, ctx->numLarge, st, ctx->smCount);
   if ((rc = record(ctx, 1))) return rc;
   launch_narrowphase(w, st, ctx->smCount);
   if ((rc = record(ctx, 2))) return rc;
@@ -513,11 +513,11 @@ int enqueue_step(avbd_ctx *ctx) {
   return record(ctx, 6);
 }
 
-// Own kernels of one step: broad phase 6 (+4 with large bodies; its two scans
-// are library code), narrow phase 4, prepare 5, colouring 1 (+2 with an
+// Own kernels of one step: broad phase 6 (+1 with large bodies), narrow phase
+// 4, prepare 5 (its two scans are library code), colouring 1 (+2 with an
 // uploaded colouring), solve 1, commit 1.
 int step_kernels(const avbd_ctx *ctx) {
-  return 6 + (ctx->numLarge > 0 ? 4 : 0) + 4 + 5 + 1 + (ctx->w.a.colorOverride ? 2 : 0) + 1 + 1;
+  return 6 + (ctx->numLarge > 0 ? 1 : 0) + 4 + 5 + 1 + (ctx->w.a.colorOverride ? 2 : 0) + 1 + 1;
 }
 
 // One step as a CUDA graph (captured on first use for this arena parity).
@@ -1098,8 +1098,10 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   w.g.entryCap = ctx->entryCap;
   w.g.candCap = ctx->candCap;
   if ((rc = dalloc(ctx, &w.g.cellLo, n)) || (rc = dalloc(ctx, &w.g.loc, n)) ||
-      (rc = dalloc(ctx, &w.g.tableCount, ctx->tableSize)) || (rc = dalloc(ctx, &w.g.tableStart, ctx->tableSize)) ||
-      (rc = dalloc(ctx, &w.g.tableCursor, ctx->tableSize)) || (rc = dalloc(ctx, &w.g.entries, ctx->entryCap)) ||
+      (rc = dalloc(ctx, &w.g.table, ctx->tableSize)) ||
+      (rc = dalloc(ctx, &w.g.rank, n)) || (rc = dalloc(ctx, &w.g.prevStart, n + 1)) ||
+      (rc = dalloc(ctx, &w.g.rangeSum, pair_ranges_max(n))) || (rc = dalloc(ctx, &w.g.entryId, ctx->entryCap)) ||
+      (rc = dalloc(ctx, &w.g.entryLoc, ctx->entryCap)) ||
       (rc = dalloc(ctx, &w.g.pairCount, n + 1)) || (rc = dalloc(ctx, &w.g.pairStart, n + 1)) ||
       (rc = dalloc(ctx, &w.g.scratch, (size_t)n * kPairScratch)))
     return rc;
@@ -1128,10 +1130,8 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
     return rc;
   CK(launch_set_grab(w, -1, nullptr, nullptr, 0.0, ctx->stream));  // nothing grabbed
   // scratch of the scans
-  ctx->bpTempBytes = broadphase_temp_bytes(n, ctx->tableSize);
   ctx->svTempBytes = solver_temp_bytes(n);
-  if ((rc = dalloc(ctx, (char **)&ctx->bpTemp, ctx->bpTempBytes)) || (rc = dalloc(ctx, (char **)&ctx->svTemp, ctx->svTempBytes)))
-    return rc;
+  if ((rc = dalloc(ctx, (char **)&ctx->svTemp, ctx->svTempBytes))) return rc;
   // launch shape of the persistent solve
   const int maxPerSm = solve_max_blocks_per_sm(ctx->lanes);
   ctx->autoLanes = P.lanes_per_body <= 0;

@@ -776,7 +776,21 @@ __device__ int exact_best_face(const BodyD &A, const BodyD &B, int mask) {
   return best;
 }
 
-// 1. Every candidate: the f32 SAT. Separated pairs get count 0; box pairs
+// The candidate's slot among the previous step's manifolds, searched in its
+// body A's run of them (-1: none with contacts).
+__device__ __forceinline__ int previous_slot(const World &w, uint64_t key, int a) {
+  if (w.ctl->prevCandidates <= 0) return -1;
+  const int end = w.g.prevStart[a + 1];
+  int l = w.g.prevStart[a], h = end;
+  while (l < h) {
+    const int m = (l + h) >> 1;
+    if (w.prev.key[m] < key) l = m + 1;
+    else h = m;
+  }
+  return l < end && w.prev.key[l] == key && w.prev.count[l] > 0 ? l : -1;
+}
+
+// 1. Every candidate: its previous manifold, and the f32 SAT. Separated pairs get count 0; box pairs
 //    with a certain winning axis go to the face or edge list, everything
 //    else (sphere pairs, undecided box pairs) to the exact list.
 __global__ void __launch_bounds__(256) classify_kernel(World w) {
@@ -784,6 +798,8 @@ __global__ void __launch_bounds__(256) classify_kernel(World w) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
     const uint64_t key = w.g.candKey[c];
     const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
+    w.g.candPrev[c] = previous_slot(w, key, ia);
+    w.cur.key[c] = key;
     const BodyD A = load_body(w, ia), B = load_body(w, ib);
     // spheres, and pairs with a contact skin (speculative contacts: the f32
     // certification covers the skin-free tests), go to the exact collider
