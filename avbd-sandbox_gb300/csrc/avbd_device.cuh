@@ -28,6 +28,7 @@ constexpr int kMaxContacts = 8;
 // (largest number of dynamic neighbours of a body) + 1; per-colour loops run
 // over the colours in use only.
 constexpr int kMaxColors = 1024;
+constexpr int kAdjRun = 128;        // bodies of a run of Adjacency::runCount
 constexpr int kLaneBuckets = 8;     // log2 of the lanes of a body's group: 0..7
 constexpr int kLaneMaxGroup = 128;  // largest group: one solve block
 
@@ -224,14 +225,15 @@ struct Grid {
 
 struct Adjacency {
   int *start;   // n + 1
-  int *count;   // n
   int *cursor;  // n
+  // per body its manifolds (low word) and contacts (high), and their sums over
+  // runs of kAdjRun bodies
+  unsigned long long *count, *runCount;
   uint32_t *entry;  // (manifold << 1) | side
   int cap;
   // per-contact adjacency of dynamic bodies: (slot << 1 | side, other body),
   // slot = manifold * 8 + contact; in manifold order, then contact order
   int *cstart;   // n + 1
-  int *ccount;   // n
   int2 *centry;
   int ccap;
   int *hpEntry;      // per body, within its manifold range: dynamic neighbours of higher colouring priority
@@ -409,8 +411,7 @@ __host__ __device__ inline uint32_t color_priority(uint32_t x) {
 int pair_ranges_max(int n);  // entries of Grid::rangeSum
 void launch_broadphase_impl(const World &w, int numLarge, cudaStream_t st, int smCount);
 void launch_narrowphase(const World &w, cudaStream_t st, int smCount);
-size_t solver_temp_bytes(int n);
-void launch_prepare(const World &w, void *temp, size_t tempBytes, cudaStream_t st, int smCount);
+void launch_prepare(const World &w, cudaStream_t st, int smCount);
 cudaError_t launch_coloring(const World &w, cudaStream_t st, int blocks);
 int coloring_grid(int smCount);  // blocks of the cooperative colouring launch
 cudaError_t launch_solve(const World &w, int lanesPerBody, int blocksPerSm, cudaStream_t st, int smCount);

@@ -57,8 +57,6 @@ struct avbd_ctx {
   int n = 0, nj = 0, ns = 0, numScenes = 1, numLarge = 0;
   int candCap = 0, entryCap = 0, tableSize = 0, adjCap = 0, colorBlocks = 0;
   int lanes = 8, blocksPerSm = 1;
-  size_t svTempBytes = 0;
-  void *svTemp = nullptr;
   double *statsOut = nullptr;
   World w{};
   Manifolds mA{}, mB{};
@@ -500,7 +498,7 @@ int enqueue_step(avbd_ctx *ctx) {
   if ((rc = record(ctx, 1))) return rc;
   launch_narrowphase(w, st, ctx->smCount);
   if ((rc = record(ctx, 2))) return rc;
-  launch_prepare(w, ctx->svTemp, ctx->svTempBytes, st, ctx->smCount);
+  launch_prepare(w, st, ctx->smCount);
   if ((rc = record(ctx, 3))) return rc;
   CK(launch_coloring(w, st, ctx->colorBlocks));
   if ((rc = record(ctx, 4))) return rc;
@@ -514,10 +512,10 @@ int enqueue_step(avbd_ctx *ctx) {
 }
 
 // Own kernels of one step: broad phase 6 (+1 with large bodies), narrow phase
-// 4, prepare 5 (its two scans are library code), colouring 1 (+2 with an
+// 4, prepare 5 (+1 with joints or springs), colouring 1 (+2 with an
 // uploaded colouring), solve 1, commit 1.
 int step_kernels(const avbd_ctx *ctx) {
-  return 6 + (ctx->numLarge > 0 ? 1 : 0) + 4 + 5 + 1 + (ctx->w.a.colorOverride ? 2 : 0) + 1 + 1;
+  return 6 + (ctx->numLarge > 0 ? 1 : 0) + 4 + 5 + (ctx->nj + ctx->ns > 0 ? 1 : 0) + 1 + (ctx->w.a.colorOverride ? 2 : 0) + 1 + 1;
 }
 
 // One step as a CUDA graph (captured on first use for this arena parity).
@@ -1109,10 +1107,10 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   // adjacency + colouring
   w.a.cap = ctx->adjCap;
   ctx->colorBlocks = std::max(1, coloring_grid(ctx->smCount));
-  if ((rc = dalloc(ctx, &w.a.start, n + 1)) || (rc = dalloc(ctx, &w.a.count, n + 1)) ||
+  if ((rc = dalloc(ctx, &w.a.start, n + 1)) || (rc = dalloc(ctx, &w.a.count, n)) ||
+      (rc = dalloc(ctx, &w.a.runCount, n / kAdjRun + 1)) ||
       (rc = dalloc(ctx, &w.a.hpCount, n)) ||
       (rc = dalloc(ctx, &w.a.cursor, n + 1)) || (rc = dalloc(ctx, &w.a.cstart, n + 1)) ||
-      (rc = dalloc(ctx, &w.a.ccount, n + 1)) ||
       (rc = dalloc(ctx, &w.a.colorStart, kMaxColors + 1)) || (rc = dalloc(ctx, &w.a.colorBodies, n)) ||
       (rc = dalloc(ctx, &w.a.colorRec, n)) ||
       (rc = dalloc(ctx, &w.a.blockHist, (size_t)ctx->colorBlocks * kMaxColors)) ||
@@ -1129,9 +1127,6 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   if ((rc = dalloc(ctx, &w.ctl, 1)) || (rc = dalloc(ctx, &ctx->statsOut, 3)) || (rc = dalloc(ctx, &w.grab, 1)))
     return rc;
   CK(launch_set_grab(w, -1, nullptr, nullptr, 0.0, ctx->stream));  // nothing grabbed
-  // scratch of the scans
-  ctx->svTempBytes = solver_temp_bytes(n);
-  if ((rc = dalloc(ctx, (char **)&ctx->svTemp, ctx->svTempBytes))) return rc;
   // launch shape of the persistent solve
   const int maxPerSm = solve_max_blocks_per_sm(ctx->lanes);
   ctx->autoLanes = P.lanes_per_body <= 0;

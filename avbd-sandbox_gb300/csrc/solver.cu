@@ -276,8 +276,8 @@ __global__ void prepare_bodies_kernel(World w) {
       w.b.dang[i] = make_float4(da.x, da.y, da.z, 0.f);
     }
     w.b.flags[i] = fl;
-    w.a.count[i] = 0;
-    w.a.ccount[i] = 0;
+    w.a.count[i] = 0ull;
+    if (i % kAdjRun == 0) w.a.runCount[i / kAdjRun] = 0ull;
     w.b.progress[i] = 0;
   }
 }
@@ -290,22 +290,55 @@ __device__ inline bool precedes(const World &w, int j, int i) {
 
 __global__ void adj_count_kernel(World w) {
   const int total = w.ctl->numCandidates;
+  int live = 0, contacts = 0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
     const int n = w.cur.count[c];
     if (n <= 0) continue;
     const uint64_t k = w.cur.key[c];
-    const int a = (int)(k >> 32), b = (int)(k & 0xffffffffu);
-    if (w.b.flags0[a] & kBodyDynamic) {
-      atomicAdd(&w.a.count[a], 1);
-      atomicAdd(&w.a.ccount[a], n);
+    const unsigned long long one = 1ull | (unsigned long long)n << 32;
+    for (int side = 0; side < 2; side++) {
+      const int i = side ? (int)(k & 0xffffffffu) : (int)(k >> 32);
+      if (!(w.b.flags0[i] & kBodyDynamic)) continue;
+      atomicAdd(&w.a.count[i], one);
+      atomicAdd(&w.a.runCount[i / kAdjRun], one);
     }
-    if (w.b.flags0[b] & kBodyDynamic) {
-      atomicAdd(&w.a.count[b], 1);
-      atomicAdd(&w.a.ccount[b], n);
-    }
-    atomicAdd(&w.ctl->liveManifolds, 1);
-    atomicAdd(&w.ctl->liveContacts, n);
+    live++;
+    contacts += n;
   }
+  __syncwarp();
+  live = __reduce_add_sync(0xffffffffu, live);
+  contacts = __reduce_add_sync(0xffffffffu, contacts);
+  if ((threadIdx.x & 31) == 0 && live) {
+    atomicAdd(&w.ctl->liveManifolds, live);
+    atomicAdd(&w.ctl->liveContacts, contacts);
+  }
+}
+
+// Where each body's manifolds and contacts start: a block sums the runs
+// before its bodies, then scans their counts.
+__global__ void __launch_bounds__(256) adj_scan_kernel(World w) {
+  typedef unsigned long long U;
+  typedef cub::BlockReduce<U, 256> R;
+  typedef cub::BlockScan<U, 256> S;
+  __shared__ union {
+    typename R::TempStorage r;
+    typename S::TempStorage s;
+  } tmp;
+  __shared__ U base;
+  static_assert(256 % kAdjRun == 0, "a block's bodies begin a run");
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  U v = 0;
+  for (int k = threadIdx.x; k < (int)blockIdx.x * (256 / kAdjRun); k += 256) v += w.a.runCount[k];
+  v = R(tmp.r).Sum(v);
+  if (threadIdx.x == 0) base = v;
+  __syncthreads();
+  U at;
+  S(tmp.s).ExclusiveSum(i < w.b.n ? w.a.count[i] : 0ull, at);
+  at += base;
+  if (i > w.b.n) return;
+  w.a.start[i] = (int)(at & 0xffffffffu);
+  w.a.cstart[i] = (int)(at >> 32);
+  if (i < w.b.n) w.a.cursor[i] = (int)(at & 0xffffffffu);
 }
 
 __global__ void adj_fill_kernel(World w) {
@@ -327,66 +360,106 @@ __global__ void adj_fill_kernel(World w) {
   }
 }
 
-// Sort each body's manifold list (determinism) and decide its precision.
-__global__ void adj_sort_kernel(World w) {
+// Sort each body's manifold list (determinism), list its contacts and decide
+// its precision: eight lanes a body (a rank sort in shared memory, the
+// contacts' places by a scan over the lanes). A thread a body took 255 us of
+// a crushed pyramid's step: an insertion sort of 30 to 100 entries in global
+// memory each, and of some 200 for the sphere that everything waited for.
+constexpr int kSortRow = 96;  // entries sorted in shared memory; more: from a copy in the body's hpEntry range
+__global__ void __launch_bounds__(256) adj_sort_kernel(World w) {
   if (step_skipped(w)) return;
+  __shared__ uint32_t row[32][kSortRow];
   const double dt2 = w.p.dt * w.p.dt;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.b.n; i += gridDim.x * blockDim.x) {
-    int fl = w.b.flags[i];
-    if (!(fl & kBodyDynamic)) continue;
-    int beg = w.a.start[i], end = w.a.start[i + 1];
-    if (end > w.a.cap) end = w.a.cap;
-    uint32_t *e = w.a.entry;
-    for (int x = beg + 1; x < end; x++) {
-      const uint32_t v = e[x];
-      int y = x - 1;
-      while (y >= beg && e[y] > v) {
-        e[y + 1] = e[y];
-        y--;
-      }
-      e[y + 1] = v;
+  const int gl = threadIdx.x & 7, group = threadIdx.x >> 3, shift = threadIdx.x & 24;
+  uint32_t *e = w.a.entry;
+  for (int i0 = blockIdx.x * 32; i0 < w.b.n; i0 += gridDim.x * 32) {
+    const int i = i0 + group;
+    int fl = i < w.b.n ? w.b.flags[i] : 0;
+    const bool dyn = (fl & kBodyDynamic) != 0;
+    int beg = 0, end = 0, at = 0, cend = 0;
+    if (dyn) {
+      beg = w.a.start[i];
+      end = min(w.a.start[i + 1], w.a.cap);
+      at = w.a.cstart[i];
+      cend = min(w.a.cstart[i + 1], w.a.ccap);
     }
+    const int n = max(end - beg, 0);
+    // entries are distinct: each goes to the number of smaller ones
+    if (n <= kSortRow) {
+      for (int x = gl; x < n; x += 8) row[group][x] = e[beg + x];
+      __syncwarp(0xffu << shift);
+      for (int x = gl; x < n; x += 8) {
+        const uint32_t v = row[group][x];
+        int r = 0;
+        for (int y = 0; y < n; y++) r += row[group][y] < v ? 1 : 0;
+        e[beg + r] = v;
+      }
+    } else {
+      uint32_t *copy = reinterpret_cast<uint32_t *>(w.a.hpEntry);  // the body's range there is written below
+      for (int x = gl; x < n; x += 8) copy[beg + x] = e[beg + x];
+      __syncwarp(0xffu << shift);
+      for (int x = gl; x < n; x += 8) {
+        const uint32_t v = copy[beg + x];
+        int r = 0;
+        for (int y = 0; y < n; y++) r += copy[beg + y] < v ? 1 : 0;
+        e[beg + r] = v;
+      }
+    }
+    __syncwarp();
     // per-contact adjacency, in manifold order then contact order; and the
     // dynamic neighbours of higher colouring priority (the only ones a
     // colouring round reads), stored in the body's own manifold range
-    {
-      int at = w.a.cstart[i];
-      const int cend = min(w.a.cstart[i + 1], w.a.ccap);
-      int hc = 0;
-      for (int x = beg; x < end; x++) {
-        const uint32_t v = e[x];
-        const int m = (int)(v >> 1), side = (int)(v & 1u);
+    int hc = 0;
+    const int most = __reduce_max_sync(0xffffffffu, n);
+    for (int x0 = 0; x0 < most; x0 += 8) {
+      const int x = x0 + gl;
+      int m = 0, side = 0, other = 0, cnt = 0;
+      bool higher = false;
+      if (x < n) {
+        const uint32_t v = e[beg + x];
+        m = (int)(v >> 1);
+        side = (int)(v & 1u);
         const uint64_t key = w.cur.key[m];
-        const int other = side ? (int)(key >> 32) : (int)(key & 0xffffffffu);
-        const int cnt = w.cur.count[m];
-        for (int k = 0; k < cnt && at < cend; k++, at++)
-          w.a.centry[at] = make_int2(((m * kMaxContacts + k) << 2) | side, other);  // owner bit set after colouring
-        if ((w.b.flags0[other] & kBodyDynamic) && precedes(w, other, i)) w.a.hpEntry[beg + hc++] = other;
+        other = side ? (int)(key >> 32) : (int)(key & 0xffffffffu);
+        cnt = w.cur.count[m];
+        higher = (w.b.flags0[other] & kBodyDynamic) && precedes(w, other, i);
       }
-      w.a.hpCount[i] = hc;
+      int incl = cnt;
+#pragma unroll
+      for (int d = 1; d < 8; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d, 8);
+        if (gl >= d) incl += v;
+      }
+      const int first = at + incl - cnt;
+      for (int k = 0; k < cnt && first + k < cend; k++)
+        w.a.centry[first + k] = make_int2(((m * kMaxContacts + k) << 2) | side, other);  // owner bit set after colouring
+      at += __shfl_sync(0xffffffffu, incl, 7, 8);
+      const unsigned hm = (__ballot_sync(0xffffffffu, higher) >> shift) & 0xffu;
+      if (higher) w.a.hpEntry[beg + hc + __popc(hm & ((1u << gl) - 1u))] = other;
+      hc += __popc(hm);
     }
-    if (w.p.fp64Ratio > 0) {
-      double kmax = 0;
-      for (int k = w.g.cStart[i]; k < w.g.cStart[i + 1]; k++) {
-        const uint32_t ref = w.g.cRef[k];
-        const uint32_t type = ref >> 30, idx = (ref >> 1) & 0x1fffffffu;
-        if (type == kRefJoint) {
-          if (w.j.state[idx]) continue;
-          const float4 kl = w.j.penLin[idx];
-          const double hard = isinf(w.j.stiff[idx].x) ? w.p.penaltyMax : 0.0;
-          kmax = fmax(kmax, fmax(fmax((double)kl.x, (double)kl.y), fmax((double)kl.z, hard)));
-        } else {
-          if (w.s.state[idx]) continue;
-          kmax = fmax(kmax, (double)w.s.penalty[idx]);
-        }
-      }
-      const double inertial = w.b.massD[i].x / dt2;
-      if (kmax > w.p.fp64Ratio * inertial) {
-        fl |= kBodyFp64;
-        atomicAdd(&w.ctl->fp64Bodies, 1);
+    if (!dyn || gl != 0) continue;
+    w.a.hpCount[i] = hc;
+    if (!w.p.mayFp64) continue;
+    double kmax = 0;
+    for (int k = w.g.cStart[i]; k < w.g.cStart[i + 1]; k++) {
+      const uint32_t ref = w.g.cRef[k];
+      const uint32_t type = ref >> 30, idx = (ref >> 1) & 0x1fffffffu;
+      if (type == kRefJoint) {
+        if (w.j.state[idx]) continue;
+        const float4 kl = w.j.penLin[idx];
+        const double hard = isinf(w.j.stiff[idx].x) ? w.p.penaltyMax : 0.0;
+        kmax = fmax(kmax, fmax(fmax((double)kl.x, (double)kl.y), fmax((double)kl.z, hard)));
+      } else {
+        if (w.s.state[idx]) continue;
+        kmax = fmax(kmax, (double)w.s.penalty[idx]);
       }
     }
-    w.b.flags[i] = fl;
+    const double inertial = w.b.massD[i].x / dt2;
+    if (kmax > w.p.fp64Ratio * inertial) {
+      w.b.flags[i] = fl | kBodyFp64;
+      atomicAdd(&w.ctl->fp64Bodies, 1);
+    }
   }
 }
 
@@ -2223,24 +2296,12 @@ __global__ void stats_kernel(World w, double *out) {
 
 }  // namespace
 
-size_t solver_temp_bytes(int n) {
-  size_t a = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, a, (int *)nullptr, (int *)nullptr, n + 1);
-  return a;
-}
-
-void launch_prepare(const World &w, void *temp, size_t tempBytes, cudaStream_t st, int smCount) {
+void launch_prepare(const World &w, cudaStream_t st, int smCount) {
   const int blocks = smCount * 4;
-  prepare_forces_kernel<<<blocks, 256, 0, st>>>(w);
+  if (w.j.n + w.s.n > 0) prepare_forces_kernel<<<blocks, 256, 0, st>>>(w);
   prepare_bodies_kernel<<<blocks, 256, 0, st>>>(w);
-  cudaMemsetAsync(w.a.count + w.b.n, 0, sizeof(int), st);
-  cudaMemsetAsync(w.a.ccount + w.b.n, 0, sizeof(int), st);
   adj_count_kernel<<<blocks, 256, 0, st>>>(w);
-  size_t tb = tempBytes;
-  cub::DeviceScan::ExclusiveSum(temp, tb, w.a.count, w.a.start, w.b.n + 1, st);
-  tb = tempBytes;
-  cub::DeviceScan::ExclusiveSum(temp, tb, w.a.ccount, w.a.cstart, w.b.n + 1, st);
-  cudaMemcpyAsync(w.a.cursor, w.a.start, sizeof(int) * w.b.n, cudaMemcpyDeviceToDevice, st);
+  adj_scan_kernel<<<w.b.n / 256 + 1, 256, 0, st>>>(w);
   adj_fill_kernel<<<blocks, 256, 0, st>>>(w);
   adj_sort_kernel<<<blocks, 256, 0, st>>>(w);
 }
