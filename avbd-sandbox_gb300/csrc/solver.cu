@@ -1134,7 +1134,10 @@ __device__ __forceinline__ ContactEval<T> eval_contact(const V3<T> n[3], T mu, f
     if (!x.projection) c0 = c0 - (T)x.bias;
     e.C.x = c0 + dot(n[0], u);
   } else {
-    e.C.x = om * (T)cA.w + dot(n[0], u);
+    // fused explicitly: left to the compiler, the staged and the wide form of
+    // the solve would round this differently
+    if constexpr (sizeof(T) == 4) e.C.x = __fmaf_rn(om, cA.w, dot(n[0], u));
+    else e.C.x = om * (T)cA.w + dot(n[0], u);
   }
   e.C.y = om * (T)cB.w + dot(n[1], u);
   e.C.z = om * (T)cK.w + dot(n[2], u);
@@ -1714,25 +1717,16 @@ __device__ inline void st_release(int *p, int v) {
 // stored (what a later body of the tail segment reads of it), before the
 // velocity and the dual updates.
 template <class T>
-__device__ __forceinline__ void finish_body(const World &w, int i, int lane, int G, unsigned mask, bool velocity,
-                                            float4 qt, Sys<T> &s, BState<T> &self, int maxG, int *publish = nullptr,
-                                            int pubValue = 0) {
+__device__ __forceinline__ void apply_solution(const World &w, int i, bool writer, bool velocity, float4 qt,
+                                               const Sys<T> &s, BState<T> &self, int *publish = nullptr,
+                                               int pubValue = 0) {
   const T dt = pick<T>(w.p.dt, w.p.dtF);
-  if constexpr (sizeof(T) == 4) {
-    if (G == 32) group_reduce32(s);
-    else if (G > 32) group_reduce_warps(s, G);
-    else if (maxG) warp_reduce(s, G, maxG);
-    else group_reduce(s, mask, G);
-  } else {
-    if (maxG) warp_reduce(s, G, maxG);
-    else group_reduce(s, mask, G);
-  }
   V3<T> xl, xa;
   ldlt_solve(s, -s.bl[0], -s.bl[1], -s.bl[2], -s.ba[0], -s.ba[1], -s.ba[2], xl, xa);
   self.dp = self.dp + xl;
   self.q = qintegrate(self.q, xa);
   self.dang = qsub(self.q, Q4<T>{(T)qt.x, (T)qt.y, (T)qt.z, (T)qt.w});
-  if (lane != 0) return;
+  if (!writer) return;
   __stcg(&w.b.dp[i], make_float4((float)self.dp.x, (float)self.dp.y, (float)self.dp.z, 0.f));
   __stcg(&w.b.quat[i], make_float4((float)self.q.x, (float)self.q.y, (float)self.q.z, (float)self.q.w));
   {  // what neighbours read: qsub of the f32 orientation, as load_state<float> forms it
@@ -1752,6 +1746,22 @@ __device__ __forceinline__ void finish_body(const World &w, int i, int lane, int
     w.b.vel[i] = make_float4((float)(self.dp.x / dt), (float)(self.dp.y / dt), (float)(self.dp.z / dt), 0.f);
     w.b.omega[i] = make_float4((float)(self.dang.x / dt), (float)(self.dang.y / dt), (float)(self.dang.z / dt), 0.f);
   }
+}
+
+template <class T>
+__device__ __forceinline__ void finish_body(const World &w, int i, int lane, int G, unsigned mask, bool velocity,
+                                            float4 qt, Sys<T> &s, BState<T> &self, int maxG, int *publish = nullptr,
+                                            int pubValue = 0) {
+  if constexpr (sizeof(T) == 4) {
+    if (G == 32) group_reduce32(s);
+    else if (G > 32) group_reduce_warps(s, G);
+    else if (maxG) warp_reduce(s, G, maxG);
+    else group_reduce(s, mask, G);
+  } else {
+    if (maxG) warp_reduce(s, G, maxG);
+    else group_reduce(s, mask, G);
+  }
+  apply_solution<T>(w, i, lane == 0, velocity, qt, s, self, publish, pubValue);
 }
 
 // One body's update (solver.js:425-457) by a group of G lanes, followed by
@@ -1923,9 +1933,9 @@ __device__ __noinline__ Sys<T> constraints_primal(const World &w, int nm, int cS
 
 template <class T, bool E>
 __device__ __noinline__ void constraints_dual(const World &w, int i, int nm, int cStart, int total, int lane, int G,
-                                              const BState<T> self, T alpha) {
+                                              const BState<T> self, T alpha, int part = 0, int parts = 1) {
   const int myColor = ld(&w.b.color[i]);
-  for (int e = first_extra(lane, nm, G); e < total; e += G) {
+  for (int e = first_extra(lane, nm, G) + part * G; e < total; e += parts * G) {
     const uint32_t ref = ld(&w.g.cRef[cStart + e - nm]);
     const uint32_t type = ref >> 30, idx = (ref >> 1) & 0x1fffffffu, side = ref & 1u;
     const int2 ab = type == kRefJoint ? ld(&w.j.bodies[idx]) : ld(&w.s.bodies[idx]);
@@ -1951,7 +1961,7 @@ __device__ __noinline__ void tail_wait_extra(const World &w, int nm, int cStart,
 
 // `tw`: the tail waits of this body (null outside the tail segment). maxG:
 // see finish_body; `act` is false on the idle lanes of a whole warp.
-template <bool E>
+template <bool E, bool J>
 __device__ void solve_body_staged(const World &w, int4 rec, int lane, int G, unsigned mask, float alpha, bool dual,
                                   bool velocity, float4 *stage, const TailWait *tw = nullptr, int maxG = 0,
                                   bool act = true) {
@@ -1987,7 +1997,7 @@ __device__ void solve_body_staged(const World &w, int4 rec, int lane, int G, uns
     cnt = nk - k0 < kStageSlots ? nk - k0 : kStageSlots;
     stage_chunk(w, cb, lane, G, k0, cnt, ent, stage, false, tw);
   }
-  if (total > nm) {
+  if (J && total > nm) {
     if (tw) tail_wait_extra(w, nm, cStart, total, lane, G, *tw);
     s = constraints_primal<T, E>(w, nm, cStart, total, lane, G, self, alpha, s);
   }
@@ -2014,7 +2024,7 @@ __device__ void solve_body_staged(const World &w, int4 rec, int lane, int G, uns
           contact_dual<T>(w, staged_contact<E>(w, stage + j * kStageVecs * kSolveBlock, ent[j], alpha), self, alpha);
     }
   }
-  if (total > nm) constraints_dual<T, E>(w, i, nm, cStart, total, lane, G, self, alpha);
+  if (J && total > nm) constraints_dual<T, E>(w, i, nm, cStart, total, lane, G, self, alpha);
 }
 
 // The FP64 path is kept out of line so that its register demand (and any
@@ -2078,6 +2088,207 @@ __device__ __forceinline__ void group_sync(int G, unsigned mask) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Wide form (FP32): four threads per lane of a body's group, for the colours
+// whose lanes leave most of the grid idle. Such a phase lasts as long as one
+// body update, and the staged form makes a lane walk its (up to four)
+// contacts one after the other, stamping all 27 entries of the system for
+// each. Here a chunk of 128 lanes is cut into units of 32, a block per unit,
+// and warp h of the block
+//   * evaluates contact h of each lane, straight from registers, and leaves
+//     its three rows in shared memory (warp 3 the inertial terms as well),
+//   * sums a quarter of the entries over the lane's contacts, in the staged
+//     form's order and with its operations, so the sums are bitwise the same,
+//   * reduces its entries over the group (the staged form's butterfly);
+// then every thread reads the 27 totals, solves, and does the dual update of
+// the contact it evaluated. Solve, with scenes without joints in instances
+// of their own: ten-cube stack 157 -> 101 us, piles of 200 / 1,777 / 8,192
+// bodies 262 / 497 / 531 -> 194 / 334 / 362, the standing 53-layer pyramid (its
+// smaller colours) 606 -> 515.
+// ---------------------------------------------------------------------------
+constexpr int kWideSplit = kSolveBlock / 32;
+constexpr int kWideRows = 6 * kSolveBlock;  // float4: three rows of two vectors a contact
+constexpr int kWideTot = 36;                // floats between two groups' entries (conflict-free)
+static_assert(kWideRows * sizeof(float4) + 2 * 8 * kWideTot * sizeof(float) <= kSolveSmem, "wide form's shared memory");
+static_assert(kWideSplit == kStageSlots, "a lane's contacts go to the warps of its block");
+
+// The entries of the system that warp H sums: the linear block, the angular
+// block, the cross block, the right-hand side.
+template <int H, class F>
+__device__ __forceinline__ void wide_entries(Sys<float> &s, F &&f) {
+  if (H == 0) {
+#pragma unroll
+    for (int k = 0; k < 6; k++) f(s.l[k], k);
+  } else if (H == 1) {
+#pragma unroll
+    for (int k = 0; k < 6; k++) f(s.a[k], 6 + k);
+  } else if (H == 2) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) f(s.c[k], 12 + k);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; k++) f(s.bl[k], 21 + k);
+#pragma unroll
+    for (int k = 0; k < 3; k++) f(s.ba[k], 24 + k);
+  }
+}
+
+template <int H, bool E, bool J>
+__device__ __forceinline__ void wide_sums(const World &w, int4 rec, int nk, int cStart, int total, bool grabbed,
+                                          const BState<float> &self, int lane, int G, int maxG, bool act, float alpha,
+                                          const float4 *rows, const float *init, float *tot) {
+  const int l = threadIdx.x & 31;
+  Sys<float> s;
+  zero(s);
+  if (H != 2 && act && lane == 0) wide_entries<H>(s, [&](float &x, int k) { x = init[(l >> 2) * kWideTot + k]; });
+#pragma unroll 1
+  for (int j = 0; j < nk; j++) {
+#pragma unroll
+    for (int row = 0; row < 3; row++) {
+      const float4 p = rows[(2 * row) * kSolveBlock + j * 32 + l], q = rows[(2 * row + 1) * kSolveBlock + j * 32 + l];
+      const float k = p.x, f = q.x;
+      const float nn[3] = {p.y, p.z, p.w}, aa[3] = {q.y, q.z, q.w};
+      if (H < 3) {
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            if (H == 0 && c <= r) s.l[L(r, c)] += k * nn[r] * nn[c];
+            if (H == 1 && c <= r) s.a[L(r, c)] += k * aa[r] * aa[c];
+            if (H == 2) s.c[r * 3 + c] += k * aa[r] * nn[c];
+          }
+      } else {
+        s.bl[0] += f * nn[0]; s.bl[1] += f * nn[1]; s.bl[2] += f * nn[2];
+        s.ba[0] += f * aa[0]; s.ba[1] += f * aa[1]; s.ba[2] += f * aa[2];
+      }
+    }
+  }
+  if (act) {
+    const int nm = rec.z - rec.y;
+    if ((J && total > nm) || grabbed) {
+      Sys<float> t;
+      zero(t);
+      float v[9];
+      constexpr int k0 = H == 0 ? 0 : H == 1 ? 6 : H == 2 ? 12 : 21;
+      wide_entries<H>(s, [&](float &x, int k) { v[k - k0] = x; });
+      wide_entries<H>(t, [&](float &x, int k) { x = v[k - k0]; });
+      if (J && total > nm) t = constraints_primal<float, E>(w, nm, cStart, total, lane, G, self, alpha, t);
+      if (grabbed) t = grab_primal<float>(w, rec.x, self, t);
+      wide_entries<H>(t, [&](float &x, int k) { v[k - k0] = x; });
+      wide_entries<H>(s, [&](float &x, int k) { x = v[k - k0]; });
+    }
+  }
+  __syncwarp();
+  for (int m = maxG >> 1; m > 0; m >>= 1) {
+    const bool on = m < G;
+    wide_entries<H>(s, [&](float &x, int) {
+      const float o = __shfl_xor_sync(0xffffffffu, x, m);
+      x = on ? x + o : x;
+    });
+  }
+  if (act && lane == 0) wide_entries<H>(s, [&](float &x, int k) { tot[(l >> 2) * kWideTot + k] = x; });
+}
+
+// One unit: the block's 32 lanes (table entry and record of lane threadIdx %
+// 32), bodies of up to 32 lanes each with at most four contacts a lane.
+template <bool E, bool J>
+__device__ __forceinline__ void wide_body(const World &w, int e, int4 rec, float alpha, bool dual, bool vel,
+                                          float4 *sm) {
+  const int l = threadIdx.x & 31, h = threadIdx.x >> 5;
+  const bool act = e >= 0 && !(e & 8);
+  const int G = act ? 1 << (e & 7) : 1, lane = act ? l & (G - 1) : 1;
+  const int maxG = __reduce_max_sync(0xffffffffu, G);
+  float4 *rows = sm;
+  float *tot = reinterpret_cast<float *>(sm + kWideRows), *init = tot + 8 * kWideTot;
+  const int i = act ? rec.x : 0, nm = act ? rec.z - rec.y : 0;
+  const int nk = lane < nm ? (nm - lane + G - 1) / G : 0;
+  const bool has = h < nk;
+  int2 ent = make_int2(0, 0);
+  if (has) ent = ld(&w.a.centry[rec.y + lane + h * G]);
+  const float4 qt = ld(&w.b.quatT[i]);
+  const float4 d0 = ldcg(&w.b.dp[i]), q0 = ldcg(&w.b.quat[i]);
+  const int cStart = ld(&w.g.cStart[i]), cEnd = ld(&w.g.cStart[i + 1]);
+  const bool grabbed = lane == 0 && ld(&w.grab->body) == i;
+  const bool lead = h == 3 && lane == 0;
+  float4 mf, y, qy;
+  bool sphere = false;
+  if (lead) {
+    mf = ld(&w.b.massF[i]);
+    y = ld(&w.b.yLin[i]);
+    qy = ld(&w.b.yAng[i]);
+    sphere = (ld(&w.b.flags0[i]) & kBodySphere) != 0;
+  }
+  const int total = act ? nm + (cEnd - cStart) : 0;
+  ContactData<float> d;
+  if (has) d = load_contact<float, E>(w, ent, alpha);
+  BState<float> self;
+  self.dp = V3<float>{d0.x, d0.y, d0.z};
+  self.q = Q4<float>{q0.x, q0.y, q0.z, q0.w};
+  self.dang = qsub(self.q, Q4<float>{qt.x, qt.y, qt.z, qt.w});
+  if (lead) {
+    Sys<float> s;
+    zero(s);
+    inertial_core<float>(w.p, mf.x, mf.y, mf.z, mf.w, y, qy, self, sphere, s);
+    float *o = init + (l >> 2) * kWideTot;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      o[k] = s.l[k];
+      o[6 + k] = s.a[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      o[21 + k] = s.bl[k];
+      o[24 + k] = s.ba[k];
+    }
+  }
+  if (has) {
+    const BState<float> &A = d.side ? d.o : self;
+    const BState<float> &B = d.side ? self : d.o;
+    const float sgn = d.side ? -1.f : 1.f;
+    const ContactEval<float> ev = eval_contact(d.n, d.mu, d.cA, d.cB, d.cK, d.cL, A, B, alpha, d.x);
+    const V3<float> r = d.side ? V3<float>{d.cB.x, d.cB.y, d.cB.z} : V3<float>{d.cA.x, d.cA.y, d.cA.z};
+    const float kk[3] = {d.cK.x, d.cK.y, d.cK.z}, ff[3] = {ev.F.x, ev.F.y, ev.F.z};
+#pragma unroll
+    for (int row = 0; row < 3; row++) {
+      const V3<float> a = cross(r, d.n[row]);
+      const float f = sgn * ff[row];
+      rows[(2 * row) * kSolveBlock + threadIdx.x] = make_float4(kk[row], d.n[row].x, d.n[row].y, d.n[row].z);
+      rows[(2 * row + 1) * kSolveBlock + threadIdx.x] = make_float4(f, a.x, a.y, a.z);
+    }
+  }
+  __syncthreads();
+  if (h == 0) wide_sums<0, E, J>(w, rec, nk, cStart, total, grabbed, self, lane, G, maxG, act, alpha, rows, init, tot);
+  else if (h == 1) wide_sums<1, E, J>(w, rec, nk, cStart, total, grabbed, self, lane, G, maxG, act, alpha, rows, init, tot);
+  else if (h == 2) wide_sums<2, E, J>(w, rec, nk, cStart, total, grabbed, self, lane, G, maxG, act, alpha, rows, init, tot);
+  else wide_sums<3, E, J>(w, rec, nk, cStart, total, grabbed, self, lane, G, maxG, act, alpha, rows, init, tot);
+  __syncthreads();
+  float v[28];
+  const float4 *t4 = reinterpret_cast<const float4 *>(tot + ((act ? l - lane : 0) >> 2) * kWideTot);
+#pragma unroll
+  for (int k = 0; k < 7; k++) {
+    const float4 x = t4[k];
+    v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
+  }
+  Sys<float> s;
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    s.l[k] = v[k];
+    s.a[k] = v[6 + k];
+  }
+#pragma unroll
+  for (int k = 0; k < 9; k++) s.c[k] = v[12 + k];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    s.bl[k] = v[21 + k];
+    s.ba[k] = v[24 + k];
+  }
+  apply_solution<float>(w, i, h == 0 && lane == 0, vel, qt, s, self);
+  if (!dual) return;
+  if (has && d.owned) contact_dual<float>(w, d, self, alpha);
+  if (J && total > nm)
+    constraints_dual<float, E>(w, i, nm, cStart, total, lane, G, self, alpha, h, kWideSplit);
+}
+
 // Colour phases separated by grid barriers. Each block takes the colour's
 // lane chunks (Adjacency::laneTab) j, j + gridDim.x, ...: one body per lane
 // group, a group's G lanes working on its constraints. j transposes the
@@ -2094,7 +2305,7 @@ __device__ __forceinline__ void group_sync(int G, unsigned mask) {
 constexpr int kTailDiv = 8;  // default of SolverParams::tailDiv
 constexpr int kTailMinColors = 16;  // automatic: steps of fewer colours have no tail segment
 constexpr int kChunkCache = 64;  // colours whose chunk bounds the solve keeps in shared memory
-template <bool E, bool F64>
+template <bool E, bool J, bool F64>
 __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
   if (step_skipped(w)) return;
   extern __shared__ float4 stageSm[];
@@ -2122,20 +2333,38 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
     const int tailDiv = P.tailDiv > 0 ? P.tailDiv : kTailDiv;
     while (tail > 0 && chunkAt(tail) - chunkAt(tail - 1) <= (int)gridDim.x / tailDiv) tail--;
   }
+  // a colour is solved in the wide form when its units fit the grid (a fixed
+  // lane count may put more than four contacts on a lane: staged form)
+  auto wide = [&](int c) {
+    return P.lanes <= 0 && (chunkAt(c + 1) - chunkAt(c)) * kWideSplit <= (int)gridDim.x;
+  };
   // the blocks that any phase gives work; the others leave, so that a small
   // scene's barriers wait for few
   int active = tail < numColors ? (int)gridDim.x : 1;
   for (int c = 0; c < tail && active < (int)gridDim.x; c++)
-    active = min((int)gridDim.x, max(active, chunkAt(c + 1) - chunkAt(c)));
+    active = min((int)gridDim.x, max(active, (chunkAt(c + 1) - chunkAt(c)) * (wide(c) ? kWideSplit : 1)));
   if (jb >= active) return;
-  // this thread's lane of a chunk
+  // this thread's lane of a chunk (wide form: of a unit of 32 lanes)
   int e = -1;
   int4 rec0 = make_int4(0, 0, 0, 0);
-  auto load = [&](int q) {
-    e = ld(&w.a.laneTab[(size_t)q * kLaneMaxGroup + threadIdx.x]);
+  bool wd = false;
+  auto load = [&](const int *t) {
+    e = ld(t);
     rec0 = e >= 0 ? ld(&w.a.colorRec[e >> 4]) : make_int4(0, 0, 0, 0);
   };
-  if (tail > 0 && chunkAt(0) + jb < chunkAt(1)) load(chunkAt(0) + jb);
+  auto first = [&](int c) {  // the block's first chunk or unit of colour c
+    wd = wide(c);
+    const int q = chunkAt(c) + (wd ? jb / kWideSplit : jb);
+    if (q >= chunkAt(c + 1)) return;
+    const int *t = w.a.laneTab + (size_t)q * kLaneMaxGroup;
+    if (wd && (ld(t) & 7) <= 5) {
+      load(t + (jb % kWideSplit) * 32 + warpLane);
+    } else {
+      wd = false;  // (a group of more than 32 lanes: the chunk's first block takes it whole)
+      load(t + threadIdx.x);
+    }
+  };
+  if (tail > 0) first(0);
   for (int it = 0; it < total; it++) {
     const double alpha = P.postStabilize ? (it < P.iterations ? 1.0 : 0.0) : P.alpha;
     const float alphaF = P.postStabilize ? (it < P.iterations ? 1.f : 0.f) : P.alphaF;
@@ -2143,16 +2372,33 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
     const bool vel = it == P.iterations - 1;
     for (int c = 0; c < tail; c++) {
       const int q0 = chunkAt(c), q1 = chunkAt(c + 1);
-      for (int q = q0 + jb; q < q1; q += active) {
+      const bool wc = wide(c);
+      const int qf = q0 + (wc ? jb / kWideSplit : jb);
+      for (int q = qf; q < q1; q += wc ? (int)gridDim.x : active) {
+        if (wd) {
+          wide_body<E, J>(w, e, rec0, alphaF, dual, vel, stageSm);
+          if (F64 && threadIdx.x < 32) {
+            const bool f64 = e >= 0 && (e & 8);
+            const unsigned any64 = __ballot_sync(0xffffffffu, f64);
+            if (any64) {
+              const int G = f64 ? 1 << (e & 7) : 1;
+              const int maxG = __shfl_sync(0xffffffffu, G, __ffs(any64) - 1);
+              solve_body_f64<E>(w, f64 ? rec0 : make_int4(0, 0, 0, 0), f64 ? warpLane & (G - 1) : 1, G, 0u, alpha, dual,
+                                vel, maxG, f64);
+            }
+          }
+          continue;
+        }
+        if (wc && jb % kWideSplit != 0) continue;
+        if (q != qf) load(w.a.laneTab + (size_t)q * kLaneMaxGroup + threadIdx.x);
         // whole warps: a lane past the colour's last group, or of a body of
         // the other precision, goes along idle
-        if (q != q0 + jb) load(q);  // the first was requested before the barrier
         const bool f32 = e >= 0 && !(e & 8), f64 = e >= 0 && (e & 8);
         const unsigned any32 = __ballot_sync(0xffffffffu, f32), any64 = __ballot_sync(0xffffffffu, f64);
         if (any32) {
           const int G = f32 ? 1 << (e & 7) : 1;
           const int maxG = __shfl_sync(0xffffffffu, G, __ffs(any32) - 1);  // groups come in decreasing size
-          solve_body_staged<E>(w, f32 ? rec0 : make_int4(0, 0, 0, 0), f32 ? threadIdx.x & (G - 1) : 1, G, 0u, alphaF,
+          solve_body_staged<E, J>(w, f32 ? rec0 : make_int4(0, 0, 0, 0), f32 ? threadIdx.x & (G - 1) : 1, G, 0u, alphaF,
                                dual, vel, stage, nullptr, maxG, f32);
         }
         if (F64 && any64) {
@@ -2163,9 +2409,8 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
         }
       }
       solve_arrive(ctl);
-      const int next = c + 1 < tail ? c + 1 : 0;
-      if ((c + 1 < tail || (it + 1 < total && tail == numColors)) && chunkAt(next) + jb < chunkAt(next + 1))
-        load(chunkAt(next) + jb);
+      if (c + 1 < tail) first(c + 1);
+      else if (it + 1 < total && tail == numColors) first(0);
       arrivals += active;
       if (!solve_wait(ctl, arrivals, w.p.barrierLimit)) return;
     }
@@ -2191,11 +2436,11 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
           if (lane == 0) st_release(&w.b.progress[rec.x], it + 1);
         } else {
           const TailWait tw{tail, c, it + 1};  // publishes the body's progress itself
-          solve_body_staged<E>(w, rec, lane, G, mask, alphaF, dual, vel, stage, &tw);
+          solve_body_staged<E, J>(w, rec, lane, G, mask, alphaF, dual, vel, stage, &tw);
         }
       }
       solve_arrive(ctl);
-      if (it + 1 < total && tail > 0 && chunkAt(0) + jb < chunkAt(1)) load(chunkAt(0) + jb);
+      if (it + 1 < total && tail > 0) first(0);
       arrivals += active;
       if (!solve_wait(ctl, arrivals, w.p.barrierLimit)) return;
     }
@@ -2214,7 +2459,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
 
 
 
-template <bool E, bool F64>
+template <bool E, bool J, bool F64>
 __global__ void __launch_bounds__(kSolveBlock, 3) wave_kernel(World w, int G) {
   if (step_skipped(w)) return;
   extern __shared__ float4 stageSm[];
@@ -2242,7 +2487,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) wave_kernel(World w, int G) {
         if (!wait_neighbors(w, i, it, lane, G, mask)) return;
         __syncwarp(mask);  // orders every lane's reads after the acquires of the others
         if (F64 && (ld(&w.b.flags[i]) & kBodyFp64)) solve_body_f64<E>(w, rec, lane, G, mask, alpha, dual, vel);
-        else solve_body_staged<E>(w, rec, lane, G, mask, (float)alpha, dual, vel, stage);
+        else solve_body_staged<E, J>(w, rec, lane, G, mask, (float)alpha, dual, vel, stage);
         // the warp barrier orders every lane's writes before lane 0's release,
         // which makes them visible at gpu scope to whoever acquires the flag
         __syncwarp(mask);
@@ -2402,26 +2647,29 @@ cudaError_t launch_joint_anchor(const World &w, int joint, double x, double y, d
 }
 
 // The solve's instantiations: the contact extensions
-// (AVBD_CONTACT_MATERIALS) and the FP64 bodies each in kernels of their own,
-// so that the others carry none of their registers. The FP64 path's calls
+// (AVBD_CONTACT_MATERIALS), joints and springs, and the FP64 bodies each in
+// kernels of their own, so that the others carry none of their registers. The
+// joints' calls cost 130 bytes of spills, the FP64 path's calls
 // cost the kernel a 1.4 KB stack frame and 260 bytes of spills, which every
 // grid barrier's acquire throws out of L1; without it there are none (148 registers;
 // solve of piles of 200 / 8,192 bodies 0.30 -> 0.27 / 0.60 -> 0.55 ms, the
 // crushed 36-layer pyramid 4.96 -> 4.58).
-static const void *solve_instance(bool wave, bool ext, bool fp64) {
-  if (wave) {
-    if (ext) return fp64 ? (const void *)wave_kernel<true, true> : (const void *)wave_kernel<true, false>;
-    return fp64 ? (const void *)wave_kernel<false, true> : (const void *)wave_kernel<false, false>;
-  }
-  if (ext) return fp64 ? (const void *)solve_kernel<true, true> : (const void *)solve_kernel<true, false>;
-  return fp64 ? (const void *)solve_kernel<false, true> : (const void *)solve_kernel<false, false>;
+template <bool E, bool J, bool F64>
+static const void *solve_instance(bool wave) {
+  return wave ? (const void *)wave_kernel<E, J, F64> : (const void *)solve_kernel<E, J, F64>;
+}
+static const void *solve_instance(bool wave, bool ext, bool joints, bool fp64) {
+  if (ext) return fp64 ? solve_instance<true, true, true>(wave) : joints ? solve_instance<true, true, false>(wave)
+                                                                        : solve_instance<true, false, false>(wave);
+  return fp64 ? solve_instance<false, true, true>(wave) : joints ? solve_instance<false, true, false>(wave)
+                                                                 : solve_instance<false, false, false>(wave);
 }
 
 int solve_max_blocks_per_sm(int lanesPerBody) {
   (void)lanesPerBody;
   int best = 1 << 30;
-  for (int k = 0; k < 8; k++) {
-    const void *f = solve_instance(k & 1, k & 2, k & 4);
+  for (int k = 0; k < 12; k++) {
+    const void *f = solve_instance(k & 1, k & 2, k / 4 >= 1, k / 4 == 2);
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem);
     int a = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f, kSolveBlock, kSolveSmem);
@@ -2438,7 +2686,7 @@ cudaError_t launch_solve(const World &w, int lanesPerBody, int blocksPerSm, cuda
   void *args2[] = {&arg, &G};
   void *args1[] = {&arg};
   const bool wave = w.p.schedule == 1;
-  return cudaLaunchCooperativeKernel(solve_instance(wave, w.p.contactModel != 0, w.p.mayFp64 != 0),
+  return cudaLaunchCooperativeKernel(solve_instance(wave, w.p.contactModel != 0, w.g.hasConstraints != 0, w.p.mayFp64 != 0),
                                      dim3(blocksPerSm * smCount), dim3(kSolveBlock), wave ? args2 : args1, kSolveSmem,
                                      st);
 }
