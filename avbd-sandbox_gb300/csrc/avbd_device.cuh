@@ -87,8 +87,6 @@ __host__ __device__ inline T pick(double d, float f) {
 // Device scalars shared by all kernels of a step.
 struct Control {
   unsigned flags;          // overflow / error bits (sticky until pack)
-  unsigned barrierCount;   // grid barrier
-  unsigned barrierGen;
   int numCandidates;
   int numColors;
   unsigned solveArrivals;  // arrivals at the solve's grid barrier this step
@@ -96,6 +94,7 @@ struct Control {
   int liveContacts;
   int fp64Bodies;
   int gridEntries;  // grid entries handed out this step
+  unsigned colorArrivals;  // arrivals at the colouring's grid barrier this step
   int prevCandidates;  // candidates (= manifold slots) of the previous step
   int npCount[3];      // narrow-phase work lists: face, edge, exact
   int colorBad;        // this step's uploaded colouring has a conflict
@@ -413,7 +412,7 @@ void launch_broadphase_impl(const World &w, int numLarge, cudaStream_t st, int s
 void launch_narrowphase(const World &w, cudaStream_t st, int smCount);
 void launch_prepare(const World &w, cudaStream_t st, int smCount);
 cudaError_t launch_coloring(const World &w, cudaStream_t st, int blocks);
-int coloring_grid(int smCount);  // blocks of the cooperative colouring launch
+int coloring_grid(int n, int smCount);  // blocks of the cooperative colouring launch
 cudaError_t launch_solve(const World &w, int lanesPerBody, int blocksPerSm, cudaStream_t st, int smCount);
 int solve_max_blocks_per_sm(int lanesPerBody);
 void launch_commit(const World &w, cudaStream_t st, int smCount);

@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -490,8 +491,9 @@ void invalidate_graphs(avbd_ctx *ctx) {
 int enqueue_step(avbd_ctx *ctx) {
   World &w = ctx->w;
   cudaStream_t st = ctx->stream;
-  // per-step counters: numCandidates .. gridEntries
-  CK(cudaMemsetAsync(&w.ctl->numCandidates, 0, sizeof(int) * 7, st));
+  // per-step counters: numCandidates .. colorArrivals
+  CK(cudaMemsetAsync(&w.ctl->numCandidates, 0,
+                     offsetof(Control, colorArrivals) + sizeof(unsigned) - offsetof(Control, numCandidates), st));
   int rc;
   if ((rc = record(ctx, 0))) return rc;
   launch_broadphase_impl(w, ctx->numLarge, st, ctx->smCount);
@@ -1106,7 +1108,7 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   w.g.hasConstraints = (ctx->nj + ctx->ns) > 0 ? 1 : 0;
   // adjacency + colouring
   w.a.cap = ctx->adjCap;
-  ctx->colorBlocks = std::max(1, coloring_grid(ctx->smCount));
+  ctx->colorBlocks = std::max(1, coloring_grid(n, ctx->smCount));
   if ((rc = dalloc(ctx, &w.a.start, n + 1)) || (rc = dalloc(ctx, &w.a.count, n)) ||
       (rc = dalloc(ctx, &w.a.runCount, n / kAdjRun + 1)) ||
       (rc = dalloc(ctx, &w.a.hpCount, n)) ||

@@ -42,59 +42,20 @@ constexpr int kStageVecs = 9;      // float4 per staged contact
 constexpr size_t kSolveSmem = (size_t)kSolveBlock * kStageSlots * kStageVecs * sizeof(float4);  // 73,728 B
 
 // ---------------------------------------------------------------------------
-// Bounded grid barrier (all blocks are co-resident: cooperative launch).
-// Returns false when the wait gave up or another block reported a timeout;
-// the caller must then return.
+// Bounded grid barrier (all blocks are co-resident: cooperative launch), in
+// two halves. Arrivals are counted in one word (zeroed with the step's
+// counters), and barrier k of `blocks` blocks is over when it reaches
+// k * blocks. Waiters poll the word the arrivals go to, and the timeout flag
+// in the same round trip: with a generation word that the last arrival
+// writes, a second fence and a closing flag read, a barrier of one busy block
+// took 3,800 cycles, with this 2,200. grid_wait returns false when the wait
+// gave up or another block reported a timeout; the caller must then return.
 // ---------------------------------------------------------------------------
-__device__ bool grid_barrier(Control *ctl, long long limit) {
-  __shared__ int ok;
+__device__ __forceinline__ void grid_arrive(unsigned *arrivals) {
   __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = 1;
-    volatile unsigned *gen = &ctl->barrierGen;
-    const unsigned g = *gen;
-    __threadfence();
-    const unsigned arrived = atomicAdd(&ctl->barrierCount, 1u) + 1u;
-    if (arrived == gridDim.x) {
-      ctl->barrierCount = 0;
-      __threadfence();
-      atomicAdd(&ctl->barrierGen, 1u);
-    } else {
-      long long spins = 0;
-      while (*gen == g) {
-        // give up after `limit` polls, or at once when another block gave up
-        if (++spins > limit || (*((volatile unsigned *)&ctl->flags) & kOvfTimeout)) {
-          atomicOr(&ctl->flags, kOvfTimeout);
-          break;
-        }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-    if (*((volatile unsigned *)&ctl->flags) & kOvfTimeout) ok = 0;
-  }
-  __syncthreads();
-  return ok != 0;
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrivals) : "memory");
 }
-
-// The solve's grid barrier: arrivals of the step are counted in one word
-// (zeroed with the step's counters), and phase k of `blocks` blocks is over
-// when it reaches k * blocks. Waiters poll the word the arrivals go to, and
-// the timeout flag in the same round trip: the generation word of
-// grid_barrier, its second fence and its closing flag read are three more
-// memory round trips a phase (3,800 cycles a barrier of one busy block with
-// grid_barrier, 2,200 with this). Gives up as grid_barrier does. In two
-// halves: while it waits, a block looks up its lanes of the next phase (two
-// dependent loads; the crushed 36-layer pyramid's solve 4.53 -> 4.39 ms, a
-// 163,000-body batch's 1.97 -> 1.90). More is not worth prefetching there: the
-// contacts' constants live across the barrier spill, and the phase is 10 %
-// slower.
-__device__ __forceinline__ void solve_arrive(Control *ctl) {
-  __syncthreads();
-  if (threadIdx.x == 0)
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->solveArrivals) : "memory");
-}
-__device__ __forceinline__ bool solve_wait(Control *ctl, unsigned target, long long limit) {
+__device__ __forceinline__ bool grid_wait(Control *ctl, const unsigned *arrivals, unsigned target, long long limit) {
   __shared__ int ok;
   if (threadIdx.x == 0) {
     int good = 1;
@@ -102,9 +63,10 @@ __device__ __forceinline__ bool solve_wait(Control *ctl, unsigned target, long l
     for (;;) {
       const unsigned f = *((volatile unsigned *)&ctl->flags);  // in flight together with the count
       unsigned v;
-      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->solveArrivals) : "memory");
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrivals) : "memory");
       if (f & kOvfTimeout) good = 0;
       if ((int)(v - target) >= 0 || !good) break;
+      // give up after `limit` polls, or at once when another block gave up
       if (++spins > limit) {
         atomicOr(&ctl->flags, kOvfTimeout);
         good = 0;
@@ -498,6 +460,13 @@ __device__ inline void constraint_neighbors(const World &w, int i, F &&f) {
   }
 }
 
+// Every block of the colouring past this point; `arrivals` counts along.
+__device__ __forceinline__ bool coloring_barrier(const World &w, unsigned &arrivals) {
+  arrivals += gridDim.x;
+  grid_arrive(&w.ctl->colorArrivals);
+  return grid_wait(w.ctl, &w.ctl->colorArrivals, arrivals, w.p.barrierLimit);
+}
+
 // log2 of the lanes of a body's group in the colour-phase solve: the fixed
 // lanes parameter, else the fewest lanes (4..128) whose staging of four
 // constraints per lane holds all of the body's constraints; FP64 bodies
@@ -523,7 +492,7 @@ __device__ __forceinline__ int lane_log2(const World &w, int4 rec) {
 // numbered in colour order. Placement within a (colour, size) class follows
 // atomics and may vary between runs; a body's arithmetic depends only on its
 // group size, so results do not.
-__device__ void lane_layout(const World &w) {
+__device__ void lane_layout(const World &w, unsigned &arrivals) {
   Control *ctl = w.ctl;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   volatile int *color = w.b.color;
@@ -543,7 +512,7 @@ __device__ void lane_layout(const World &w) {
     const unsigned peers = __match_any_sync(0xffffffffu, key);
     if (key >= 0 && lane == __ffs(peers) - 1) atomicAdd(&cnt[key], __popc(peers));
   }
-  if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+  if (!coloring_barrier(w, arrivals)) return;
   if (blockIdx.x == 0) {
     // per colour: the offsets of its size classes (largest first) and its
     // lane count; then the colours' first chunks by a block-wide scan
@@ -582,7 +551,7 @@ __device__ void lane_layout(const World &w) {
     lanesTotal = __reduce_add_sync(0xffffffffu, lanesTotal);
     if (lane == 0 && lanesTotal) atomicAdd(&ctl->laneTotal, lanesTotal);
   }
-  if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+  if (!coloring_barrier(w, arrivals)) return;
   for (int k = tid; k < numColors * kLaneBuckets; k += stride) cnt[k] = 0;  // for the next step
   for (int r = tid; r - lane < nrec; r += stride) {
     int key = -1, c = 0, b = 0, e = 0;
@@ -621,7 +590,7 @@ __device__ void lane_layout(const World &w) {
 // barriers inside). Per-colour loops run over the colours in use only
 // (Control::numColors, from the largest colour found), so a step of few
 // colours pays nothing for the colour capacity.
-__device__ void coloring_finish(const World &w) {
+__device__ void coloring_finish(const World &w, unsigned &arrivals) {
   Control *ctl = w.ctl;
   const int n = w.b.n;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -645,7 +614,7 @@ __device__ void coloring_finish(const World &w) {
   maxColor = __reduce_max_sync(0xffffffffu, maxColor);
   if ((threadIdx.x & 31) == 0 && maxColor >= 0) atomicMax(&ctl->numColors, maxColor + 1);
   if (tid == 0) ctl->laneTotal = 0;  // summed by lane_layout after the next barriers
-  if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+  if (!coloring_barrier(w, arrivals)) return;
   const int numColors = *((volatile int *)&ctl->numColors);
   // --- stable counting sort by colour (per-block chunk of body indices) ---
   __shared__ int hist[kMaxColors];
@@ -660,7 +629,7 @@ __device__ void coloring_finish(const World &w) {
   }
   __syncthreads();
   for (int c = threadIdx.x; c < numColors; c += blockDim.x) w.a.blockHist[blockIdx.x * kMaxColors + c] = hist[c];
-  if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+  if (!coloring_barrier(w, arrivals)) return;
   if (blockIdx.x == 0) {
     // per colour: the blocks' offsets (a scan over blocks), then the colours'
     // starts (a block-wide scan over colours, in rounds of blockDim colours).
@@ -713,7 +682,7 @@ __device__ void coloring_finish(const World &w) {
     }
     for (int c = numColors + (int)threadIdx.x; c <= kMaxColors; c += blockDim.x) w.a.colorStart[c] = carry;
   }
-  if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+  if (!coloring_barrier(w, arrivals)) return;
   for (int c = threadIdx.x; c < numColors; c += blockDim.x)
     base[c] = w.a.colorStart[c] + w.a.blockHist[blockIdx.x * kMaxColors + c];
   __syncthreads();
@@ -746,8 +715,8 @@ __device__ void coloring_finish(const World &w) {
       for (int k = threadIdx.x; k < warpLen[q]; k += blockDim.x) atomicAdd(&base[warpList[q][k].x], warpList[q][k].y);
     __syncthreads();
   }
-  if (!grid_barrier(ctl, w.p.barrierLimit)) return;
-  lane_layout(w);
+  if (!coloring_barrier(w, arrivals)) return;
+  lane_layout(w, arrivals);
 }
 
 // Smallest colour no neighbour of higher priority holds, searched in windows
@@ -770,11 +739,12 @@ __global__ void __launch_bounds__(256) coloring_kernel(World w) {
   const int n = w.b.n;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   volatile int *color = w.b.color;
+  unsigned arrivals = 0;
   // an uploaded colouring (copied and checked by the kernels before this
   // one) is used when proper; otherwise the priority colouring is computed
   if (w.a.colorOverride) {
     if (*((volatile int *)&ctl->colorBad) == 0) {
-      coloring_finish(w);
+      coloring_finish(w, arrivals);
       return;
     }
     if (tid == 0) atomicOr(&ctl->flags, kErrColoring);
@@ -791,7 +761,7 @@ __global__ void __launch_bounds__(256) coloring_kernel(World w) {
   int round = 0;
   for (;; round++) {
     if (tid == 0) ctl->pad[1 + (round + 1) % 3] = 0;
-    if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+    if (!coloring_barrier(w, arrivals)) return;
     int changed = 0;
     for (int i = tid; i < n; i += stride) {
       if (!(w.b.flags0[i] & kBodyDynamic)) continue;
@@ -813,7 +783,7 @@ __global__ void __launch_bounds__(256) coloring_kernel(World w) {
       }
     }
     if (changed) atomicOr(&ctl->pad[1 + round % 3], 1);
-    if (!grid_barrier(ctl, w.p.barrierLimit)) return;
+    if (!coloring_barrier(w, arrivals)) return;
     const int any = *((volatile int *)&ctl->pad[1 + round % 3]);
     if (!any) break;
     if (round > 4096) {
@@ -821,7 +791,7 @@ __global__ void __launch_bounds__(256) coloring_kernel(World w) {
       break;
     }
   }
-  coloring_finish(w);
+  coloring_finish(w, arrivals);
 }
 
 // ---------------------------------------------------------------------------
@@ -2344,7 +2314,11 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
   for (int c = 0; c < tail && active < (int)gridDim.x; c++)
     active = min((int)gridDim.x, max(active, (chunkAt(c + 1) - chunkAt(c)) * (wide(c) ? kWideSplit : 1)));
   if (jb >= active) return;
-  // this thread's lane of a chunk (wide form: of a unit of 32 lanes)
+  // this thread's lane of a chunk (wide form: of a unit of 32 lanes), looked up
+  // while the block waits at the barrier before (two dependent loads: the
+  // crushed 36-layer pyramid's solve 4.53 -> 4.39 ms, a 163,000-body batch's
+  // 1.97 -> 1.90; with the contacts' constants requested there too, what is
+  // live across the barrier spills and a phase is 10 % slower)
   int e = -1;
   int4 rec0 = make_int4(0, 0, 0, 0);
   bool wd = false;
@@ -2408,11 +2382,11 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
                             vel, maxG, f64);
         }
       }
-      solve_arrive(ctl);
+      grid_arrive(&ctl->solveArrivals);
       if (c + 1 < tail) first(c + 1);
       else if (it + 1 < total && tail == numColors) first(0);
       arrivals += active;
-      if (!solve_wait(ctl, arrivals, w.p.barrierLimit)) return;
+      if (!grid_wait(ctl, &ctl->solveArrivals, arrivals, w.p.barrierLimit)) return;
     }
     if (tail < numColors) {  // the tail segment of iteration it
       int c = tail;
@@ -2439,10 +2413,10 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
           solve_body_staged<E, J>(w, rec, lane, G, mask, alphaF, dual, vel, stage, &tw);
         }
       }
-      solve_arrive(ctl);
+      grid_arrive(&ctl->solveArrivals);
       if (it + 1 < total && tail > 0) first(0);
       arrivals += active;
-      if (!solve_wait(ctl, arrivals, w.p.barrierLimit)) return;
+      if (!grid_wait(ctl, &ctl->solveArrivals, arrivals, w.p.barrierLimit)) return;
     }
   }
 }
@@ -2572,14 +2546,13 @@ void launch_prepare(const World &w, cudaStream_t st, int smCount) {
   adj_sort_kernel<<<blocks, 256, 0, st>>>(w);
 }
 
-static int coloring_blocks(int smCount) {
+// A block per 64 bodies, so that a small scene's dozen barriers wait for few
+// blocks (a pile of 200 bodies: four), at most two blocks an SM.
+int coloring_grid(int n, int smCount) {
   int perSm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, coloring_kernel, 256, 0);
-  if (perSm > 2) perSm = 2;
-  return perSm * smCount;
+  return std::max(1, std::min((n + 63) / 64, std::min(perSm, 2) * smCount));
 }
-
-int coloring_grid(int smCount) { return coloring_blocks(smCount); }
 
 // An uploaded colouring: copied, then checked against this step's graph.
 __global__ void color_copy_kernel(World w) {
