@@ -69,6 +69,16 @@ struct avbd_ctx {
   // a non-finite position of an upload (hBad: its pinned copy)
   double *d64 = nullptr;
   int *dBad = nullptr, *hBad = nullptr;
+  // small worlds (kSmallBodies): the per-step state of bodies, joints and
+  // springs in pinned host memory, which one kernel reads or writes in place
+  struct SmallState {
+    double *d64 = nullptr;  // as the device's d64
+    D4 *lamLin, *lamAng;
+    float4 *penLin, *penAng;
+    double *peak;
+    int *jState, *sState;
+    float *sPen;
+  } small;
   // of the latest completed step (pinned, written by the stream): [0] steps
   // skipped for a candidate overflow since the last regrow, [1] candidates
   int *hCand = nullptr;
@@ -157,6 +167,8 @@ void free_all(avbd_ctx *ctx) {
   ctx->hCand = nullptr;
   if (ctx->hBad) cudaFreeHost(ctx->hBad);
   ctx->hBad = nullptr;
+  if (ctx->small.d64) cudaFreeHost(ctx->small.d64);
+  ctx->small.d64 = nullptr;
   ctx->d64 = nullptr;  // (in allocs)
   ctx->dBad = nullptr;
   ctx->packed = false;
@@ -314,35 +326,114 @@ __global__ void state_check_kernel(const double *pos, int n, int *bad) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     if (!(isfinite(pos[i * 3]) && isfinite(pos[i * 3 + 1]) && isfinite(pos[i * 3 + 2]))) atomicMin(bad, i);
 }
-__global__ void state_in_kernel(const double *d64, int n, unsigned present, const int *bad, D4 *pos, float4 *quat,
-                                float4 *vel, float4 *omega, float4 *prev) {
-  if (*bad < n) return;  // a non-finite position: the state stays as it was
+// Worlds of at most this many bodies, joints and springs exchange their state
+// through pinned memory that a kernel of one block reads or writes in place:
+// a call is one launch and one wait, where the copies are five to thirteen of
+// some 8 us each. Write / read in us, with the copies and with the kernel:
+// 64 bodies 35 / 53 and 17 / 12, with 63 joints 73 / 101 and 20 / 14; 2,048
+// bodies 50 / 58 and 28 / 32; 4,096 bodies 76 / 57 and 46 / 54; 8,192 bodies
+// 80 / 61 and 82 / 104, more than one block should move.
+constexpr int kSmallBodies = 2048;
+
+size_t small_state_bytes(size_t n, size_t nj, size_t ns) {
+  return 16 * n * sizeof(double) + nj * (2 * sizeof(D4) + 2 * sizeof(float4) + sizeof(int)) +
+         ns * (sizeof(double) + sizeof(int) + sizeof(float));
+}
+
+int alloc_small_state(avbd_ctx *ctx) {
+  if (ctx->n > kSmallBodies || ctx->nj > kSmallBodies || ctx->ns > kSmallBodies) return AVBD_OK;
+  const size_t n = ctx->n, nj = ctx->nj, ns = ctx->ns;
+  auto &h = ctx->small;
+  CK(cudaMallocHost((void **)&h.d64, small_state_bytes(n, nj, ns)));
+  // in decreasing alignment
+  h.lamLin = reinterpret_cast<D4 *>(h.d64 + 16 * n);
+  h.lamAng = h.lamLin + nj;
+  h.penLin = reinterpret_cast<float4 *>(h.lamAng + nj);
+  h.penAng = h.penLin + nj;
+  h.peak = reinterpret_cast<double *>(h.penAng + nj);
+  h.jState = reinterpret_cast<int *>(h.peak + ns);
+  h.sState = h.jState + nj;
+  h.sPen = reinterpret_cast<float *>(h.sState + ns);
+  return AVBD_OK;
+}
+
+__device__ __forceinline__ void state_in(const double *d64, int i, int n, unsigned present, const Bodies &b) {
   const double *p = d64, *q = d64 + 3 * (size_t)n, *v = q + 4 * (size_t)n, *om = v + 3 * (size_t)n,
                *pv = om + 3 * (size_t)n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    pos[i] = mkd4(p[i * 3], p[i * 3 + 1], p[i * 3 + 2], 0.0);
-    quat[i] = present & 1u ? make_float4((float)q[i * 4], (float)q[i * 4 + 1], (float)q[i * 4 + 2], (float)q[i * 4 + 3])
+  b.pos[i] = mkd4(p[i * 3], p[i * 3 + 1], p[i * 3 + 2], 0.0);
+  b.quat[i] = present & 1u ? make_float4((float)q[i * 4], (float)q[i * 4 + 1], (float)q[i * 4 + 2], (float)q[i * 4 + 3])
                            : make_float4(0.f, 0.f, 0.f, 1.f);
-    const float4 vv = present & 2u ? make_float4((float)v[i * 3], (float)v[i * 3 + 1], (float)v[i * 3 + 2], 0.f)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
-    vel[i] = vv;
-    omega[i] = present & 4u ? make_float4((float)om[i * 3], (float)om[i * 3 + 1], (float)om[i * 3 + 2], 0.f)
+  const float4 vv = present & 2u ? make_float4((float)v[i * 3], (float)v[i * 3 + 1], (float)v[i * 3 + 2], 0.f)
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+  b.vel[i] = vv;
+  b.omega[i] = present & 4u ? make_float4((float)om[i * 3], (float)om[i * 3 + 1], (float)om[i * 3 + 2], 0.f)
                             : make_float4(0.f, 0.f, 0.f, 0.f);
-    prev[i] = present & 8u ? make_float4((float)pv[i * 3], (float)pv[i * 3 + 1], (float)pv[i * 3 + 2], 0.f) : vv;
+  b.prevVel[i] = present & 8u ? make_float4((float)pv[i * 3], (float)pv[i * 3 + 1], (float)pv[i * 3 + 2], 0.f) : vv;
+}
+__device__ __forceinline__ void state_out(double *d64, int i, int n, const Bodies &b) {
+  double *p = d64, *q = d64 + 3 * (size_t)n, *v = q + 4 * (size_t)n, *om = v + 3 * (size_t)n, *pv = om + 3 * (size_t)n;
+  const D4 a = b.pos[i];
+  p[i * 3] = a.x; p[i * 3 + 1] = a.y; p[i * 3 + 2] = a.z;
+  const float4 t = b.quat[i];
+  q[i * 4] = t.x; q[i * 4 + 1] = t.y; q[i * 4 + 2] = t.z; q[i * 4 + 3] = t.w;
+  const float4 c = b.vel[i], d = b.omega[i], e = b.prevVel[i];
+  v[i * 3] = c.x; v[i * 3 + 1] = c.y; v[i * 3 + 2] = c.z;
+  om[i * 3] = d.x; om[i * 3 + 1] = d.y; om[i * 3 + 2] = d.z;
+  pv[i * 3] = e.x; pv[i * 3 + 1] = e.y; pv[i * 3 + 2] = e.z;
+}
+
+__global__ void state_in_kernel(const double *d64, unsigned present, const int *bad, Bodies b) {
+  if (*bad < b.n) return;  // a non-finite position: the state stays as it was
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < b.n; i += gridDim.x * blockDim.x)
+    state_in(d64, i, b.n, present, b);
+}
+__global__ void state_out_kernel(Bodies b, double *d64) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < b.n; i += gridDim.x * blockDim.x) state_out(d64, i, b.n, b);
+}
+
+// One block: the positions checked first (the first body with a non-finite one
+// goes to *bad, and the state stays as it was), then everything converted.
+__global__ void __launch_bounds__(1024) small_in_kernel(const __grid_constant__ World w, avbd_ctx::SmallState h,
+                                                        unsigned present, int *bad) {
+  __shared__ int first;
+  const int n = w.b.n;
+  if (threadIdx.x == 0) first = 0x7fffffff;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double *p = h.d64 + 3 * i;
+    if (!(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]))) atomicMin(&first, i);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *bad = first;
+  if (first < n) return;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) state_in(h.d64, i, n, present, w.b);
+  for (int j = threadIdx.x; j < w.j.n; j += blockDim.x) {
+    w.j.penLin[j] = h.penLin[j];
+    w.j.penAng[j] = h.penAng[j];
+    w.j.lamLin[j] = h.lamLin[j];
+    w.j.lamAng[j] = h.lamAng[j];
+    w.j.state[j] = h.jState[j];
+  }
+  for (int s = threadIdx.x; s < w.s.n; s += blockDim.x) {
+    w.s.penalty[s] = h.sPen[s];
+    w.s.peak[s] = h.peak[s];
+    w.s.state[s] = h.sState[s];
   }
 }
-__global__ void state_out_kernel(const D4 *pos, const float4 *quat, const float4 *vel, const float4 *omega,
-                                 const float4 *prev, int n, double *d64) {
-  double *p = d64, *q = d64 + 3 * (size_t)n, *v = q + 4 * (size_t)n, *om = v + 3 * (size_t)n, *pv = om + 3 * (size_t)n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const D4 a = pos[i];
-    p[i * 3] = a.x; p[i * 3 + 1] = a.y; p[i * 3 + 2] = a.z;
-    const float4 b = quat[i];
-    q[i * 4] = b.x; q[i * 4 + 1] = b.y; q[i * 4 + 2] = b.z; q[i * 4 + 3] = b.w;
-    const float4 c = vel[i], d = omega[i], e = prev[i];
-    v[i * 3] = c.x; v[i * 3 + 1] = c.y; v[i * 3 + 2] = c.z;
-    om[i * 3] = d.x; om[i * 3 + 1] = d.y; om[i * 3 + 2] = d.z;
-    pv[i * 3] = e.x; pv[i * 3 + 1] = e.y; pv[i * 3 + 2] = e.z;
+__global__ void __launch_bounds__(1024) small_out_kernel(const __grid_constant__ World w, avbd_ctx::SmallState h) {
+  const int n = w.b.n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) state_out(h.d64, i, n, w.b);
+  for (int j = threadIdx.x; j < w.j.n; j += blockDim.x) {
+    h.penLin[j] = w.j.penLin[j];
+    h.penAng[j] = w.j.penAng[j];
+    h.lamLin[j] = w.j.lamLin[j];
+    h.lamAng[j] = w.j.lamAng[j];
+    h.jState[j] = w.j.state[j];
+  }
+  for (int s = threadIdx.x; s < w.s.n; s += blockDim.x) {
+    h.sPen[s] = w.s.penalty[s];
+    h.peak[s] = w.s.peak[s];
+    h.sState[s] = w.s.state[s];
   }
 }
 
@@ -351,31 +442,10 @@ int write_state(avbd_ctx *ctx, const avbd_world *world, bool keepManifolds) {
   const int n = ctx->n;
   World &w = ctx->w;
   cudaStream_t st = ctx->stream;
-  {  // the caller's arrays straight to the device (GB300: host memory over NVLink-C2C), converted there
-    const size_t N = (size_t)n;
-    double *p = ctx->d64, *q = p + 3 * N, *v = q + 4 * N, *om = v + 3 * N, *pv = om + 3 * N;
-    const unsigned present = (B.quat ? 1u : 0u) | (B.vel ? 2u : 0u) | (B.omega ? 4u : 0u) | (B.prev_vel ? 8u : 0u);
-    CK(cudaMemcpyAsync(p, B.pos, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
-    if (B.quat) CK(cudaMemcpyAsync(q, B.quat, 4 * N * sizeof(double), cudaMemcpyHostToDevice, st));
-    if (B.vel) CK(cudaMemcpyAsync(v, B.vel, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
-    if (B.omega) CK(cudaMemcpyAsync(om, B.omega, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
-    if (B.prev_vel) CK(cudaMemcpyAsync(pv, B.prev_vel, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(ctx->dBad, 0x7f, sizeof(int), st));  // 0x7f7f7f7f: above any body index
-    const int grid = std::max(1, std::min((n + 255) / 256, ctx->smCount * 4));
-    state_check_kernel<<<grid, 256, 0, st>>>(p, n, ctx->dBad);
-    state_in_kernel<<<grid, 256, 0, st>>>(ctx->d64, n, present, ctx->dBad, w.b.pos, w.b.quat, w.b.vel, w.b.omega,
-                                          w.b.prevVel);
-    CK(cudaMemcpyAsync(ctx->hBad, ctx->dBad, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    CK(cudaGetLastError());
-    if (*ctx->hBad < n) return fail(ctx, AVBD_ERR_NAN, "body %d: non-finite position", *ctx->hBad);
-  }
-
+  const unsigned present = (B.quat ? 1u : 0u) | (B.vel ? 2u : 0u) | (B.omega ? 4u : 0u) | (B.prev_vel ? 8u : 0u);
   const avbd_joint_soa &J = world->joints;
-  if (ctx->nj) {
-    std::vector<float4> kl(ctx->nj), ka(ctx->nj);
-    std::vector<D4> ll(ctx->nj), la(ctx->nj);
-    std::vector<int> st(ctx->nj);
+  const avbd_spring_soa &S = world->springs;
+  auto joints_in = [&](float4 *kl, float4 *ka, D4 *ll, D4 *la, int *st) {
     for (int j = 0; j < ctx->nj; j++) {
       auto f = [&](const double *a) { return a ? make_float4((float)a[j * 3], (float)a[j * 3 + 1], (float)a[j * 3 + 2], 0.f)
                                                : make_float4(0, 0, 0, 0); };
@@ -389,25 +459,68 @@ int write_state(avbd_ctx *ctx, const avbd_world *world, bool keepManifolds) {
       // the force list (Joint.initialize, src/physics/joint.js:131-160)
       st[j] = (J.broken && J.broken[j]) ? kBroken : 0;
     }
-    CK(cudaMemcpy(w.j.penLin, kl.data(), ctx->nj * sizeof(float4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(w.j.penAng, ka.data(), ctx->nj * sizeof(float4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(w.j.lamLin, ll.data(), ctx->nj * sizeof(D4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(w.j.lamAng, la.data(), ctx->nj * sizeof(D4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(w.j.state, st.data(), ctx->nj * sizeof(int), cudaMemcpyHostToDevice));
-  }
-  const avbd_spring_soa &S = world->springs;
-  if (ctx->ns) {
-    std::vector<float> pen(ctx->ns);
-    std::vector<double> peak(ctx->ns);
-    std::vector<int> st(ctx->ns);
+  };
+  auto springs_in = [&](float *pen, double *peak, int *st) {
     for (int s = 0; s < ctx->ns; s++) {
       pen[s] = S.penalty ? (float)S.penalty[s] : 0.f;
       peak[s] = S.peak_strain ? S.peak_strain[s] : 0.0;
       st[s] = (S.broken && S.broken[s]) ? kBroken : 0;
     }
-    CK(cudaMemcpy(w.s.penalty, pen.data(), ctx->ns * sizeof(float), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(w.s.peak, peak.data(), ctx->ns * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(w.s.state, st.data(), ctx->ns * sizeof(int), cudaMemcpyHostToDevice));
+  };
+  if (ctx->small.d64) {
+    const size_t N = (size_t)n;
+    auto &h = ctx->small;
+    auto put = [&](size_t at, const double *a, size_t k) {
+      if (a) std::memcpy(h.d64 + at, a, k * sizeof(double));
+    };
+    put(0, B.pos, 3 * N);
+    put(3 * N, B.quat, 4 * N);
+    put(7 * N, B.vel, 3 * N);
+    put(10 * N, B.omega, 3 * N);
+    put(13 * N, B.prev_vel, 3 * N);
+    joints_in(h.penLin, h.penAng, h.lamLin, h.lamAng, h.jState);
+    springs_in(h.sPen, h.peak, h.sState);
+    small_in_kernel<<<1, 1024, 0, st>>>(w, h, present, ctx->hBad);
+    CK(cudaStreamSynchronize(st));
+    CK(cudaGetLastError());
+    if (*ctx->hBad < n) return fail(ctx, AVBD_ERR_NAN, "body %d: non-finite position", *ctx->hBad);
+  } else {
+    // the caller's arrays straight to the device (GB300: host memory over NVLink-C2C), converted there
+    const size_t N = (size_t)n;
+    double *p = ctx->d64, *q = p + 3 * N, *v = q + 4 * N, *om = v + 3 * N, *pv = om + 3 * N;
+    CK(cudaMemcpyAsync(p, B.pos, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
+    if (B.quat) CK(cudaMemcpyAsync(q, B.quat, 4 * N * sizeof(double), cudaMemcpyHostToDevice, st));
+    if (B.vel) CK(cudaMemcpyAsync(v, B.vel, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
+    if (B.omega) CK(cudaMemcpyAsync(om, B.omega, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
+    if (B.prev_vel) CK(cudaMemcpyAsync(pv, B.prev_vel, 3 * N * sizeof(double), cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(ctx->dBad, 0x7f, sizeof(int), st));  // 0x7f7f7f7f: above any body index
+    const int grid = std::max(1, std::min((n + 255) / 256, ctx->smCount * 4));
+    state_check_kernel<<<grid, 256, 0, st>>>(p, n, ctx->dBad);
+    state_in_kernel<<<grid, 256, 0, st>>>(ctx->d64, present, ctx->dBad, w.b);
+    CK(cudaMemcpyAsync(ctx->hBad, ctx->dBad, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    CK(cudaGetLastError());
+    if (*ctx->hBad < n) return fail(ctx, AVBD_ERR_NAN, "body %d: non-finite position", *ctx->hBad);
+    if (ctx->nj) {
+      std::vector<float4> kl(ctx->nj), ka(ctx->nj);
+      std::vector<D4> ll(ctx->nj), la(ctx->nj);
+      std::vector<int> js(ctx->nj);
+      joints_in(kl.data(), ka.data(), ll.data(), la.data(), js.data());
+      CK(cudaMemcpy(w.j.penLin, kl.data(), ctx->nj * sizeof(float4), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(w.j.penAng, ka.data(), ctx->nj * sizeof(float4), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(w.j.lamLin, ll.data(), ctx->nj * sizeof(D4), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(w.j.lamAng, la.data(), ctx->nj * sizeof(D4), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(w.j.state, js.data(), ctx->nj * sizeof(int), cudaMemcpyHostToDevice));
+    }
+    if (ctx->ns) {
+      std::vector<float> pen(ctx->ns);
+      std::vector<double> peak(ctx->ns);
+      std::vector<int> ss(ctx->ns);
+      springs_in(pen.data(), peak.data(), ss.data());
+      CK(cudaMemcpy(w.s.penalty, pen.data(), ctx->ns * sizeof(float), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(w.s.peak, peak.data(), ctx->ns * sizeof(double), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(w.s.state, ss.data(), ctx->ns * sizeof(int), cudaMemcpyHostToDevice));
+    }
   }
 
   // warm-start manifolds -> the "previous step" arena, sorted by pair key
@@ -1145,6 +1258,7 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   CK(cudaMemset(w.b.color, 0, sizeof(int) * n));
   if ((rc = dalloc(ctx, &ctx->d64, (size_t)16 * n)) || (rc = dalloc(ctx, &ctx->dBad, 1))) return rc;
   CK(cudaMallocHost((void **)&ctx->hBad, sizeof(int)));
+  if ((rc = alloc_small_state(ctx))) return rc;
   // dalloc's zero fills run on the legacy default stream, which the context's
   // non-blocking stream does not wait for: finish them before the upload
   CK(cudaDeviceSynchronize());
@@ -1182,36 +1296,18 @@ int avbd_synchronize(avbd_ctx *ctx) {
 int avbd_read_state(avbd_ctx *ctx, avbd_world *out) {
   if (!ctx || !out) return AVBD_ERR_ARG;
   if (!ctx->packed) return fail(ctx, AVBD_ERR_STATE, "avbd_read_state before avbd_pack");
-  int rs = resolve_skips(ctx);  // steps skipped for an overflow run again first
-  if (rs) return rs;
   const World &w = ctx->w;
   const int n = ctx->n;
   avbd_body_soa &B = out->bodies;
-  if (B.count < n) return fail(ctx, AVBD_ERR_ARG, "avbd_read_state: body arrays hold %d < %d", B.count, n);
-  cudaStream_t st = ctx->stream;
-  {  // converted on the device, then straight into the caller's arrays
-    const size_t N = (size_t)n;
-    const double *p = ctx->d64, *q = p + 3 * N, *v = q + 4 * N, *om = v + 3 * N, *pv = om + 3 * N;
-    const int grid = std::max(1, std::min((n + 255) / 256, ctx->smCount * 4));
-    state_out_kernel<<<grid, 256, 0, st>>>(w.b.pos, w.b.quat, w.b.vel, w.b.omega, w.b.prevVel, n, ctx->d64);
-    if (B.pos) CK(cudaMemcpyAsync(B.pos, p, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (B.quat) CK(cudaMemcpyAsync(B.quat, q, 4 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (B.vel) CK(cudaMemcpyAsync(B.vel, v, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (B.omega) CK(cudaMemcpyAsync(B.omega, om, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (B.prev_vel) CK(cudaMemcpyAsync(B.prev_vel, pv, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    CK(cudaGetLastError());
+  if (B.count < n) {
+    int rs = resolve_skips(ctx);
+    if (rs) return rs;
+    return fail(ctx, AVBD_ERR_ARG, "avbd_read_state: body arrays hold %d < %d", B.count, n);
   }
+  cudaStream_t st = ctx->stream;
   avbd_joint_soa &J = out->joints;
-  if (ctx->nj && J.count >= ctx->nj) {
-    std::vector<float4> kl(ctx->nj), ka(ctx->nj);
-    std::vector<D4> ll(ctx->nj), la(ctx->nj);
-    std::vector<int> st(ctx->nj);
-    CK(cudaMemcpy(kl.data(), w.j.penLin, ctx->nj * sizeof(float4), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(ka.data(), w.j.penAng, ctx->nj * sizeof(float4), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(ll.data(), w.j.lamLin, ctx->nj * sizeof(D4), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(la.data(), w.j.lamAng, ctx->nj * sizeof(D4), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(st.data(), w.j.state, ctx->nj * sizeof(int), cudaMemcpyDeviceToHost));
+  avbd_spring_soa &SP = out->springs;
+  auto joints_out = [&](const float4 *kl, const float4 *ka, const D4 *ll, const D4 *la, const int *js) {
     for (int j = 0; j < ctx->nj; j++) {
       const float kv[6] = {kl[j].x, kl[j].y, kl[j].z, ka[j].x, ka[j].y, ka[j].z};
       const double lv[6] = {ll[j].x, ll[j].y, ll[j].z, la[j].x, la[j].y, la[j].z};
@@ -1221,21 +1317,73 @@ int avbd_read_state(avbd_ctx *ctx, avbd_world *out) {
         if (J.lambda_lin) J.lambda_lin[j * 3 + k] = lv[k];
         if (J.lambda_ang) J.lambda_ang[j * 3 + k] = lv[3 + k];
       }
-      if (J.broken) J.broken[j] = (st[j] & kBroken) ? 1 : 0;
+      if (J.broken) J.broken[j] = (js[j] & kBroken) ? 1 : 0;
     }
-  }
-  avbd_spring_soa &SP = out->springs;
-  if (ctx->ns && SP.count >= ctx->ns) {
-    std::vector<float> pen(ctx->ns);
-    std::vector<double> peak(ctx->ns);
-    std::vector<int> st(ctx->ns);
-    CK(cudaMemcpy(pen.data(), w.s.penalty, ctx->ns * sizeof(float), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(peak.data(), w.s.peak, ctx->ns * sizeof(double), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(st.data(), w.s.state, ctx->ns * sizeof(int), cudaMemcpyDeviceToHost));
+  };
+  auto springs_out = [&](const float *pen, const double *peak, const int *ss) {
     for (int s = 0; s < ctx->ns; s++) {
       if (SP.penalty) SP.penalty[s] = pen[s];
       if (SP.peak_strain) SP.peak_strain[s] = peak[s];
-      if (SP.broken) SP.broken[s] = (st[s] & kBroken) ? 1 : 0;
+      if (SP.broken) SP.broken[s] = (ss[s] & kBroken) ? 1 : 0;
+    }
+  };
+  if (ctx->small.d64) {
+    // queued behind the steps, so that one wait covers both; steps skipped for
+    // an overflow run again first, and the state is read once more
+    auto &h = ctx->small;
+    for (int round = 0;; round++) {
+      small_out_kernel<<<1, 1024, 0, st>>>(w, h);
+      CK(cudaStreamSynchronize(st));
+      CK(cudaGetLastError());
+      if (round > 0 || ctx->hCand[0] <= 0) break;
+      int rs = resolve_skips(ctx);
+      if (rs) return rs;
+    }
+    const size_t N = (size_t)n;
+    auto get = [&](double *a, size_t at, size_t k) {
+      if (a) std::memcpy(a, h.d64 + at, k * sizeof(double));
+    };
+    get(B.pos, 0, 3 * N);
+    get(B.quat, 3 * N, 4 * N);
+    get(B.vel, 7 * N, 3 * N);
+    get(B.omega, 10 * N, 3 * N);
+    get(B.prev_vel, 13 * N, 3 * N);
+    if (ctx->nj && J.count >= ctx->nj) joints_out(h.penLin, h.penAng, h.lamLin, h.lamAng, h.jState);
+    if (ctx->ns && SP.count >= ctx->ns) springs_out(h.sPen, h.peak, h.sState);
+  } else {
+    int rs = resolve_skips(ctx);  // steps skipped for an overflow run again first
+    if (rs) return rs;
+    // converted on the device, then straight into the caller's arrays
+    const size_t N = (size_t)n;
+    const double *p = ctx->d64, *q = p + 3 * N, *v = q + 4 * N, *om = v + 3 * N, *pv = om + 3 * N;
+    const int grid = std::max(1, std::min((n + 255) / 256, ctx->smCount * 4));
+    state_out_kernel<<<grid, 256, 0, st>>>(w.b, ctx->d64);
+    if (B.pos) CK(cudaMemcpyAsync(B.pos, p, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (B.quat) CK(cudaMemcpyAsync(B.quat, q, 4 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (B.vel) CK(cudaMemcpyAsync(B.vel, v, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (B.omega) CK(cudaMemcpyAsync(B.omega, om, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (B.prev_vel) CK(cudaMemcpyAsync(B.prev_vel, pv, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    CK(cudaGetLastError());
+    if (ctx->nj && J.count >= ctx->nj) {
+      std::vector<float4> kl(ctx->nj), ka(ctx->nj);
+      std::vector<D4> ll(ctx->nj), la(ctx->nj);
+      std::vector<int> js(ctx->nj);
+      CK(cudaMemcpy(kl.data(), w.j.penLin, ctx->nj * sizeof(float4), cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(ka.data(), w.j.penAng, ctx->nj * sizeof(float4), cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(ll.data(), w.j.lamLin, ctx->nj * sizeof(D4), cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(la.data(), w.j.lamAng, ctx->nj * sizeof(D4), cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(js.data(), w.j.state, ctx->nj * sizeof(int), cudaMemcpyDeviceToHost));
+      joints_out(kl.data(), ka.data(), ll.data(), la.data(), js.data());
+    }
+    if (ctx->ns && SP.count >= ctx->ns) {
+      std::vector<float> pen(ctx->ns);
+      std::vector<double> peak(ctx->ns);
+      std::vector<int> ss(ctx->ns);
+      CK(cudaMemcpy(pen.data(), w.s.penalty, ctx->ns * sizeof(float), cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(peak.data(), w.s.peak, ctx->ns * sizeof(double), cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(ss.data(), w.s.state, ctx->ns * sizeof(int), cudaMemcpyDeviceToHost));
+      springs_out(pen.data(), peak.data(), ss.data());
     }
   }
   // manifolds of the last step (now the "previous" arena)
