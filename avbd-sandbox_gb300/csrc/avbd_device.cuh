@@ -164,6 +164,11 @@ struct Joints {
   const D4 *stiff;    // stiffnessLin, stiffnessAng, fracture, torqueArm
   float4 *penLin, *penAng;
   D4 *lamLin, *lamAng;
+  // f32 copies for the FP32 solve (a conversion there runs on the FP64 pipe):
+  // the multipliers as of the last write, and x = 1 / y = 1 when the linear /
+  // angular rows are hard, z = torqueArm
+  float4 *lamLinF, *lamAngF;
+  const float4 *stiffF;
   float4 *c0Lin, *c0Ang;   // per step, C*(x_t)
   float4 *dpt;             // per step, p_A(t) - p_B(t) (or world anchor - p_B(t))
   D4 *dptD;
@@ -220,6 +225,7 @@ struct Grid {
   // static joint/spring adjacency (pack time)
   const int *cStart;
   const uint32_t *cRef;
+  const int *cOther;  // per entry of cRef: the other body (-1: a world anchor)
 };
 
 struct Adjacency {

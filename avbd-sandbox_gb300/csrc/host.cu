@@ -1039,7 +1039,8 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   std::vector<int2> jb(ctx->nj), sb(ctx->ns);
   std::vector<D4> jrA(ctx->nj), jrB(ctx->nj), jst(ctx->nj), srA(ctx->ns), srB(ctx->ns), sprm(ctx->ns);
   std::vector<float4> jrAf(ctx->nj), jrBf(ctx->nj), srAf(ctx->ns), srBf(ctx->ns);
-  std::vector<std::vector<uint32_t>> refs(n);
+  std::vector<std::vector<std::pair<uint32_t, int>>> refs(n);  // reference, the other body
+  std::vector<float4> jstF(ctx->nj);
   for (int j = 0; j < ctx->nj; j++) {
     const int a = J.body_a[j], b = J.body_b[j];
     if (b < 0 || b >= n || a >= n || a == b) return fail(ctx, AVBD_ERR_ARG, "joint %d: bad body indices", j);
@@ -1054,8 +1055,9 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
     const double sy = (a >= 0 ? B.size[a * 3 + 1] : 0) + B.size[b * 3 + 1];
     const double sz = (a >= 0 ? B.size[a * 3 + 2] : 0) + B.size[b * 3 + 2];
     jst[j] = mkd4(J.stiffness_lin[j], J.stiffness_ang[j], J.fracture[j], sx * sx + sy * sy + sz * sz);
-    if (a >= 0) refs[a].push_back(make_ref(kRefJoint, j, 0));
-    refs[b].push_back(make_ref(kRefJoint, j, 1));
+    jstF[j] = make_float4(std::isinf(jst[j].x) ? 1.f : 0.f, std::isinf(jst[j].y) ? 1.f : 0.f, (float)jst[j].w, 0.f);
+    if (a >= 0) refs[a].push_back({make_ref(kRefJoint, j, 0), b});
+    refs[b].push_back({make_ref(kRefJoint, j, 1), a});
   }
   for (int s = 0; s < ctx->ns; s++) {
     const int a = SP.body_a[s], b = SP.body_b[s];
@@ -1068,14 +1070,18 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
     srAf[s] = make_float4((float)srA[s].x, (float)srA[s].y, (float)srA[s].z, 0);
     srBf[s] = make_float4((float)srB[s].x, (float)srB[s].y, (float)srB[s].z, 0);
     sprm[s] = mkd4(SP.stiffness[s], SP.rest[s], SP.tear_strain ? SP.tear_strain[s] : INFINITY, 0);
-    refs[a].push_back(make_ref(kRefSpring, s, 0));
-    refs[b].push_back(make_ref(kRefSpring, s, 1));
+    refs[a].push_back({make_ref(kRefSpring, s, 0), b});
+    refs[b].push_back({make_ref(kRefSpring, s, 1), a});
   }
   std::vector<int> cStart(n + 1, 0);
   std::vector<uint32_t> cRef;
+  std::vector<int> cOther;
   for (int i = 0; i < n; i++) {
     cStart[i] = (int)cRef.size();
-    cRef.insert(cRef.end(), refs[i].begin(), refs[i].end());
+    for (const auto &r : refs[i]) {
+      cRef.push_back(r.first);
+      cOther.push_back(r.second < 0 ? -1 : r.second);
+    }
   }
   cStart[n] = (int)cRef.size();
 
@@ -1130,7 +1136,7 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   float4 *massFP;
   double *fricP, *invCellP;
   float *cellFP;
-  int *flags0P, *sceneP, *sceneStartP, *largeStartP, *largeListP, *cStartP;
+  int *flags0P, *sceneP, *sceneStartP, *largeStartP, *largeListP, *cStartP, *cOtherP;
   uint32_t *prioP, *cRefP;
   std::vector<float> cellF(S);
   for (int s = 0; s < S; s++) cellF[s] = (float)(1.0 / invCell[s]);
@@ -1138,7 +1144,8 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
       (rc = upload(ctx, &fricP, friction)) || (rc = upload(ctx, &flags0P, flags0)) || (rc = upload(ctx, &sceneP, scene)) ||
       (rc = upload(ctx, &prioP, prio)) || (rc = upload(ctx, &invCellP, invCell)) || (rc = upload(ctx, &cellFP, cellF)) ||
       (rc = upload(ctx, &sceneStartP, sceneStart)) || (rc = upload(ctx, &largeStartP, largeStart)) ||
-      (rc = upload(ctx, &largeListP, largeList)) || (rc = upload(ctx, &cStartP, cStart)) || (rc = upload(ctx, &cRefP, cRef)))
+      (rc = upload(ctx, &largeListP, largeList)) || (rc = upload(ctx, &cStartP, cStart)) || (rc = upload(ctx, &cRefP, cRef)) ||
+      (rc = upload(ctx, &cOtherP, cOther)))
     return rc;
   w.b.n = n;
   w.b.mat = nullptr;
@@ -1177,13 +1184,16 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   // joints
   w.j.n = ctx->nj;
   {
-    int2 *jbP; D4 *a, *b, *c; float4 *af, *bf;
+    int2 *jbP; D4 *a, *b, *c; float4 *af, *bf, *cf;
     if ((rc = upload(ctx, &jbP, jb)) || (rc = upload(ctx, &a, jrA)) || (rc = upload(ctx, &b, jrB)) ||
-        (rc = upload(ctx, &c, jst)) || (rc = upload(ctx, &af, jrAf)) || (rc = upload(ctx, &bf, jrBf)))
+        (rc = upload(ctx, &c, jst)) || (rc = upload(ctx, &af, jrAf)) || (rc = upload(ctx, &bf, jrBf)) ||
+        (rc = upload(ctx, &cf, jstF)))
       return rc;
+    w.j.stiffF = cf;
     w.j.bodies = jbP; w.j.rAD = a; w.j.rBD = b; w.j.stiff = c; w.j.rAF = af; w.j.rBF = bf;
     if ((rc = dalloc(ctx, &w.j.penLin, ctx->nj)) || (rc = dalloc(ctx, &w.j.penAng, ctx->nj)) ||
         (rc = dalloc(ctx, &w.j.lamLin, ctx->nj)) || (rc = dalloc(ctx, &w.j.lamAng, ctx->nj)) ||
+        (rc = dalloc(ctx, &w.j.lamLinF, ctx->nj)) || (rc = dalloc(ctx, &w.j.lamAngF, ctx->nj)) ||
         (rc = dalloc(ctx, &w.j.c0Lin, ctx->nj)) || (rc = dalloc(ctx, &w.j.c0Ang, ctx->nj)) ||
         (rc = dalloc(ctx, &w.j.dpt, ctx->nj)) || (rc = dalloc(ctx, &w.j.dptD, ctx->nj)) ||
         (rc = dalloc(ctx, &w.j.state, ctx->nj)))
@@ -1206,7 +1216,7 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   w.g.sceneStart = sceneStartP; w.g.invCell = invCellP; w.g.cellF = cellFP; w.g.largeStart = largeStartP; w.g.largeList = largeListP;
   w.g.maxChunks = maxChunks;
   if ((rc = dalloc(ctx, &w.g.largeChunk, (size_t)std::max(ctx->numLarge, 1) * maxChunks))) return rc;
-  w.g.cStart = cStartP; w.g.cRef = cRefP;
+  w.g.cStart = cStartP; w.g.cRef = cRefP; w.g.cOther = cOtherP;
   w.g.tableMask = (unsigned)(ctx->tableSize - 1);
   w.g.entryCap = ctx->entryCap;
   w.g.candCap = ctx->candCap;

@@ -158,6 +158,8 @@ __global__ void prepare_forces_kernel(World w) {
     }
     w.j.lamLin[j] = ll;
     w.j.lamAng[j] = la;
+    w.j.lamLinF[j] = make_float4((float)ll.x, (float)ll.y, (float)ll.z, 0.f);
+    w.j.lamAngF[j] = make_float4((float)la.x, (float)la.y, (float)la.z, 0.f);
     float4 kl = w.j.penLin[j], ka = w.j.penAng[j];
     auto warm = [&](float k, double cap) {
       return (float)jsmin(clampd((double)k * P.gamma, P.penaltyMin, P.penaltyMax), cap);
@@ -1251,33 +1253,86 @@ struct JointGeo {
   V3<T> rAw, rBw;
 };
 
+// What a joint's rows and dual update read beside the two states, requested
+// at once (with a load a branch, a bonded brick's joint rows took 9,700 cycles
+// and its dual updates 10,100 of a 31,000-cycle phase, most of it waiting; with
+// this and the f32 copies the solve of 16 x 16 bonded bricks went from 1,109
+// to 844 us).
 template <class T>
-__device__ __forceinline__ JointGeo<T> joint_geo(const World &w, int j, int2 ab, const BState<T> &A, const BState<T> &B,
-                                        bool hasA) {
+struct JointData {
+  int state;
+  float4 kl, ka, c0l, c0a;
+  V3<T> dpt, rA, rB;
+  bool hardLin, hardAng;
+  T arm;
+};
+
+__device__ __forceinline__ V3<float> load_v3(const float4 *f, const D4 *, int j, float) { return f3(ld(&f[j])); }
+__device__ __forceinline__ V3<double> load_v3(const float4 *, const D4 *d, int j, double) { return d3(ld(&d[j])); }
+
+template <class T>
+__device__ __forceinline__ JointData<T> load_joint(const World &w, int j) {
+  JointData<T> d;
+  d.state = __ldcg(&w.j.state[j]);
+  d.kl = __ldcg(&w.j.penLin[j]);
+  d.ka = __ldcg(&w.j.penAng[j]);
+  d.c0l = ld(&w.j.c0Lin[j]);
+  d.c0a = ld(&w.j.c0Ang[j]);
+  d.dpt = load_v3(w.j.dpt, w.j.dptD, j, T(0));
+  d.rA = load_v3(w.j.rAF, w.j.rAD, j, T(0));
+  d.rB = load_v3(w.j.rBF, w.j.rBD, j, T(0));
+  const float4 sf = ld(&w.j.stiffF[j]);
+  d.hardLin = sf.x != 0.f;
+  d.hardAng = sf.y != 0.f;
+  if constexpr (sizeof(T) == 4) d.arm = sf.z;
+  else d.arm = ld(&w.j.stiff[j]).w;
+  return d;
+}
+
+// qsub with its sums fused in a fixed order: where it is inlined the compiler
+// picks which of two products of a sum it fuses, and the primal rows and the
+// dual update of a joint have to see the same angle.
+__device__ __forceinline__ V3<float> joint_angle(Q4<float> a, Q4<float> b) {
+  const float r = 1.f / __fmaf_rn(b.w, b.w, __fmaf_rn(b.z, b.z, __fmaf_rn(b.x, b.x, __fmul_rn(b.y, b.y))));
+  const float ix = -b.x * r, iy = -b.y * r, iz = -b.z * r, iw = b.w * r;
+  return V3<float>{__fmaf_rn(-a.z, iy, __fmaf_rn(a.y, iz, __fmaf_rn(a.w, ix, __fmul_rn(a.x, iw)))) * 2.f,
+                   __fmaf_rn(a.z, ix, __fmaf_rn(a.y, iw, __fmaf_rn(a.w, iy, -__fmul_rn(a.x, iz)))) * 2.f,
+                   __fmaf_rn(a.z, iw, __fmaf_rn(-a.y, ix, __fmaf_rn(a.w, iz, __fmul_rn(a.x, iy)))) * 2.f};
+}
+__device__ __forceinline__ V3<double> joint_angle(Q4<double> a, Q4<double> b) { return qsub(a, b); }
+
+template <class T>
+__device__ __forceinline__ JointGeo<T> joint_geo(const JointData<T> &d, const BState<T> &A, const BState<T> &B,
+                                                 bool hasA) {
   JointGeo<T> g;
-  V3<T> dpt;
-  if (sizeof(T) == 8) {
-    const D4 d = ld(&w.j.dptD[j]);
-    dpt = V3<T>{(T)d.x, (T)d.y, (T)d.z};
-  } else {
-    const float4 d = ld(&w.j.dpt[j]);
-    dpt = V3<T>{(T)d.x, (T)d.y, (T)d.z};
-  }
-  const float4 ra = ld(&w.j.rAF[j]), rb = ld(&w.j.rBF[j]);
-  const D4 raD = ld(&w.j.rAD[j]), rbD = ld(&w.j.rBD[j]);
-  const V3<T> rAl = sizeof(T) == 8 ? V3<T>{(T)raD.x, (T)raD.y, (T)raD.z} : V3<T>{(T)ra.x, (T)ra.y, (T)ra.z};
-  const V3<T> rBl = sizeof(T) == 8 ? V3<T>{(T)rbD.x, (T)rbD.y, (T)rbD.z} : V3<T>{(T)rb.x, (T)rb.y, (T)rb.z};
-  g.rBw = qrotate(B.q, rBl);
+  g.rBw = qrotate(B.q, d.rB);
   if (hasA) {
-    g.rAw = qrotate(A.q, rAl);
-    g.Clin = ((dpt + (A.dp - B.dp)) + g.rAw) - g.rBw;
+    g.rAw = qrotate(A.q, d.rA);
+    g.Clin = ((d.dpt + (A.dp - B.dp)) + g.rAw) - g.rBw;
   } else {
     g.rAw = V3<T>{0, 0, 0};
-    g.Clin = (dpt - B.dp) - g.rBw;
+    g.Clin = (d.dpt - B.dp) - g.rBw;
   }
   const Q4<T> qA = hasA ? A.q : Q4<T>{0, 0, 0, 1};
-  g.Cang = qsub(qA, B.q) * (T)ld(&w.j.stiff[j]).w;
+  g.Cang = joint_angle(qA, B.q) * d.arm;
   return g;
+}
+
+// C - alpha c0, fused so that it rounds once wherever it is inlined (next to
+// the product that C is, the compiler would be free to fuse that one instead).
+__device__ __forceinline__ V3<float> less_alpha(V3<float> C, float4 c0, float alpha) {
+  return V3<float>{__fmaf_rn(-c0.x, alpha, C.x), __fmaf_rn(-c0.y, alpha, C.y), __fmaf_rn(-c0.z, alpha, C.z)};
+}
+__device__ __forceinline__ V3<double> less_alpha(V3<double> C, float4 c0, double alpha) {
+  return V3<double>{fma(-(double)c0.x, alpha, C.x), fma(-(double)c0.y, alpha, C.y), fma(-(double)c0.z, alpha, C.z)};
+}
+
+// A joint's or spring's other body: its state, or nothing for a world anchor.
+template <class T>
+__device__ __forceinline__ BState<T> load_partner(const World &w, int other) {
+  BState<T> o;
+  if (other >= 0) o = load_state<T>(w, other);
+  return o;
 }
 
 // The linear rows of a ball socket on one of its bodies (joint.js:162-221):
@@ -1346,37 +1401,43 @@ __device__ __noinline__ Sys<T> grab_primal(const World &w, int i, const BState<T
 }
 
 template <class T>
-__device__ __forceinline__ void joint_primal(const World &w, int j, int side, const BState<T> &self, T alpha, Sys<T> &s) {
-  if (__ldcg(&w.j.state[j])) return;
-  const int2 ab = ld(&w.j.bodies[j]);
-  const bool hasA = ab.x >= 0;
-  BState<T> o;
-  if (side == 0) o = load_state<T>(w, ab.y);
-  else if (hasA) o = load_state<T>(w, ab.x);
+__device__ __forceinline__ V3<T> joint_lambda(const float4 *f, const D4 *d, int j) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 v = __ldcg(&f[j]);
+    return V3<T>{v.x, v.y, v.z};
+  } else {
+    const D4 v = ldcg(&d[j]);
+    return V3<T>{v.x, v.y, v.z};
+  }
+}
+
+template <class T>
+__device__ __forceinline__ void joint_primal(const World &w, int j, int side, int other, const BState<T> &self, T alpha,
+                                             Sys<T> &s) {
+  const JointData<T> d = load_joint<T>(w, j);
+  const V3<T> ll = joint_lambda<T>(w.j.lamLinF, w.j.lamLin, j), la = joint_lambda<T>(w.j.lamAngF, w.j.lamAng, j);
+  const BState<T> o = load_partner<T>(w, other);
+  if (d.state) return;
+  const bool hasA = side == 0 || other >= 0;
   const BState<T> &A = side ? o : self;
   const BState<T> &B = side ? self : o;
-  const JointGeo<T> g = joint_geo(w, j, ab, A, B, hasA);
-  const D4 sf = ld(&w.j.stiff[j]);
-  const float4 kl = __ldcg(&w.j.penLin[j]);
+  const JointGeo<T> g = joint_geo(d, A, B, hasA);
+  const float4 kl = d.kl;
   if (kl.x * kl.x + kl.y * kl.y + kl.z * kl.z > 0.f) {
-    const D4 lam = ldcg(&w.j.lamLin[j]);
-    const float4 c0 = ld(&w.j.c0Lin[j]);
     V3<T> C = g.Clin;
-    if (isinf(sf.x)) C = C - V3<T>{(T)c0.x, (T)c0.y, (T)c0.z} * alpha;
+    if (d.hardLin) C = less_alpha(C, d.c0l, alpha);
     const T K[3] = {(T)kl.x, (T)kl.y, (T)kl.z};
-    const T F[3] = {K[0] * C.x + (T)lam.x, K[1] * C.y + (T)lam.y, K[2] * C.z + (T)lam.z};
+    const T F[3] = {K[0] * C.x + ll.x, K[1] * C.y + ll.y, K[2] * C.z + ll.z};
     // A: jLin = I, jAng = skew(-rAw), r = rAw ; B: jLin = -I, jAng = skew(rBw), r = -rBw
     stamp_ball_socket<T>(s, K, F, side ? g.rBw : -g.rAw, side ? -g.rBw : g.rAw, side ? T(-1) : T(1));
   }
-  const float4 ka = __ldcg(&w.j.penAng[j]);
+  const float4 ka = d.ka;
   if (ka.x * ka.x + ka.y * ka.y + ka.z * ka.z > 0.f) {
-    const D4 lam = ldcg(&w.j.lamAng[j]);
-    const float4 c0 = ld(&w.j.c0Ang[j]);
     V3<T> C = g.Cang;
-    if (isinf(sf.y)) C = C - V3<T>{(T)c0.x, (T)c0.y, (T)c0.z} * alpha;
-    const T st = side ? -(T)sf.w : (T)sf.w;
+    if (d.hardAng) C = less_alpha(C, d.c0a, alpha);
+    const T st = side ? -d.arm : d.arm;
     const T K[3] = {(T)ka.x, (T)ka.y, (T)ka.z};
-    const T F[3] = {K[0] * C.x + (T)lam.x, K[1] * C.y + (T)lam.y, K[2] * C.z + (T)lam.z};
+    const T F[3] = {K[0] * C.x + la.x, K[1] * C.y + la.y, K[2] * C.z + la.z};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       s.a[L(a, a)] += st * K[a] * st;
@@ -1386,49 +1447,45 @@ __device__ __forceinline__ void joint_primal(const World &w, int j, int side, co
 }
 
 template <class T>
-__device__ __forceinline__ void joint_dual(const World &w, int j, int side, const BState<T> &self, T alpha) {
-  if (__ldcg(&w.j.state[j])) return;
-  const int2 ab = ld(&w.j.bodies[j]);
-  const bool hasA = ab.x >= 0;
-  BState<T> o;
-  if (side == 0) o = load_state<T>(w, ab.y);
-  else if (hasA) o = load_state<T>(w, ab.x);
+__device__ __forceinline__ void joint_dual(const World &w, int j, int side, int other, const BState<T> &self, T alpha) {
+  const JointData<T> d = load_joint<T>(w, j);
+  const D4 sf = ld(&w.j.stiff[j]);
+  D4 ll = ldcg(&w.j.lamLin[j]), la = ldcg(&w.j.lamAng[j]);
+  const BState<T> o = load_partner<T>(w, other);
+  if (d.state) return;
+  const bool hasA = side == 0 || other >= 0;
   const BState<T> &A = side ? o : self;
   const BState<T> &B = side ? self : o;
-  const JointGeo<T> g = joint_geo(w, j, ab, A, B, hasA);
-  const D4 sf = ld(&w.j.stiff[j]);
+  const JointGeo<T> g = joint_geo(d, A, B, hasA);
   const double kmax = w.p.penaltyMax;
-  float4 kl = __ldcg(&w.j.penLin[j]);
-  D4 ll = ldcg(&w.j.lamLin[j]);
+  float4 kl = d.kl;
   if (kl.x * kl.x + kl.y * kl.y + kl.z * kl.z > 0.f) {
     V3<T> C = g.Clin;
-    if (isinf(sf.x)) {
-      const float4 c0 = ld(&w.j.c0Lin[j]);
-      C = C - V3<T>{(T)c0.x, (T)c0.y, (T)c0.z} * alpha;
+    if (d.hardLin) {
+      C = less_alpha(C, d.c0l, alpha);
       ll.x = (double)kl.x * (double)C.x + ll.x;
       ll.y = (double)kl.y * (double)C.y + ll.y;
       ll.z = (double)kl.z * (double)C.z + ll.z;
     }
-    const double cap = fmin(sf.x, kmax);
-    kl.x = (float)fmin((double)kl.x + w.p.betaLin * fabs((double)C.x), cap);
-    kl.y = (float)fmin((double)kl.y + w.p.betaLin * fabs((double)C.y), cap);
-    kl.z = (float)fmin((double)kl.z + w.p.betaLin * fabs((double)C.z), cap);
+    // (a minimum of rounded values is the rounded minimum)
+    const float cap = (float)fmin(sf.x, kmax);
+    kl.x = fminf((float)((double)kl.x + w.p.betaLin * fabs((double)C.x)), cap);
+    kl.y = fminf((float)((double)kl.y + w.p.betaLin * fabs((double)C.y)), cap);
+    kl.z = fminf((float)((double)kl.z + w.p.betaLin * fabs((double)C.z)), cap);
   }
-  float4 ka = __ldcg(&w.j.penAng[j]);
-  D4 la = ldcg(&w.j.lamAng[j]);
+  float4 ka = d.ka;
   if (ka.x * ka.x + ka.y * ka.y + ka.z * ka.z > 0.f) {
     V3<T> C = g.Cang;
-    if (isinf(sf.y)) {
-      const float4 c0 = ld(&w.j.c0Ang[j]);
-      C = C - V3<T>{(T)c0.x, (T)c0.y, (T)c0.z} * alpha;
+    if (d.hardAng) {
+      C = less_alpha(C, d.c0a, alpha);
       la.x = (double)ka.x * (double)C.x + la.x;
       la.y = (double)ka.y * (double)C.y + la.y;
       la.z = (double)ka.z * (double)C.z + la.z;
     }
-    const double cap = fmin(sf.y, kmax);
-    ka.x = (float)fmin((double)ka.x + w.p.betaAng * fabs((double)C.x), cap);
-    ka.y = (float)fmin((double)ka.y + w.p.betaAng * fabs((double)C.y), cap);
-    ka.z = (float)fmin((double)ka.z + w.p.betaAng * fabs((double)C.z), cap);
+    const float cap = (float)fmin(sf.y, kmax);
+    ka.x = fminf((float)((double)ka.x + w.p.betaAng * fabs((double)C.x)), cap);
+    ka.y = fminf((float)((double)ka.y + w.p.betaAng * fabs((double)C.y)), cap);
+    ka.z = fminf((float)((double)ka.z + w.p.betaAng * fabs((double)C.z)), cap);
   }
   // fracture on |lambda_ang| (joint.js:307-316)
   if (la.x * la.x + la.y * la.y + la.z * la.z > sf.z * sf.z) {
@@ -1442,6 +1499,8 @@ __device__ __forceinline__ void joint_dual(const World &w, int j, int side, cons
   __stcg(&w.j.penAng[j], ka);
   stcg(&w.j.lamLin[j], ll);
   stcg(&w.j.lamAng[j], la);
+  __stcg(&w.j.lamLinF[j], make_float4((float)ll.x, (float)ll.y, (float)ll.z, 0.f));
+  __stcg(&w.j.lamAngF[j], make_float4((float)la.x, (float)la.y, (float)la.z, 0.f));
 }
 
 // spring.js:447-458: d, |d| and C at the current iterate.
@@ -1468,10 +1527,11 @@ __device__ __forceinline__ bool spring_eval(const World &w, int sIdx, const BSta
 }
 
 template <class T>
-__device__ __forceinline__ void spring_primal(const World &w, int sIdx, int side, const BState<T> &self, Sys<T> &s) {
-  if (__ldcg(&w.s.state[sIdx])) return;
-  const int2 ab = ld(&w.s.bodies[sIdx]);
-  const BState<T> o = load_state<T>(w, side ? ab.x : ab.y);
+__device__ __forceinline__ void spring_primal(const World &w, int sIdx, int side, int other, const BState<T> &self,
+                                              Sys<T> &s) {
+  const int state = __ldcg(&w.s.state[sIdx]);
+  const BState<T> o = load_state<T>(w, other);
+  if (state) return;
   const BState<T> &A = side ? o : self;
   const BState<T> &B = side ? self : o;
   V3<T> d, rAw, rBw;
@@ -1531,10 +1591,10 @@ __device__ __forceinline__ void spring_primal(const World &w, int sIdx, int side
 }
 
 template <class T>
-__device__ __forceinline__ void spring_dual(const World &w, int sIdx, int side, const BState<T> &self) {
-  if (__ldcg(&w.s.state[sIdx])) return;
-  const int2 ab = ld(&w.s.bodies[sIdx]);
-  const BState<T> o = load_state<T>(w, side ? ab.x : ab.y);
+__device__ __forceinline__ void spring_dual(const World &w, int sIdx, int side, int other, const BState<T> &self) {
+  const int state = __ldcg(&w.s.state[sIdx]);
+  const BState<T> o = load_state<T>(w, other);
+  if (state) return;
   const BState<T> &A = side ? o : self;
   const BState<T> &B = side ? self : o;
   V3<T> d, rAw, rBw;
@@ -1586,9 +1646,10 @@ __device__ __noinline__ void extra_primal(const World &w, int i, int cb, int nm,
   if (e < nm) contact_primal<T>(load_contact<T, E>(w, ld(&w.a.centry[cb + e]), alpha), self, alpha, s);
   for (e = first_extra(lane, nm, G); e < total; e += G) {
     const uint32_t ref = ld(&w.g.cRef[cStart + e - nm]);
+    const int other = ld(&w.g.cOther[cStart + e - nm]);
     const uint32_t type = ref >> 30, idx = (ref >> 1) & 0x1fffffffu, side = ref & 1u;
-    if (type == kRefJoint) joint_primal<T>(w, (int)idx, (int)side, self, alpha, s);
-    else spring_primal<T>(w, (int)idx, (int)side, self, s);
+    if (type == kRefJoint) joint_primal<T>(w, (int)idx, (int)side, other, self, alpha, s);
+    else spring_primal<T>(w, (int)idx, (int)side, other, self, s);
   }
 }
 
@@ -1615,13 +1676,12 @@ __device__ __noinline__ void extra_dual(const World &w, int i, int cb, int nm, i
   const int myColor = total > nm ? ld(&w.b.color[i]) : 0;
   for (int e = first_extra(lane, nm, G); e < total; e += G) {
     const uint32_t ref = ld(&w.g.cRef[cStart + e - nm]);
+    const int other = ld(&w.g.cOther[cStart + e - nm]);
     const uint32_t type = ref >> 30, idx = (ref >> 1) & 0x1fffffffu, side = ref & 1u;
-    const int2 ab = type == kRefJoint ? ld(&w.j.bodies[idx]) : ld(&w.s.bodies[idx]);
-    const int other = side ? ab.x : ab.y;
     const int oc = other >= 0 ? ld(&w.b.color[other]) : -1;
     if (!owns(myColor, oc)) continue;
-    if (type == kRefJoint) joint_dual<T>(w, (int)idx, (int)side, self, alpha);
-    else spring_dual<T>(w, (int)idx, (int)side, self);
+    if (type == kRefJoint) joint_dual<T>(w, (int)idx, (int)side, other, self, alpha);
+    else spring_dual<T>(w, (int)idx, (int)side, other, self);
   }
 }
 
@@ -1894,9 +1954,10 @@ __device__ __noinline__ Sys<T> constraints_primal(const World &w, int nm, int cS
                                                   const BState<T> self, T alpha, Sys<T> s) {
   for (int e = first_extra(lane, nm, G); e < total; e += G) {
     const uint32_t ref = ld(&w.g.cRef[cStart + e - nm]);
+    const int other = ld(&w.g.cOther[cStart + e - nm]);
     const uint32_t type = ref >> 30, idx = (ref >> 1) & 0x1fffffffu, side = ref & 1u;
-    if (type == kRefJoint) joint_primal<T>(w, (int)idx, (int)side, self, alpha, s);
-    else spring_primal<T>(w, (int)idx, (int)side, self, s);
+    if (type == kRefJoint) joint_primal<T>(w, (int)idx, (int)side, other, self, alpha, s);
+    else spring_primal<T>(w, (int)idx, (int)side, other, self, s);
   }
   return s;
 }
@@ -1907,13 +1968,12 @@ __device__ __noinline__ void constraints_dual(const World &w, int i, int nm, int
   const int myColor = ld(&w.b.color[i]);
   for (int e = first_extra(lane, nm, G) + part * G; e < total; e += parts * G) {
     const uint32_t ref = ld(&w.g.cRef[cStart + e - nm]);
+    const int other = ld(&w.g.cOther[cStart + e - nm]);
     const uint32_t type = ref >> 30, idx = (ref >> 1) & 0x1fffffffu, side = ref & 1u;
-    const int2 ab = type == kRefJoint ? ld(&w.j.bodies[idx]) : ld(&w.s.bodies[idx]);
-    const int other = side ? ab.x : ab.y;
     const int oc = other >= 0 ? ld(&w.b.color[other]) : -1;
     if (!owns(myColor, oc)) continue;
-    if (type == kRefJoint) joint_dual<T>(w, (int)idx, (int)side, self, alpha);
-    else spring_dual<T>(w, (int)idx, (int)side, self);
+    if (type == kRefJoint) joint_dual<T>(w, (int)idx, (int)side, other, self, alpha);
+    else spring_dual<T>(w, (int)idx, (int)side, other, self);
   }
 }
 
