@@ -96,7 +96,8 @@ struct Control {
   int gridEntries;  // grid entries handed out this step
   unsigned colorArrivals;  // arrivals at the colouring's grid barrier this step
   int prevCandidates;  // candidates (= manifold slots) of the previous step
-  int npCount[3];      // narrow-phase work lists: face, edge, exact
+  int npCount[4];      // narrow-phase work lists: face, edge, exact, late (face pairs that need the exact collider)
+  int npNext;          // the next unit of the lists
   int colorBad;        // this step's uploaded colouring has a conflict
   int laneTotal;       // lanes of one iteration's colour phases (sum over bodies)
   int pad[4];

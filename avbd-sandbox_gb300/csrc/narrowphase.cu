@@ -824,69 +824,63 @@ __global__ void __launch_bounds__(256) classify_kernel(World w) {
   }
 }
 
-// 2. Face manifolds: the exact normal and basis in f64, the clipping in f32
-//    with certified decisions; an undecided pair moves to the exact list.
-__global__ void __launch_bounds__(128) face_kernel(World w) {
-  const int total = *((volatile int *)&w.ctl->npCount[0]);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int2 e = w.g.npFace[t];
-    const int c = e.x;
-    bool refIsA = (e.y & 4) != 0;
-    int refAxis = e.y & 3;
-    const uint64_t key = w.g.candKey[c];
-    const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
-    const BodyD A = load_body(w, ia), B = load_body(w, ib);
-    if (e.y >> 8) {  // tied face axes: their exact separations decide (first largest wins)
-      const int k = exact_best_face(A, B, e.y >> 8);
-      refIsA = k < 3;
-      refAxis = refIsA ? k : k - 3;
-    }
-    // f64: the reference axis, the incident box's axes, the exact normal
-    const QD qRef = refIsA ? A.q : B.q, qInc = refIsA ? B.q : A.q;
-    const D3 e3[3] = {mk(1, 0, 0), mk(0, 1, 0), mk(0, 0, 1)};
-    const D3 refAx = rot(qRef, e3[refAxis]);
-    const D3 ibAx[3] = {rot(qInc, e3[0]), rot(qInc, e3[1]), rot(qInc, e3[2])};
-    const D3 n = Collider::axisNormal(refAx, sub(B.p, A.p));
-    double basis[9];
-    orthonormal(basis, neg(n));
-    const BoxF F = make_boxf(A, B);
-    NewContactF ncf[kMaxContacts];
-    FaceF face(F, A, B, ncf);
-    const int num = face.build(refIsA, refAxis, n, refAx, ibAx);
-    if (num < 0) {
-      push_exact(w, c);
-      continue;
-    }
-    write_box_manifold(w, c, ia, ib, A, B, ncf, num, basis);
+// 2. A face manifold: the exact normal and basis in f64, the clipping in f32
+//    with certified decisions; an undecided pair moves to the late list.
+__device__ __noinline__ void face_pair(const World &w, int t) {
+  const int2 e = w.g.npFace[t];
+  const int c = e.x;
+  bool refIsA = (e.y & 4) != 0;
+  int refAxis = e.y & 3;
+  const uint64_t key = w.g.candKey[c];
+  const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
+  const BodyD A = load_body(w, ia), B = load_body(w, ib);
+  if (e.y >> 8) {  // tied face axes: their exact separations decide (first largest wins)
+    const int k = exact_best_face(A, B, e.y >> 8);
+    refIsA = k < 3;
+    refAxis = refIsA ? k : k - 3;
   }
+  // f64: the reference axis, the incident box's axes, the exact normal
+  const QD qRef = refIsA ? A.q : B.q, qInc = refIsA ? B.q : A.q;
+  const D3 e3[3] = {mk(1, 0, 0), mk(0, 1, 0), mk(0, 0, 1)};
+  const D3 refAx = rot(qRef, e3[refAxis]);
+  const D3 ibAx[3] = {rot(qInc, e3[0]), rot(qInc, e3[1]), rot(qInc, e3[2])};
+  const D3 n = Collider::axisNormal(refAx, sub(B.p, A.p));
+  double basis[9];
+  orthonormal(basis, neg(n));
+  const BoxF F = make_boxf(A, B);
+  NewContactF ncf[kMaxContacts];
+  FaceF face(F, A, B, ncf);
+  const int num = face.build(refIsA, refAxis, n, refAx, ibAx);
+  if (num < 0) {
+    w.g.npExact[w.g.candCap - 1 - push_slot(&w.ctl->npCount[3])] = c;
+    return;
+  }
+  write_box_manifold(w, c, ia, ib, A, B, ncf, num, basis);
 }
 
 // 3. Edge-edge contacts (collide.js:475-493), exact f64.
-__global__ void __launch_bounds__(128) edge_kernel(World w) {
-  const int total = *((volatile int *)&w.ctl->npCount[1]);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int2 e = w.g.npEdge[t];
-    const int c = e.x, i = e.y / 3, j = e.y % 3;
-    const uint64_t key = w.g.candKey[c];
-    const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
-    const BodyD A = load_body(w, ia), B = load_body(w, ib);
-    NewContact nc[2];
-    Collider col(A, B, nc);
-    Collider::makeOBB(col.boxA, A);
-    Collider::makeOBB(col.boxB, B);
-    const D3 delta = sub(col.boxB.c, col.boxA.c);
-    const D3 n = Collider::axisNormal(crs(col.boxA.ax[i], col.boxB.ax[j]), delta);
-    double basis[9];
-    orthonormal(basis, neg(n));
-    const int num = col.edgeContact(i, j, n);
-    NewContactF ncf[2];
-    for (int k = 0; k < num; k++) {
-      ncf[k].feature = nc[k].feature;
-      ncf[k].ra[0] = (float)nc[k].rA.x; ncf[k].ra[1] = (float)nc[k].rA.y; ncf[k].ra[2] = (float)nc[k].rA.z;
-      ncf[k].rb[0] = (float)nc[k].rB.x; ncf[k].rb[1] = (float)nc[k].rB.y; ncf[k].rb[2] = (float)nc[k].rB.z;
-    }
-    write_box_manifold(w, c, ia, ib, A, B, ncf, num, basis);
+__device__ __noinline__ void edge_pair(const World &w, int t) {
+  const int2 e = w.g.npEdge[t];
+  const int c = e.x, i = e.y / 3, j = e.y % 3;
+  const uint64_t key = w.g.candKey[c];
+  const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
+  const BodyD A = load_body(w, ia), B = load_body(w, ib);
+  NewContact nc[2];
+  Collider col(A, B, nc);
+  Collider::makeOBB(col.boxA, A);
+  Collider::makeOBB(col.boxB, B);
+  const D3 delta = sub(col.boxB.c, col.boxA.c);
+  const D3 n = Collider::axisNormal(crs(col.boxA.ax[i], col.boxB.ax[j]), delta);
+  double basis[9];
+  orthonormal(basis, neg(n));
+  const int num = col.edgeContact(i, j, n);
+  NewContactF ncf[2];
+  for (int k = 0; k < num; k++) {
+    ncf[k].feature = nc[k].feature;
+    ncf[k].ra[0] = (float)nc[k].rA.x; ncf[k].ra[1] = (float)nc[k].rA.y; ncf[k].ra[2] = (float)nc[k].rA.z;
+    ncf[k].rb[0] = (float)nc[k].rB.x; ncf[k].rb[1] = (float)nc[k].rB.y; ncf[k].rb[2] = (float)nc[k].rB.z;
   }
+  write_box_manifold(w, c, ia, ib, A, B, ncf, num, basis);
 }
 
 // ---------------------------------------------------------------------------
@@ -894,10 +888,10 @@ __global__ void __launch_bounds__(128) edge_kernel(World w) {
 // SAT axis a lane, then a polygon vertex a lane. An FP64 warp instruction
 // costs the same for one lane as for 32, and a pair decided by one thread is
 // a chain of some 2,500 of them (150-230 us for a list of ten pairs); here it
-// is about 500 (the list of a 200-box pile: 150 -> 39 us; the narrow phase of
-// a ten-cube stack 233 -> 82 us, of the standing 53-layer pyramid 338 -> 205). Every value is formed by ColliderT's operations in their
-// order, so the contacts are bitwise the serial collider's. Both halves of a
-// warp run in step; `act` is false for a half without a box pair.
+// is about 500 (the list of a 200-box pile: 150 -> 39 us). Every value is
+// formed by ColliderT's operations in their order, so the contacts are bitwise
+// the serial collider's. Both halves of a warp run in step; `act` is false for
+// a half without a box pair.
 // ---------------------------------------------------------------------------
 constexpr int kGroup = 16;
 
@@ -1133,58 +1127,115 @@ __device__ __noinline__ void exact_pair(const World &w, int c) {
 //    pairs: 0.70 ms on lanes, 0.72 by threads; of a crushed pyramid with 37,825:
 //    1.24 and 0.93).
 constexpr int kGroupMax = 16384;
-__global__ void __launch_bounds__(128) exact_kernel(const __grid_constant__ World w) {
-  const int total = *((volatile int *)&w.ctl->npCount[2]);
-  if (total > kGroupMax) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x)
-      exact_pair(w, w.g.npExact[t]);
-    return;
-  }
-  __shared__ D3 poly[8][geo::kPolyCap];
-  __shared__ NewContactF held[8][kMaxContacts];
-  const int group = threadIdx.x / kGroup, gl = threadIdx.x & (kGroup - 1);
-  // warps dealt over the blocks first
-  const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (blockDim.x >> 5);
-  for (int t0 = warp * 2; t0 < total; t0 += warps * 2) {
-    const int t = t0 + (group & 1);
-    const int c = t < total ? w.g.npExact[t] : -1;
-    const uint64_t key = w.g.candKey[c >= 0 ? c : w.g.npExact[t0]];
-    const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
-    const BodyD A = load_body(w, ia), B = load_body(w, ib);
-    const bool sphere = A.sphere || B.sphere, act = c >= 0 && !sphere;
-    if (__any_sync(0xffffffffu, act)) {
-      double basis[9];
-      NewContactF nc;
-      int slot;
-      const int num = collide_group(A, B, pair_skin(w, ia, ib), act, poly[group], basis, nc, slot);
-      if (act && gl == 0) w.cur.count[c] = num;
-      if (w.p.contactModel) {  // the materials merge claims old contacts one after the other
-        if (act && slot >= 0) held[group][slot] = nc;
-        __syncwarp();
-        if (act && num && gl == 0) write_box_manifold(w, c, ia, ib, A, B, held[group], num, basis);
-        __syncwarp();
-      } else if (act && num) {
-        float bf[9];
-        for (int k = 0; k < 9; k++) bf[k] = (float)basis[k];
-        const int pi = w.g.candPrev[c];
-        const int oldNum = pi >= 0 ? w.prev.count[pi] : 0;
-        if (slot >= 0) write_box_contact(w, c, slot, pi, oldNum, A, B, nc, bf);
-        if (gl == 0) write_box_header(w, c, ia, ib, basis, bf);
-      }
+struct GroupShared {
+  D3 poly[geo::kPolyCap];
+  NewContactF held[kMaxContacts];
+};
+
+// Two pairs of one warp, a half each; c < 0: none (the first is one).
+__device__ __forceinline__ void exact_groups(const World &w, int c, GroupShared &sh) {
+  const int gl = threadIdx.x & (kGroup - 1);
+  const int first = __shfl_sync(0xffffffffu, c, 0);
+  const uint64_t key = w.g.candKey[c >= 0 ? c : first];
+  const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
+  const BodyD A = load_body(w, ia), B = load_body(w, ib);
+  const bool sphere = A.sphere || B.sphere, act = c >= 0 && !sphere;
+  if (__any_sync(0xffffffffu, act)) {
+    double basis[9];
+    NewContactF nc;
+    int slot;
+    const int num = collide_group(A, B, pair_skin(w, ia, ib), act, sh.poly, basis, nc, slot);
+    if (act && gl == 0) w.cur.count[c] = num;
+    if (w.p.contactModel) {  // the materials merge claims old contacts one after the other
+      if (act && slot >= 0) sh.held[slot] = nc;
+      __syncwarp();
+      if (act && num && gl == 0) write_box_manifold(w, c, ia, ib, A, B, sh.held, num, basis);
+      __syncwarp();
+    } else if (act && num) {
+      float bf[9];
+      for (int k = 0; k < 9; k++) bf[k] = (float)basis[k];
+      const int pi = w.g.candPrev[c];
+      const int oldNum = pi >= 0 ? w.prev.count[pi] : 0;
+      if (slot >= 0) write_box_contact(w, c, slot, pi, oldNum, A, B, nc, bf);
+      if (gl == 0) write_box_header(w, c, ia, ib, basis, bf);
     }
-    if (c >= 0 && sphere && gl == 0) exact_pair(w, c);
-    __syncwarp();
+  }
+  if (c >= 0 && sphere && gl == 0) exact_pair(w, c);
+  __syncwarp();
+}
+
+// The three lists side by side, in units of a warp: two exact pairs on lanes
+// (or 32, a thread each), 32 face pairs or 32 edge pairs, the longest chains
+// first. A short list is one pair's chain of instructions (some 55, 30 and
+// 40-80 us for the face, edge and exact lists of 200-body piles), and the
+// chains now overlap; a long one keeps every warp busy to the end (a kernel
+// per list, each with a grid for the whole device, had a last wave apiece).
+// When there are fewer units than warps they are dealt over the SMs, else a
+// free warp claims the next one (claimed, not dealt, and not before the warp
+// is free: both cost the crushed pyramid 5 %). Narrow phase, three kernels
+// and this one: the 200-body pile 119 -> 62 us, spheres among boxes 173 ->
+// 117, a 2,000-body pile 141 -> 102, a crushed 36-layer pyramid 949 -> 843,
+// a batch of 163,000 bodies 704 -> 606.
+__global__ void __launch_bounds__(128) collide_kernel(const __grid_constant__ World w) {
+  __shared__ GroupShared shared[8];
+  const int lane = threadIdx.x & 31;
+  const int nFace = w.ctl->npCount[0], nEdge = w.ctl->npCount[1], nExact = w.ctl->npCount[2];
+  const int per = nExact > kGroupMax ? 32 : 2;
+  const int uExact = (nExact + per - 1) / per, uFace = (nFace + 31) / 32, uEdge = (nEdge + 31) / 32;
+  const int units = uExact + uFace + uEdge, warps = gridDim.x * (blockDim.x >> 5);
+  const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  for (bool dealt = units < warps;; dealt = false) {
+    int u = warp;
+    if (!dealt) {
+      if (units < warps) return;
+      if (lane == 0) u = atomicAdd(&w.ctl->npNext, 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
+    }
+    if (u >= units) return;
+    if (u < uExact) {
+      if (per == 2) {
+        const int t = u * 2 + lane / kGroup;
+        exact_groups(w, t < nExact ? w.g.npExact[t] : -1, shared[threadIdx.x / kGroup]);
+      } else if (u * 32 + lane < nExact) {
+        exact_pair(w, w.g.npExact[u * 32 + lane]);
+      }
+      continue;
+    }
+    u -= uExact;
+    if (u < uFace) {
+      if (u * 32 + lane < nFace) face_pair(w, u * 32 + lane);
+      continue;
+    }
+    u -= uFace;
+    if (u * 32 + lane < nEdge) edge_pair(w, u * 32 + lane);
+  }
+}
+
+// 5. The face pairs that f32 could not decide, by the same rule (from the
+//    exact list's far end down).
+__global__ void __launch_bounds__(128) late_kernel(const __grid_constant__ World w) {
+  __shared__ GroupShared shared[8];
+  const int total = w.ctl->npCount[3], lane = threadIdx.x & 31;
+  const int *last = w.g.npExact + w.g.candCap - 1;
+  const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (blockDim.x >> 5);
+  const int per = total > kGroupMax ? 32 : 2;
+  for (int u = warp; u * per < total; u += warps) {
+    if (per == 2) {
+      const int t = u * 2 + lane / kGroup;
+      exact_groups(w, t < total ? last[-t] : -1, shared[threadIdx.x / kGroup]);
+    } else if (u * 32 + lane < total) {
+      exact_pair(w, last[-(u * 32 + lane)]);
+    }
   }
 }
 
 }  // namespace
 
 void launch_narrowphase(const World &w, cudaStream_t st, int smCount) {
-  cudaMemsetAsync(w.ctl->npCount, 0, sizeof(w.ctl->npCount), st);
+  cudaMemsetAsync(w.ctl->npCount, 0, sizeof(w.ctl->npCount) + sizeof(w.ctl->npNext), st);
   classify_kernel<<<smCount * 8, 256, 0, st>>>(w);
-  face_kernel<<<smCount * 8, 128, 0, st>>>(w);
-  edge_kernel<<<smCount * 4, 128, 0, st>>>(w);
-  exact_kernel<<<smCount * 4, 128, 0, st>>>(w);
+  collide_kernel<<<smCount * 2, 128, 0, st>>>(w);
+  late_kernel<<<smCount * 2, 128, 0, st>>>(w);
 }
 
 }  // namespace avbd
