@@ -95,9 +95,9 @@ struct Control {
   int fp64Bodies;
   int gridEntries;  // grid entries handed out this step
   unsigned colorArrivals;  // arrivals at the colouring's grid barrier this step
-  int prevCandidates;  // candidates (= manifold slots) of the previous step
   int npCount[4];      // narrow-phase work lists: face, edge, exact, late (face pairs that need the exact collider)
   int npNext;          // the next unit of the lists
+  int prevCandidates;  // candidates (= manifold slots) of the previous step
   int colorBad;        // this step's uploaded colouring has a conflict
   int laneTotal;       // lanes of one iteration's colour phases (sum over bodies)
   int pad[4];
@@ -381,6 +381,34 @@ __device__ inline Q4<T> cvtq(Q4<float> v) {
 }
 
 // Read-only-path loads (data not written during the kernel).
+// A step of a small scene is some twenty kernels of a few microseconds, and
+// as much time went by between them. A kernel launched with launch_early may
+// be set up, and its blocks become resident, while the kernel ahead of it in
+// the stream still runs; it starts with await_previous, which returns when
+// that kernel has finished and its writes are visible, and then lets the
+// kernel behind it do the same. (No __ldg of what a kernel of the chain wrote:
+// that path takes memory to be constant for as long as the kernel is there.)
+// A step of ten cubes 269 -> 240 us, of a pile of 200 376 -> 344, a static pair
+// query of 20,011 bodies 86 -> 68.
+template <class... P, class... A>
+inline void launch_early(void (*kernel)(P...), int grid, int block, cudaStream_t st, const A &...args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+__device__ __forceinline__ void next_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void await_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  next_may_launch();
+}
+
 template <class T>
 __device__ inline T ld(const T *p) {
   return __ldg(p);

@@ -125,6 +125,7 @@ __device__ __forceinline__ uint32_t bucket_of(const World &w, int4 c) {
 // the broad phase of a 163,000-body batch 0.55 -> 0.42 ms with the fewer
 // launches, of a crushed pyramid 0.54 -> 0.28.
 __global__ void cells_kernel(World w) {
+  await_previous();
   const int prevCount = w.ctl->prevCandidates;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= w.b.n; i += gridDim.x * blockDim.x) {
     if (prevCount > 0) {
@@ -156,6 +157,7 @@ __global__ void cells_kernel(World w) {
 // The first body of each bucket takes the bucket's run of entries: one atomic
 // a warp.
 __global__ void bucket_kernel(World w) {
+  await_previous();
   const int lane = threadIdx.x & 31;
   for (int i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < w.b.n; i0 += gridDim.x * blockDim.x) {
     const int i = i0 + lane;
@@ -181,6 +183,7 @@ __global__ void bucket_kernel(World w) {
 }
 
 __global__ void scatter_kernel(World w) {
+  await_previous();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < w.b.n; i += gridDim.x * blockDim.x) {
     const int4 c = w.g.cellLo[i];
     if (c.w < 0 || is_large(w, i)) continue;
@@ -224,6 +227,7 @@ __device__ int large_rejects(const World &w, int a) {
 // 2. per large body: chunk counts -> chunk offsets, plus the rejected old
 //    manifolds; the body's partner count, added to its run's total
 __global__ void __launch_bounds__(256) large_total_kernel(World w, int per) {
+  await_previous();
   const int li = blockIdx.x;
   const int a = w.g.largeList[li];
   const int extra = large_rejects(w, a);
@@ -364,6 +368,7 @@ PairRanges pair_ranges(int n, int smCount) {
 // runs count the large bodies' chunks.
 template <int kRow>
 __global__ void __launch_bounds__(256) pairs_kernel(World w, int blocks, int per) {
+  await_previous();
   if ((int)blockIdx.x >= blocks) {
     const int k = blockIdx.x - blocks;
     large_count(w, k / w.g.maxChunks, k % w.g.maxChunks);
@@ -464,6 +469,7 @@ __device__ void large_write(const World &w, int li, int ch, int per) {
 // partners, before the shared-memory form took those).
 template <int kRow>
 __global__ void __launch_bounds__(256) copy_kernel(World w, int blocks, int per) {
+  await_previous();
   if ((int)blockIdx.x >= blocks) {
     const int k = blockIdx.x - blocks;
     large_write(w, k / w.g.maxChunks, k % w.g.maxChunks, per);
@@ -543,6 +549,7 @@ __global__ void __launch_bounds__(256) copy_kernel(World w, int blocks, int per)
 //    reaches the narrow phase and every later kernel of the step returns at
 //    once (Control::skip).
 __global__ void __launch_bounds__(256) finish_kernel(World w, int numLarge) {
+  await_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     const int total = w.g.pairStart[w.b.n];
     w.ctl->wantCandidates = total;
@@ -580,13 +587,13 @@ void launch_broadphase_impl(const World &w, int numLarge, cudaStream_t st, int s
   const PairRanges R = pair_ranges(w.b.n, smCount);
   const int grid = R.blocks + numLarge * w.g.maxChunks;
   cudaMemsetAsync(w.g.table, 0, sizeof(int2) * T, st);
-  cells_kernel<<<blocks, 256, 0, st>>>(w);
-  bucket_kernel<<<blocks, 256, 0, st>>>(w);
-  scatter_kernel<<<blocks, 256, 0, st>>>(w);
-  pairs_kernel<kPairScratch><<<grid, 256, 0, st>>>(w, R.blocks, R.per);
-  if (numLarge > 0) large_total_kernel<<<numLarge, 256, 0, st>>>(w, R.per);
-  copy_kernel<kPairScratch><<<grid, 256, 0, st>>>(w, R.blocks, R.per);
-  finish_kernel<<<std::max(numLarge, 1), 256, 0, st>>>(w, numLarge);
+  launch_early(cells_kernel, blocks, 256, st, w);
+  launch_early(bucket_kernel, blocks, 256, st, w);
+  launch_early(scatter_kernel, blocks, 256, st, w);
+  launch_early(pairs_kernel<kPairScratch>, grid, 256, st, w, R.blocks, R.per);
+  if (numLarge > 0) launch_early(large_total_kernel, numLarge, 256, st, w, R.per);
+  launch_early(copy_kernel<kPairScratch>, grid, 256, st, w, R.blocks, R.per);
+  launch_early(finish_kernel, std::max(numLarge, 1), 256, st, w, numLarge);
 }
 
 }  // namespace avbd
@@ -655,6 +662,7 @@ __global__ void static_stage_kernel(World w, D4 *pos, D4 *size, D4 *massD, int *
                                     int *largeList, int *largeStart, int *sceneStart, double *invCell, float *cellF,
                                     const double *p, const double *radius, const int32_t *dynamic, double cell,
                                     double inv) {
+  await_previous();
   const int n = w.b.n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double r = radius[i];
@@ -680,6 +688,7 @@ __global__ void static_stage_kernel(World w, D4 *pos, D4 *size, D4 *massD, int *
 // The large bodies' counts and segments with the large-body count read on the
 // device and no previous manifolds.
 __global__ void static_large_count_kernel(World w, int per) {
+  await_previous();
   const int numLarge = w.g.largeStart[1];
   typedef cub::BlockReduce<int, 256> R;
   __shared__ typename R::TempStorage tmp;
@@ -697,6 +706,7 @@ __global__ void static_large_count_kernel(World w, int per) {
 }
 
 __global__ void static_large_write_kernel(World w) {
+  await_previous();
   const int numLarge = w.g.largeStart[1];
   const int cap = w.g.candCap;
   typedef cub::BlockScan<int, 256> S;
@@ -725,6 +735,7 @@ __global__ void static_large_write_kernel(World w) {
 }
 
 __global__ void static_finish_kernel(World w, int32_t *count) {
+  await_previous();
   count[0] = (w.ctl->flags & (kErrNaN | kOvfCells)) ? -1 : w.g.pairStart[w.b.n];
 }
 
@@ -843,14 +854,14 @@ extern "C" int avbd_overlap_pairs_static(int32_t n, const double *pos, const dou
                                                 (int *)(base + L.sceneStart), (double *)(base + L.invCell),
                                                 (float *)(base + L.cellF), pos, radius, dynamic, cell_size,
                                                 1.0 / cell_size);
-    cells_kernel<<<blocks, 256, 0, st>>>(w);
-    bucket_kernel<<<blocks, 256, 0, st>>>(w);
-    scatter_kernel<<<blocks, 256, 0, st>>>(w);
-    pairs_kernel<kStaticPairRow><<<R.blocks, 256, 0, st>>>(w, R.blocks, R.per);
-    static_large_count_kernel<<<smCount, 256, 0, st>>>(w, R.per);
-    copy_kernel<kStaticPairRow><<<R.blocks, 256, 0, st>>>(w, R.blocks, R.per);
-    static_large_write_kernel<<<smCount, 256, 0, st>>>(w);
-    static_finish_kernel<<<1, 1, 0, st>>>(w, count);
+    launch_early(cells_kernel, blocks, 256, st, w);
+    launch_early(bucket_kernel, blocks, 256, st, w);
+    launch_early(scatter_kernel, blocks, 256, st, w);
+    launch_early(pairs_kernel<kStaticPairRow>, R.blocks, 256, st, w, R.blocks, R.per);
+    launch_early(static_large_count_kernel, smCount, 256, st, w, R.per);
+    launch_early(copy_kernel<kStaticPairRow>, R.blocks, 256, st, w, R.blocks, R.per);
+    launch_early(static_large_write_kernel, smCount, 256, st, w);
+    launch_early(static_finish_kernel, 1, 1, st, w, count);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

@@ -604,9 +604,9 @@ void invalidate_graphs(avbd_ctx *ctx) {
 int enqueue_step(avbd_ctx *ctx) {
   World &w = ctx->w;
   cudaStream_t st = ctx->stream;
-  // per-step counters: numCandidates .. colorArrivals
+  // per-step counters: numCandidates .. npNext
   CK(cudaMemsetAsync(&w.ctl->numCandidates, 0,
-                     offsetof(Control, colorArrivals) + sizeof(unsigned) - offsetof(Control, numCandidates), st));
+                     offsetof(Control, npNext) + sizeof(int) - offsetof(Control, numCandidates), st));
   int rc;
   if ((rc = record(ctx, 0))) return rc;
   launch_broadphase_impl(w, ctx->numLarge, st, ctx->smCount);

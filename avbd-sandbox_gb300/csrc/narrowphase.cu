@@ -794,6 +794,7 @@ __device__ __forceinline__ int previous_slot(const World &w, uint64_t key, int a
 //    with a certain winning axis go to the face or edge list, everything
 //    else (sphere pairs, undecided box pairs) to the exact list.
 __global__ void __launch_bounds__(256) classify_kernel(World w) {
+  await_previous();
   const int total = *((volatile int *)&w.ctl->numCandidates);
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
     const uint64_t key = w.g.candKey[c];
@@ -1177,6 +1178,7 @@ __device__ __forceinline__ void exact_groups(const World &w, int c, GroupShared 
 // 117, a 2,000-body pile 141 -> 102, a crushed 36-layer pyramid 949 -> 843,
 // a batch of 163,000 bodies 704 -> 606.
 __global__ void __launch_bounds__(128) collide_kernel(const __grid_constant__ World w) {
+  await_previous();
   __shared__ GroupShared shared[8];
   const int lane = threadIdx.x & 31;
   const int nFace = w.ctl->npCount[0], nEdge = w.ctl->npCount[1], nExact = w.ctl->npCount[2];
@@ -1214,6 +1216,7 @@ __global__ void __launch_bounds__(128) collide_kernel(const __grid_constant__ Wo
 // 5. The face pairs that f32 could not decide, by the same rule (from the
 //    exact list's far end down).
 __global__ void __launch_bounds__(128) late_kernel(const __grid_constant__ World w) {
+  await_previous();
   __shared__ GroupShared shared[8];
   const int total = w.ctl->npCount[3], lane = threadIdx.x & 31;
   const int *last = w.g.npExact + w.g.candCap - 1;
@@ -1232,10 +1235,9 @@ __global__ void __launch_bounds__(128) late_kernel(const __grid_constant__ World
 }  // namespace
 
 void launch_narrowphase(const World &w, cudaStream_t st, int smCount) {
-  cudaMemsetAsync(w.ctl->npCount, 0, sizeof(w.ctl->npCount) + sizeof(w.ctl->npNext), st);
-  classify_kernel<<<smCount * 8, 256, 0, st>>>(w);
-  collide_kernel<<<smCount * 2, 128, 0, st>>>(w);
-  late_kernel<<<smCount * 2, 128, 0, st>>>(w);
+  launch_early(classify_kernel, smCount * 8, 256, st, w);
+  launch_early(collide_kernel, smCount * 2, 128, st, w);
+  launch_early(late_kernel, smCount * 2, 128, st, w);
 }
 
 }  // namespace avbd

@@ -99,6 +99,7 @@ __device__ inline Q4<double> body_q_t(const World &w, int i) {
 
 // joint.js:131-160 / spring.js:472-507, plus the f64 offsets p_A(t) - p_B(t).
 __global__ void prepare_forces_kernel(World w) {
+  await_previous();
   if (step_skipped(w)) return;
   const SolverParams &P = w.p;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -211,6 +212,7 @@ __global__ void prepare_forces_kernel(World w) {
 
 // solver.js:369-401, in delta form.
 __global__ void prepare_bodies_kernel(World w) {
+  await_previous();
   if (step_skipped(w)) return;
   const SolverParams &P = w.p;
   const double dt = P.dt, g = P.gravity;
@@ -261,6 +263,7 @@ __device__ inline bool precedes(const World &w, int j, int i) {
 }
 
 __global__ void adj_count_kernel(World w) {
+  await_previous();
   const int total = w.ctl->numCandidates;
   int live = 0, contacts = 0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
@@ -289,6 +292,7 @@ __global__ void adj_count_kernel(World w) {
 // Where each body's manifolds and contacts start: a block sums the runs
 // before its bodies, then scans their counts.
 __global__ void __launch_bounds__(256) adj_scan_kernel(World w) {
+  await_previous();
   typedef unsigned long long U;
   typedef cub::BlockReduce<U, 256> R;
   typedef cub::BlockScan<U, 256> S;
@@ -314,6 +318,7 @@ __global__ void __launch_bounds__(256) adj_scan_kernel(World w) {
 }
 
 __global__ void adj_fill_kernel(World w) {
+  await_previous();
   const int total = w.ctl->numCandidates;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
     if (w.cur.count[c] <= 0) continue;
@@ -339,6 +344,7 @@ __global__ void adj_fill_kernel(World w) {
 // memory each, and of some 200 for the sphere that everything waited for.
 constexpr int kSortRow = 96;  // entries sorted in shared memory; more: from a copy in the body's hpEntry range
 __global__ void __launch_bounds__(256) adj_sort_kernel(World w) {
+  await_previous();
   if (step_skipped(w)) return;
   __shared__ uint32_t row[32][kSortRow];
   const double dt2 = w.p.dt * w.p.dt;
@@ -2337,6 +2343,7 @@ constexpr int kTailMinColors = 16;  // automatic: steps of fewer colours have no
 constexpr int kChunkCache = 64;  // colours whose chunk bounds the solve keeps in shared memory
 template <bool E, bool J, bool F64>
 __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
+  next_may_launch();
   if (step_skipped(w)) return;
   extern __shared__ float4 stageSm[];
   float4 *stage = stageSm + threadIdx.x;
@@ -2495,6 +2502,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) solve_kernel(World w) {
 
 template <bool E, bool J, bool F64>
 __global__ void __launch_bounds__(kSolveBlock, 3) wave_kernel(World w, int G) {
+  next_may_launch();
   if (step_skipped(w)) return;
   extern __shared__ float4 stageSm[];
   float4 *stage = stageSm + threadIdx.x;
@@ -2535,6 +2543,7 @@ __global__ void __launch_bounds__(kSolveBlock, 3) wave_kernel(World w, int G) {
 // Also the step's bookkeeping: its candidates become the next step's previous
 // manifolds, or, for a skipped step, the skip is counted and nothing moves.
 __global__ void commit_kernel(World w) {
+  await_previous();
   if (step_skipped(w)) {
     if (blockIdx.x == 0 && threadIdx.x == 0) w.ctl->stepsSkipped++;
     return;
@@ -2598,12 +2607,12 @@ __global__ void stats_kernel(World w, double *out) {
 
 void launch_prepare(const World &w, cudaStream_t st, int smCount) {
   const int blocks = smCount * 4;
-  if (w.j.n + w.s.n > 0) prepare_forces_kernel<<<blocks, 256, 0, st>>>(w);
-  prepare_bodies_kernel<<<blocks, 256, 0, st>>>(w);
-  adj_count_kernel<<<blocks, 256, 0, st>>>(w);
-  adj_scan_kernel<<<w.b.n / 256 + 1, 256, 0, st>>>(w);
-  adj_fill_kernel<<<blocks, 256, 0, st>>>(w);
-  adj_sort_kernel<<<blocks, 256, 0, st>>>(w);
+  if (w.j.n + w.s.n > 0) launch_early(prepare_forces_kernel, blocks, 256, st, w);
+  launch_early(prepare_bodies_kernel, blocks, 256, st, w);
+  launch_early(adj_count_kernel, blocks, 256, st, w);
+  launch_early(adj_scan_kernel, w.b.n / 256 + 1, 256, st, w);
+  launch_early(adj_fill_kernel, blocks, 256, st, w);
+  launch_early(adj_sort_kernel, blocks, 256, st, w);
 }
 
 // A block per 64 bodies, so that a small scene's dozen barriers wait for few
@@ -2724,7 +2733,7 @@ cudaError_t launch_solve(const World &w, int lanesPerBody, int blocksPerSm, cuda
                                      st);
 }
 
-void launch_commit(const World &w, cudaStream_t st, int smCount) { commit_kernel<<<smCount * 4, 256, 0, st>>>(w); }
+void launch_commit(const World &w, cudaStream_t st, int smCount) { launch_early(commit_kernel, smCount * 4, 256, st, w); }
 
 void launch_stats(const World &w, double *out3, cudaStream_t st, int smCount) {
   cudaMemsetAsync(out3, 0, sizeof(double) * 3, st);
