@@ -380,7 +380,6 @@ __device__ inline Q4<T> cvtq(Q4<float> v) {
   return Q4<T>{T(v.x), T(v.y), T(v.z), T(v.w)};
 }
 
-// Read-only-path loads (data not written during the kernel).
 // A step of a small scene is some twenty kernels of a few microseconds, and
 // as much time went by between them. A kernel launched with launch_early may
 // be set up, and its blocks become resident, while the kernel ahead of it in
@@ -409,6 +408,7 @@ __device__ __forceinline__ void await_previous() {
   next_may_launch();
 }
 
+// Read-only-path loads (data not written during the kernel).
 template <class T>
 __device__ inline T ld(const T *p) {
   return __ldg(p);

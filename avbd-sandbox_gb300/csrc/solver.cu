@@ -470,6 +470,10 @@ __device__ inline void constraint_neighbors(const World &w, int i, F &&f) {
 
 // Every block of the colouring past this point; `arrivals` counts along.
 __device__ __forceinline__ bool coloring_barrier(const World &w, unsigned &arrivals) {
+  if (gridDim.x == 1) {
+    __syncthreads();
+    return true;
+  }
   arrivals += gridDim.x;
   grid_arrive(&w.ctl->colorArrivals);
   return grid_wait(w.ctl, &w.ctl->colorArrivals, arrivals, w.p.barrierLimit);
@@ -2615,12 +2619,17 @@ void launch_prepare(const World &w, cudaStream_t st, int smCount) {
   launch_early(adj_sort_kernel, blocks, 256, st, w);
 }
 
-// A block per 64 bodies, so that a small scene's dozen barriers wait for few
-// blocks (a pile of 200 bodies: four), at most two blocks an SM.
+// One block up to kColorAlone bodies, whose dozen barriers then stay in the
+// block (a pile of 60 / 120 bodies: 29 -> 21 / 45 -> 27 us). Beyond, a block
+// per 64 bodies, so that they wait for few blocks, at most two an SM. (One
+// block would be ahead up to 500 bodies, 43 us for 49, but these barriers are
+// also where the wait limit is met in steps of the wavefront schedule whose
+// bodies do not wait for one another.)
+constexpr int kColorAlone = 128;
 int coloring_grid(int n, int smCount) {
   int perSm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, coloring_kernel, 256, 0);
-  return std::max(1, std::min((n + 63) / 64, std::min(perSm, 2) * smCount));
+  return n <= kColorAlone ? 1 : std::max(1, std::min((n + 63) / 64, std::min(perSm, 2) * smCount));
 }
 
 // An uploaded colouring: copied, then checked against this step's graph.
