@@ -714,7 +714,7 @@ int one_step(avbd_ctx *ctx) {
     ctx->prof.fp64_bodies = c.fp64Bodies;
     ctx->prof.np_face = c.npCount[0];
     ctx->prof.np_edge = c.npCount[1];
-    ctx->prof.np_exact = c.npCount[2] + c.npCount[3];
+    ctx->prof.np_exact = c.npCount[2] + c.npCount[3] + c.npCount[4];
     ctx->prof.lanes_per_body = ctx->params.schedule == 1 || !ctx->autoLanes
                                    ? wave_lanes(ctx)
                                    : (c.laneTotal + std::max(ctx->nDyn, 1) / 2) / std::max(ctx->nDyn, 1);

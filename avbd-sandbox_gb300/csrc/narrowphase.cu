@@ -791,8 +791,9 @@ __device__ __forceinline__ int previous_slot(const World &w, uint64_t key, int a
 }
 
 // 1. Every candidate: its previous manifold, and the f32 SAT. Separated pairs get count 0; box pairs
-//    with a certain winning axis go to the face or edge list, everything
-//    else (sphere pairs, undecided box pairs) to the exact list.
+//    with a certain winning axis go to the face or edge list, undecided ones
+//    to the exact list, sphere pairs to a list that fills the edge list's
+//    array from its far end (a candidate is in one list only).
 __global__ void __launch_bounds__(256) classify_kernel(World w) {
   await_previous();
   const int total = *((volatile int *)&w.ctl->numCandidates);
@@ -802,9 +803,13 @@ __global__ void __launch_bounds__(256) classify_kernel(World w) {
     w.g.candPrev[c] = previous_slot(w, key, ia);
     w.cur.key[c] = key;
     const BodyD A = load_body(w, ia), B = load_body(w, ib);
-    // spheres, and pairs with a contact skin (speculative contacts: the f32
-    // certification covers the skin-free tests), go to the exact collider
-    if (A.sphere || B.sphere || pair_skin(w, ia, ib) != 0.0) {
+    if (A.sphere || B.sphere) {
+      w.g.npEdge[w.g.candCap - 1 - push_slot(&w.ctl->npCount[4])].x = c;
+      continue;
+    }
+    // pairs with a contact skin (speculative contacts: the f32 certification
+    // covers the skin-free tests) go to the exact collider
+    if (pair_skin(w, ia, ib) != 0.0) {
       push_exact(w, c);
       continue;
     }
@@ -1121,8 +1126,10 @@ __device__ __noinline__ void exact_pair(const World &w, int c) {
   write_box_manifold(w, c, ia, ib, A, B, ncf, num, basis);
 }
 
-// 4. Sphere pairs and undecided box pairs: the whole f64 collider. Lists of up
-//    to kGroupMax pairs: box pairs on sixteen lanes each. Longer ones keep every
+// 4. Sphere pairs and undecided box pairs: the whole f64 collider. Sphere pairs
+//    a thread each (a short chain: in halves of warps of their own, as the box
+//    pairs, they made it 113 us for 88 in a pile of 1,777 boxes and spheres). Lists of up to
+//    kGroupMax box pairs on sixteen lanes a pair; longer ones keep every
 //    sub-partition's FP64 pipe busy either way, and a pair a thread then needs
 //    about half the warp instructions (narrow phase of a batch with 10,257 such
 //    pairs: 0.70 ms on lanes, 0.72 by threads; of a crushed pyramid with 37,825:
@@ -1140,33 +1147,30 @@ __device__ __forceinline__ void exact_groups(const World &w, int c, GroupShared 
   const uint64_t key = w.g.candKey[c >= 0 ? c : first];
   const int ia = (int)(key >> 32), ib = (int)(key & 0xffffffffu);
   const BodyD A = load_body(w, ia), B = load_body(w, ib);
-  const bool sphere = A.sphere || B.sphere, act = c >= 0 && !sphere;
-  if (__any_sync(0xffffffffu, act)) {
-    double basis[9];
-    NewContactF nc;
-    int slot;
-    const int num = collide_group(A, B, pair_skin(w, ia, ib), act, sh.poly, basis, nc, slot);
-    if (act && gl == 0) w.cur.count[c] = num;
-    if (w.p.contactModel) {  // the materials merge claims old contacts one after the other
-      if (act && slot >= 0) sh.held[slot] = nc;
-      __syncwarp();
-      if (act && num && gl == 0) write_box_manifold(w, c, ia, ib, A, B, sh.held, num, basis);
-      __syncwarp();
-    } else if (act && num) {
-      float bf[9];
-      for (int k = 0; k < 9; k++) bf[k] = (float)basis[k];
-      const int pi = w.g.candPrev[c];
-      const int oldNum = pi >= 0 ? w.prev.count[pi] : 0;
-      if (slot >= 0) write_box_contact(w, c, slot, pi, oldNum, A, B, nc, bf);
-      if (gl == 0) write_box_header(w, c, ia, ib, basis, bf);
-    }
+  const bool act = c >= 0;
+  double basis[9];
+  NewContactF nc;
+  int slot;
+  const int num = collide_group(A, B, pair_skin(w, ia, ib), act, sh.poly, basis, nc, slot);
+  if (act && gl == 0) w.cur.count[c] = num;
+  if (w.p.contactModel) {  // the materials merge claims old contacts one after the other
+    if (act && slot >= 0) sh.held[slot] = nc;
+    __syncwarp();
+    if (act && num && gl == 0) write_box_manifold(w, c, ia, ib, A, B, sh.held, num, basis);
+    __syncwarp();
+  } else if (act && num) {
+    float bf[9];
+    for (int k = 0; k < 9; k++) bf[k] = (float)basis[k];
+    const int pi = w.g.candPrev[c];
+    const int oldNum = pi >= 0 ? w.prev.count[pi] : 0;
+    if (slot >= 0) write_box_contact(w, c, slot, pi, oldNum, A, B, nc, bf);
+    if (gl == 0) write_box_header(w, c, ia, ib, basis, bf);
   }
-  if (c >= 0 && sphere && gl == 0) exact_pair(w, c);
   __syncwarp();
 }
 
 // The three lists side by side, in units of a warp: two exact pairs on lanes
-// (or 32, a thread each), 32 face pairs or 32 edge pairs, the longest chains
+// (or 32, a thread each), or 32 face, sphere or edge pairs, the longest chains
 // first. A short list is one pair's chain of instructions (some 55, 30 and
 // 40-80 us for the face, edge and exact lists of 200-body piles), and the
 // chains now overlap; a long one keeps every warp busy to the end (a kernel
@@ -1182,9 +1186,10 @@ __global__ void __launch_bounds__(128) collide_kernel(const __grid_constant__ Wo
   __shared__ GroupShared shared[8];
   const int lane = threadIdx.x & 31;
   const int nFace = w.ctl->npCount[0], nEdge = w.ctl->npCount[1], nExact = w.ctl->npCount[2];
+  const int nSphere = w.ctl->npCount[4];
   const int per = nExact > kGroupMax ? 32 : 2;
   const int uExact = (nExact + per - 1) / per, uFace = (nFace + 31) / 32, uEdge = (nEdge + 31) / 32;
-  const int units = uExact + uFace + uEdge, warps = gridDim.x * (blockDim.x >> 5);
+  const int uSphere = (nSphere + 31) / 32, units = uExact + uFace + uSphere + uEdge, warps = gridDim.x * (blockDim.x >> 5);
   const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   for (bool dealt = units < warps;; dealt = false) {
     int u = warp;
@@ -1209,6 +1214,11 @@ __global__ void __launch_bounds__(128) collide_kernel(const __grid_constant__ Wo
       continue;
     }
     u -= uFace;
+    if (u < uSphere) {
+      if (u * 32 + lane < nSphere) exact_pair(w, w.g.npEdge[w.g.candCap - 1 - (u * 32 + lane)].x);
+      continue;
+    }
+    u -= uSphere;
     if (u * 32 + lane < nEdge) edge_pair(w, u * 32 + lane);
   }
 }
