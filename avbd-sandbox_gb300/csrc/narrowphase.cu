@@ -606,127 +606,164 @@ __device__ void write_sphere_manifold(const World &w, int c, int ia, int ib, con
 // the normal is measured to the rest distance; a new or re-armed impact
 // (the old contact still outside rest and without a bias) faster than the
 // restitution threshold gets a one-frame bias.
+struct MaterialsPair {
+  int pi, oldNum;  // the previous manifold and its contacts
+  double ob[9];    // its basis
+  double mus, mud, restitution, contactDistance, restDistance, persistence, psq;
+  bool compatible, curved;
+};
+
+__device__ MaterialsPair materials_pair(const World &w, int c, int ia, int ib, const BodyD &A, const BodyD &B,
+                                        const double *basis) {
+  MaterialsPair m;
+  m.pi = w.g.candPrev[c];
+  m.oldNum = m.pi >= 0 ? w.prev.count[m.pi] : 0;
+  for (int k = 0; k < 9; k++) m.ob[k] = m.oldNum > 0 ? w.prev.basisD[m.pi * 9 + k] : basis[k];
+  const D4 ma = w.b.mat[ia], mb = w.b.mat[ib];
+  m.mus = sqrt(ma.x * mb.x);
+  m.mud = sqrt(ma.y * mb.y);
+  m.restitution = ma.z > mb.z ? ma.z : (mb.z > ma.z ? mb.z : ma.z);
+  m.contactDistance = w.b.contactOffset[ia] + w.b.contactOffset[ib];
+  m.restDistance = ma.w + mb.w;
+  m.compatible = m.oldNum > 0 && (m.ob[0] * basis[0] + m.ob[1] * basis[1] + m.ob[2] * basis[2]) > 0.85;
+  const double minA = fmin(A.half.x, fmin(A.half.y, A.half.z)), minB = fmin(B.half.x, fmin(B.half.y, B.half.z));
+  const double minExtent = 2.0 * fmin(minA, minB);
+  m.persistence = fmax(w.p.contactPersistence, fmax(m.contactDistance, minExtent * 0.02));
+  m.psq = m.persistence * m.persistence;
+  m.curved = A.sphere || B.sphere;
+  return m;
+}
+
+__device__ __forceinline__ D3 midpoint(D3 a, D3 b) {
+  return mk((a.x + b.x) * 0.5, (a.y + b.y) * 0.5, (a.z + b.z) * 0.5);
+}
+__device__ __forceinline__ double dist_sq(D3 a, D3 b) {
+  const D3 d = mk(a.x - b.x, a.y - b.y, a.z - b.z);
+  return d.x * d.x + d.y * d.y + d.z * d.z;
+}
+
+// Old contact os at the new poses: its midpoint, and whether its separation
+// and tangential offset along the new normal keep it a candidate.
+__device__ __forceinline__ bool old_contact(const World &w, const MaterialsPair &m, int os, const BodyD &A,
+                                            const BodyD &B, D3 nN, D3 &mid) {
+  const float4 oa = w.prev.rA[os], obb = w.prev.rB[os];
+  const D3 oxA = add(rot(A.q, mk(oa.x, oa.y, oa.z)), A.p);
+  const D3 oxB = add(rot(B.q, mk(obb.x, obb.y, obb.z)), B.p);
+  const D3 od = sub(oxA, oxB);
+  const double sep = nN.x * od.x + nN.y * od.y + nN.z * od.z;
+  const D3 td = mk(od.x - nN.x * sep, od.y - nN.y * sep, od.z - nN.z * sep);
+  mid = midpoint(oxA, oxB);
+  return !(sep > m.contactDistance + m.persistence) && !(td.x * td.x + td.y * td.y + td.z * td.z > m.psq);
+}
+
+// New contact i, matched with old contact `match` (-1: none).
+__device__ void write_materials_contact(const World &w, int c, int i, int ia, int ib, const BodyD &A, const BodyD &B,
+                                        const MaterialsPair &m, const double *basis, D3 rA, D3 rB, uint32_t feature,
+                                        int match) {
+  const SolverParams &P = w.p;
+  const double *ob = m.ob;
+  const bool found = match >= 0;
+  double lam[3] = {0, 0, 0}, pen[3] = {0, 0, 0};
+  bool stick = true, priorOut = false, priorBias = false;
+  if (found) {
+    const int os = m.pi * kMaxContacts + match;
+    const float4 ok = w.prev.cK[os], ol = w.prev.cL[os];
+    for (int r = 0; r < 3; r++) {  // transport into the new basis (shaders.js:1050-1085)
+      const double *nr = &basis[r * 3];
+      const double a = nr[0] * ob[0] + nr[1] * ob[1] + nr[2] * ob[2];
+      const double b = nr[0] * ob[3] + nr[1] * ob[4] + nr[2] * ob[5];
+      const double cc = nr[0] * ob[6] + nr[1] * ob[7] + nr[2] * ob[8];
+      pen[r] = (double)ok.x * (a * a) + (double)ok.y * (b * b) + (double)ok.z * (cc * cc);
+      lam[r] = (double)ol.x * a + (double)ol.y * b + (double)ol.z * cc;
+    }
+    stick = ol.w != 0.0f;
+    priorOut = w.prev.cA[os].w > 0.0f;
+    priorBias = w.prev.cX[os] > 0.0f;
+    if (stick && !m.curved) {
+      const float4 oa = w.prev.rA[os], obb = w.prev.rB[os];
+      rA = mk(oa.x, oa.y, oa.z);
+      rB = mk(obb.x, obb.y, obb.z);
+    }
+  }
+  const D3 nN = mk(basis[0], basis[1], basis[2]);
+  const D3 rAw = rot(A.q, rA), rBw = rot(B.q, rB);
+  const D3 d = sub(add(rAw, A.p), add(rBw, B.p));
+  double C0[3];
+  C0[0] = basis[0] * d.x + basis[1] * d.y + basis[2] * d.z - m.restDistance;
+  C0[1] = basis[3] * d.x + basis[4] * d.y + basis[5] * d.z;
+  C0[2] = basis[6] * d.x + basis[7] * d.y + basis[8] * d.z;
+  double bias = 0.0;
+  if ((!found || (priorOut && !priorBias)) && m.restitution > 0.0) {
+    const float4 vA = w.b.vel[ia], wA = w.b.omega[ia], vB = w.b.vel[ib], wB = w.b.omega[ib];
+    const D3 ua = add(mk(vA.x, vA.y, vA.z), crs(mk(wA.x, wA.y, wA.z), rAw));
+    const D3 ub = add(mk(vB.x, vB.y, vB.z), crs(mk(wB.x, wB.y, wB.z), rBw));
+    const D3 rel = sub(ua, ub);
+    const double vn = nN.x * rel.x + nN.y * rel.y + nN.z * rel.z;
+    const double closing = fmax(0.0, -vn * P.dt), toRest = fmax(0.0, C0[0]);
+    if (vn < -P.restitutionThreshold && closing > toRest) bias = m.restitution * (closing - toRest);
+  }
+  if (!P.postStabilize)
+    for (int k = 0; k < 3; k++) lam[k] = lam[k] * P.alpha * P.gamma;
+  for (int k = 0; k < 3; k++) pen[k] = clampd(pen[k] * P.gamma, P.penaltyMin, P.penaltyMax);
+  const int s = c * kMaxContacts + i;
+  w.cur.feat[s] = feature;
+  w.cur.rA[s] = make_float4((float)rA.x, (float)rA.y, (float)rA.z, 0.f);
+  w.cur.rB[s] = make_float4((float)rB.x, (float)rB.y, (float)rB.z, 0.f);
+  w.cur.cA[s] = make_float4((float)rAw.x, (float)rAw.y, (float)rAw.z, (float)C0[0]);
+  w.cur.cB[s] = make_float4((float)rBw.x, (float)rBw.y, (float)rBw.z, (float)C0[1]);
+  w.cur.cK[s] = make_float4((float)pen[0], (float)pen[1], (float)pen[2], (float)C0[2]);
+  w.cur.cL[s] = make_float4((float)lam[0], (float)lam[1], (float)lam[2], stick ? 1.f : 0.f);
+  w.cur.cX[s] = (float)bias;
+}
+
+__device__ __forceinline__ void write_materials_header(const World &w, int c, const MaterialsPair &m,
+                                                       const double *basis) {
+  for (int k = 0; k < 9; k++) w.cur.basisD[c * 9 + k] = basis[k];
+  const float flags = (m.curved ? 1.f : 0.f) + (m.contactDistance > 0.0 ? 2.f : 0.f);
+  w.cur.basis0[c] = make_float4((float)basis[0], (float)basis[1], (float)basis[2], (float)m.mus);
+  w.cur.basis1[c] = make_float4((float)basis[3], (float)basis[4], (float)basis[5], flags);
+  w.cur.basis2[c] = make_float4((float)basis[6], (float)basis[7], (float)basis[8], (float)m.mud);
+}
+
 __device__ void write_manifold_materials(const World &w, int c, int ia, int ib, const BodyD &A, const BodyD &B,
                                          const D3 *ncA, const D3 *ncB, const uint32_t *feat, int num,
                                          const double *basis) {
-  const SolverParams &P = w.p;
   w.cur.count[c] = num;
   if (num == 0) return;
-  const int pi = w.g.candPrev[c];
-  const int oldNum = pi >= 0 ? w.prev.count[pi] : 0;
-  double ob[9];
-  for (int k = 0; k < 9; k++) ob[k] = oldNum > 0 ? w.prev.basisD[pi * 9 + k] : basis[k];
-  const D4 ma = w.b.mat[ia], mb = w.b.mat[ib];
-  const double mus = sqrt(ma.x * mb.x), mud = sqrt(ma.y * mb.y);
-  const double restitution = ma.z > mb.z ? ma.z : (mb.z > ma.z ? mb.z : ma.z);
-  const double contactDistance = w.b.contactOffset[ia] + w.b.contactOffset[ib];
-  const double restDistance = ma.w + mb.w;
+  const MaterialsPair m = materials_pair(w, c, ia, ib, A, B, basis);
   const D3 nN = mk(basis[0], basis[1], basis[2]);
-  const bool compatible = oldNum > 0 && (ob[0] * basis[0] + ob[1] * basis[1] + ob[2] * basis[2]) > 0.85;
-  const double minA = fmin(A.half.x, fmin(A.half.y, A.half.z)), minB = fmin(B.half.x, fmin(B.half.y, B.half.z));
-  const double minExtent = 2.0 * fmin(minA, minB);
-  const double persistence = fmax(P.contactPersistence, fmax(contactDistance, minExtent * 0.02));
-  const double psq = persistence * persistence;
-  const bool curved = A.sphere || B.sphere;
-  const float4 vA4 = w.b.vel[ia], wA4 = w.b.omega[ia], vB4 = w.b.vel[ib], wB4 = w.b.omega[ib];
-  const D3 vA = mk(vA4.x, vA4.y, vA4.z), wA = mk(wA4.x, wA4.y, wA4.z);
-  const D3 vB = mk(vB4.x, vB4.y, vB4.z), wB = mk(wB4.x, wB4.y, wB4.z);
   unsigned used = 0u;
   for (int i = 0; i < num; i++) {
-    D3 rA = ncA[i], rB = ncB[i];
-    double lam[3] = {0, 0, 0}, pen[3] = {0, 0, 0};
-    bool stick = true, priorOut = false, priorBias = false, found = false, exact = false;
     int match = -1;
-    double best = psq;
-    const D3 nxA = add(rot(A.q, rA), A.p), nxB = add(rot(B.q, rB), B.p);
-    const D3 mid = mk((nxA.x + nxB.x) * 0.5, (nxA.y + nxB.y) * 0.5, (nxA.z + nxB.z) * 0.5);
-    if (compatible) {
-      for (int j = 0; j < oldNum; j++) {
+    double best = m.psq;
+    if (m.compatible) {
+      const D3 mid = midpoint(add(rot(A.q, ncA[i]), A.p), add(rot(B.q, ncB[i]), B.p));
+      for (int j = 0; j < m.oldNum; j++) {
         if (used & (1u << j)) continue;
-        const int os = pi * kMaxContacts + j;
+        const int os = m.pi * kMaxContacts + j;
         const bool same = w.prev.feat[os] == feat[i];
-        if (curved && same) {
+        if (m.curved && same) {
           match = j;
-          exact = true;
           break;
         }
-        const float4 oa = w.prev.rA[os], obb = w.prev.rB[os];
-        const D3 oxA = add(rot(A.q, mk(oa.x, oa.y, oa.z)), A.p);
-        const D3 oxB = add(rot(B.q, mk(obb.x, obb.y, obb.z)), B.p);
-        const D3 od = sub(oxA, oxB);
-        const double sep = nN.x * od.x + nN.y * od.y + nN.z * od.z;
-        const D3 td = mk(od.x - nN.x * sep, od.y - nN.y * sep, od.z - nN.z * sep);
-        if (sep > contactDistance + persistence) continue;
-        if (td.x * td.x + td.y * td.y + td.z * td.z > psq) continue;
-        const D3 md = mk(mid.x - (oxA.x + oxB.x) * 0.5, mid.y - (oxA.y + oxB.y) * 0.5, mid.z - (oxA.z + oxB.z) * 0.5);
-        const double mdSq = md.x * md.x + md.y * md.y + md.z * md.z;
-        if (mdSq > psq) continue;
+        D3 oldMid;
+        if (!old_contact(w, m, os, A, B, nN, oldMid)) continue;
+        const double mdSq = dist_sq(mid, oldMid);
+        if (mdSq > m.psq) continue;
         if (same) {
           match = j;
-          exact = true;
           break;
         }
-        if (!found || mdSq < best) {
-          found = true;
+        if (match < 0 || mdSq < best) {
           match = j;
           best = mdSq;
         }
       }
     }
-    found = found || exact;
-    if (found) {
-      const int os = pi * kMaxContacts + match;
-      used |= 1u << match;
-      const float4 ok = w.prev.cK[os], ol = w.prev.cL[os];
-      for (int r = 0; r < 3; r++) {  // transport into the new basis (shaders.js:1050-1085)
-        const double *nr = &basis[r * 3];
-        const double a = nr[0] * ob[0] + nr[1] * ob[1] + nr[2] * ob[2];
-        const double b = nr[0] * ob[3] + nr[1] * ob[4] + nr[2] * ob[5];
-        const double cc = nr[0] * ob[6] + nr[1] * ob[7] + nr[2] * ob[8];
-        pen[r] = (double)ok.x * (a * a) + (double)ok.y * (b * b) + (double)ok.z * (cc * cc);
-        lam[r] = (double)ol.x * a + (double)ol.y * b + (double)ol.z * cc;
-      }
-      stick = ol.w != 0.0f;
-      priorOut = w.prev.cA[os].w > 0.0f;
-      priorBias = w.prev.cX[os] > 0.0f;
-      if (stick && !A.sphere && !B.sphere) {
-        const float4 oa = w.prev.rA[os], obb = w.prev.rB[os];
-        rA = mk(oa.x, oa.y, oa.z);
-        rB = mk(obb.x, obb.y, obb.z);
-      }
-    }
-    const D3 rAw = rot(A.q, rA), rBw = rot(B.q, rB);
-    const D3 d = sub(add(rAw, A.p), add(rBw, B.p));
-    double C0[3];
-    C0[0] = basis[0] * d.x + basis[1] * d.y + basis[2] * d.z - restDistance;
-    C0[1] = basis[3] * d.x + basis[4] * d.y + basis[5] * d.z;
-    C0[2] = basis[6] * d.x + basis[7] * d.y + basis[8] * d.z;
-    double bias = 0.0;
-    if ((!found || (priorOut && !priorBias)) && restitution > 0.0) {
-      const D3 ua = add(vA, crs(wA, rAw)), ub = add(vB, crs(wB, rBw));
-      const D3 rel = sub(ua, ub);
-      const double vn = nN.x * rel.x + nN.y * rel.y + nN.z * rel.z;
-      const double closing = fmax(0.0, -vn * P.dt), toRest = fmax(0.0, C0[0]);
-      if (vn < -P.restitutionThreshold && closing > toRest) bias = restitution * (closing - toRest);
-    }
-    if (!P.postStabilize)
-      for (int k = 0; k < 3; k++) lam[k] = lam[k] * P.alpha * P.gamma;
-    for (int k = 0; k < 3; k++) pen[k] = clampd(pen[k] * P.gamma, P.penaltyMin, P.penaltyMax);
-    const int s = c * kMaxContacts + i;
-    w.cur.feat[s] = feat[i];
-    w.cur.rA[s] = make_float4((float)rA.x, (float)rA.y, (float)rA.z, 0.f);
-    w.cur.rB[s] = make_float4((float)rB.x, (float)rB.y, (float)rB.z, 0.f);
-    w.cur.cA[s] = make_float4((float)rAw.x, (float)rAw.y, (float)rAw.z, (float)C0[0]);
-    w.cur.cB[s] = make_float4((float)rBw.x, (float)rBw.y, (float)rBw.z, (float)C0[1]);
-    w.cur.cK[s] = make_float4((float)pen[0], (float)pen[1], (float)pen[2], (float)C0[2]);
-    w.cur.cL[s] = make_float4((float)lam[0], (float)lam[1], (float)lam[2], stick ? 1.f : 0.f);
-    w.cur.cX[s] = (float)bias;
+    if (match >= 0) used |= 1u << match;
+    write_materials_contact(w, c, i, ia, ib, A, B, m, basis, ncA[i], ncB[i], feat[i], match);
   }
-  for (int k = 0; k < 9; k++) w.cur.basisD[c * 9 + k] = basis[k];
-  const float flags = (curved ? 1.f : 0.f) + (contactDistance > 0.0 ? 2.f : 0.f);
-  w.cur.basis0[c] = make_float4((float)basis[0], (float)basis[1], (float)basis[2], (float)mus);
-  w.cur.basis1[c] = make_float4((float)basis[3], (float)basis[4], (float)basis[5], flags);
-  w.cur.basis2[c] = make_float4((float)basis[6], (float)basis[7], (float)basis[8], (float)mud);
+  write_materials_header(w, c, m, basis);
 }
 
 // Append to one of the work lists, one atomic per coalesced group of lanes.
@@ -1102,6 +1139,52 @@ __device__ int collide_group(const BodyD &A, const BodyD &B, double cd, bool act
   return live ? count : 0;
 }
 
+// write_manifold_materials of a box pair on the sixteen lanes: an old contact
+// and a new one a lane, the claims one new contact after the other (a lane for
+// the pair took 162 us of the narrow phase of 1,000 such boxes, this
+// 100). `slot` is the lane's new contact, nc, or -1.
+__device__ void write_materials_group(const World &w, int c, int ia, int ib, const BodyD &A, const BodyD &B, bool act,
+                                      const NewContactF &nc, int slot, int num, const double *basis) {
+  const int gl = threadIdx.x & (kGroup - 1);
+  const unsigned shift = threadIdx.x & (32 - kGroup);
+  auto ballot = [&](bool p) { return (__ballot_sync(0xffffffffu, p) >> shift) & 0xffffu; };
+  const bool own = act && slot >= 0;
+  const MaterialsPair m = materials_pair(w, act ? c : 0, ia, ib, A, B, basis);
+  const D3 rA = own ? mk(nc.ra[0], nc.ra[1], nc.ra[2]) : mk(0, 0, 0);
+  const D3 rB = own ? mk(nc.rb[0], nc.rb[1], nc.rb[2]) : mk(0, 0, 0);
+  const bool merge = act && num > 0 && m.compatible;
+  int match = -1;
+  if (__any_sync(0xffffffffu, merge)) {
+    const D3 mid = midpoint(add(rot(A.q, rA), A.p), add(rot(B.q, rB), B.p));
+    const bool old = merge && gl < m.oldNum;
+    D3 oldMid = mk(0, 0, 0);
+    bool pass = false;
+    uint32_t oldFeat = 0u;
+    if (old) {
+      const int os = m.pi * kMaxContacts + gl;
+      oldFeat = w.prev.feat[os];
+      pass = old_contact(w, m, os, A, B, mk(basis[0], basis[1], basis[2]), oldMid);
+    }
+    unsigned used = 0u;
+#pragma unroll 1
+    for (int i = 0; __any_sync(0xffffffffu, merge && i < num); i++) {
+      const unsigned at = ballot(own && slot == i);
+      const int src = at ? __ffs(at) - 1 : 0;
+      const double mdSq = dist_sq(gshfl(mid, src), oldMid);
+      const uint32_t feat = __shfl_sync(0xffffffffu, own ? nc.feature : 0u, src, kGroup);
+      const bool ok = pass && i < num && !((used >> gl) & 1u) && !(mdSq > m.psq);
+      const unsigned okMask = ballot(ok), sameMask = ballot(ok && oldFeat == feat), nanMask = ballot(ok && mdSq != mdSq);
+      const int nearest = group_argmax(-mdSq, ok), first = __ffs(okMask) - 1;
+      int j = sameMask ? __ffs(sameMask) - 1 : nearest;
+      if (!sameMask && okMask && ((nanMask >> first) & 1u)) j = first;  // (nothing is less than NaN)
+      if (j >= 0) used |= 1u << j;
+      if (own && slot == i) match = j;
+    }
+  }
+  if (own) write_materials_contact(w, c, slot, ia, ib, A, B, m, basis, rA, rB, nc.feature, match);
+  if (act && num > 0 && gl == 0) write_materials_header(w, c, m, basis);
+}
+
 // A lane's pair decided by the serial collider: every sphere pair, and box
 // pairs of long lists.
 __device__ __noinline__ void exact_pair(const World &w, int c) {
@@ -1137,7 +1220,6 @@ __device__ __noinline__ void exact_pair(const World &w, int c) {
 constexpr int kGroupMax = 16384;
 struct GroupShared {
   D3 poly[geo::kPolyCap];
-  NewContactF held[kMaxContacts];
 };
 
 // Two pairs of one warp, a half each; c < 0: none (the first is one).
@@ -1153,11 +1235,8 @@ __device__ __forceinline__ void exact_groups(const World &w, int c, GroupShared 
   int slot;
   const int num = collide_group(A, B, pair_skin(w, ia, ib), act, sh.poly, basis, nc, slot);
   if (act && gl == 0) w.cur.count[c] = num;
-  if (w.p.contactModel) {  // the materials merge claims old contacts one after the other
-    if (act && slot >= 0) sh.held[slot] = nc;
-    __syncwarp();
-    if (act && num && gl == 0) write_box_manifold(w, c, ia, ib, A, B, sh.held, num, basis);
-    __syncwarp();
+  if (w.p.contactModel) {
+    if (__any_sync(0xffffffffu, num > 0)) write_materials_group(w, c, ia, ib, A, B, act, nc, slot, num, basis);
   } else if (act && num) {
     float bf[9];
     for (int k = 0; k < 9; k++) bf[k] = (float)basis[k];

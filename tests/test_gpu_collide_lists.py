@@ -72,3 +72,35 @@ def test_contacts_do_not_depend_on_the_lists(abi, scenes, backend_mod, bodies, c
     for f in ("num_contacts", "basis", "friction", "feature", "r_a", "r_b", "c0", "restitution_bias"):
         a, b = getattr(one, "m_" + f)[:m], getattr(many, "m_" + f)[:copies * m].reshape((copies, m) + getattr(one, "m_" + f).shape[1:])
         assert np.all(b == a[None]), f
+
+
+@pytest.mark.parametrize("bodies", [12, 40, 120])
+def test_materials_merge_on_lanes_and_by_threads(abi, scenes, backend_mod, bodies):
+    """Under the materials model a box pair's contacts claim the previous
+    step's on sixteen lanes, in lists of more than 16,384 pairs by a thread:
+    the same claims, so the same bits over several steps."""
+    outs = []
+    for filler in (0, 16400):
+        s = cluster(scenes, abi, bodies, True, seed=3)
+        s.params.update(gravity=-9.81, iterations=4)
+        for k in range(filler):
+            at = np.array([40.0 + 4.0 * (k % 128), 4.0 * (k // 128), 0.0])
+            s.box((1.0, 1.0, 1.0), 100.0, 0.5, at)
+            s.box((1.0, 1.0, 1.0), 100.0, 0.5, at + (0.0, 0.0, 0.99))
+        w = s.world()
+        w.set_materials(static_friction=0.7, dynamic_friction=0.5, restitution=0.2, contact_offset=0.02)
+        gpu = backend_mod.GpuBackend(abi.default_params(**s.params, body_order=abi.ORDER_PRIORITY))
+        gpu.pack(w)
+        gpu.set_profiling(True)
+        gpu.step(6)
+        gpu.idle()
+        assert (gpu.last_profile["np_exact"] > 16384) == (filler > 0)
+        outs.append(gpu.read_state(manifolds=True))
+        gpu.destroy()
+    short, long_ = outs
+    m = short.m_count
+    assert m > 0 and np.all(long_.m_body_a[:m] < bodies)
+    for f in ("body_a", "body_b", "num_contacts", "basis", "feature", "r_a", "r_b", "c0", "penalty", "lambda", "stick",
+              "restitution_bias"):
+        assert np.array_equal(getattr(short, "m_" + f)[:m], getattr(long_, "m_" + f)[:m]), f
+    assert np.array_equal(short.pos, long_.pos[:bodies]) and np.array_equal(short.quat, long_.quat[:bodies])
