@@ -29,6 +29,7 @@ constexpr int kMaxContacts = 8;
 // over the colours in use only.
 constexpr int kMaxColors = 1024;
 constexpr int kAdjRun = 128;        // bodies of a run of Adjacency::runCount
+constexpr int kAdjAlone = 1024;     // scenes of fewer bodies build the adjacency in one block
 constexpr int kLaneBuckets = 8;     // log2 of the lanes of a body's group: 0..7
 constexpr int kLaneMaxGroup = 128;  // largest group: one solve block
 

@@ -630,7 +630,9 @@ int enqueue_step(avbd_ctx *ctx) {
 // 4, prepare 5 (+1 with joints or springs), colouring 1 (+2 with an
 // uploaded colouring), solve 1, commit 1.
 int step_kernels(const avbd_ctx *ctx) {
-  return 6 + (ctx->numLarge > 0 ? 1 : 0) + 4 + 5 + (ctx->nj + ctx->ns > 0 ? 1 : 0) + 1 + (ctx->w.a.colorOverride ? 2 : 0) + 1 + 1;
+  const int broad = 6 + (ctx->numLarge > 0 ? 1 : 0);
+  const int prepare = (ctx->n < kAdjAlone ? 3 : 5) + (ctx->nj + ctx->ns > 0 ? 1 : 0);
+  return broad + 3 + prepare + 1 + (ctx->w.a.colorOverride ? 2 : 0) + 1 + 1;
 }
 
 // One step as a CUDA graph (captured on first use for this arena parity).
