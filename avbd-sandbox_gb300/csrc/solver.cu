@@ -2758,11 +2758,10 @@ cudaError_t launch_joint_anchor(const World &w, int joint, double x, double y, d
 // The solve's instantiations: the contact extensions
 // (AVBD_CONTACT_MATERIALS), joints and springs, and the FP64 bodies each in
 // kernels of their own, so that the others carry none of their registers. The
-// joints' calls cost 130 bytes of spills, the FP64 path's calls
-// cost the kernel a 1.4 KB stack frame and 260 bytes of spills, which every
-// grid barrier's acquire throws out of L1; without it there are none (148 registers;
-// solve of piles of 200 / 8,192 bodies 0.30 -> 0.27 / 0.60 -> 0.55 ms, the
-// crushed 36-layer pyramid 4.96 -> 4.58).
+// joints' calls cost some 180 bytes of spills, the FP64 path's a 1.5 KB stack
+// frame and 800, which every grid barrier's acquire throws out of L1; without
+// them there are none (168 registers; solve of piles of 200 / 8,192 bodies 0.30
+// -> 0.27 / 0.60 -> 0.55 ms, the crushed 36-layer pyramid 4.96 -> 4.58).
 template <bool E, bool J, bool F64>
 static const void *solve_instance(bool wave) {
   return wave ? (const void *)wave_kernel<E, J, F64> : (const void *)solve_kernel<E, J, F64>;
