@@ -473,6 +473,7 @@ int write_state(avbd_ctx *ctx, const avbd_world *world, bool keepManifolds) {
     auto put = [&](size_t at, const double *a, size_t k) {
       if (a) std::memcpy(h.d64 + at, a, k * sizeof(double));
     };
+    if (n > 0 && !B.pos) return fail(ctx, AVBD_ERR_CUDA, "no positions");  // (as the copy from null)
     put(0, B.pos, 3 * N);
     put(3 * N, B.quat, 4 * N);
     put(7 * N, B.vel, 3 * N);

@@ -4,6 +4,7 @@ state, above it arrays are copied one by one. What was written comes back as
 the device holds it (positions in f64, the rest of a body in f32), joints and
 springs included, and a position that is not finite changes nothing at all.
 """
+import ctypes
 import importlib
 
 import numpy as np
@@ -66,3 +67,16 @@ def test_round_trip(abi, scenes, backend_mod, bodies, joints, springs):
         for f in F32:
             assert np.array_equal(getattr(got, f), getattr(host, f).astype(np.float32).astype(np.float64)), f
         assert np.array_equal(got.j_broken, host.j_broken) and np.array_equal(got.s_broken, host.s_broken)
+
+
+def test_no_positions_is_refused(abi, scenes, backend_mod):
+    gpu = backend_mod.GpuBackend(abi.default_params())
+    w = world_of(scenes, 5, 2, 1).world()
+    gpu.pack(w)
+    before = gpu.read_state()
+    w.vel[:] = 3.0
+    wc = w.c(with_manifolds=False)
+    wc.bodies.pos = None
+    assert gpu.L.avbd_write_state(gpu.h, ctypes.byref(wc)) == abi.AVBD_ERR_CUDA
+    assert np.array_equal(gpu.read_state().vel, before.vel)
+    gpu.destroy()
