@@ -4,8 +4,8 @@ on sixteen lanes each, longer lists a pair a thread.
 The same pairs - boxes touching within rounding along a face or an edge axis,
 clipped to polygons of three to eight vertices or to a support point,
 separated by a hair, and sphere pairs - are decided once in a short list
-(pair counts that fill a half, both and several warps) and once behind enough
-sphere pairs to make the list long. Every manifold must be bitwise the same,
+(pair counts that fill a half, both and several warps) and once ahead of enough
+touching boxes to make the list long. Every manifold must be bitwise the same,
 and its topology the oracle's.
 """
 import importlib
@@ -34,7 +34,8 @@ def rotation(q):
 
 
 def touching_pairs(scenes, count, filler, seed=11):
-    """`count` pairs around x = 0, 12, 24, ..., then `filler` sphere pairs."""
+    """`count` pairs around x = 0, 12, 24, ..., then `filler` box pairs that
+    touch within rounding (undecided in f32)."""
     s = scenes.Scene("touching")
     s.params = dict(gravity=0.0, iterations=1)
     rng = np.random.default_rng(seed)
@@ -73,8 +74,8 @@ def touching_pairs(scenes, count, filler, seed=11):
         s.box(2 * hb, 100.0, 0.5, at + n * reach + side, quat=tuple(qb))
     for k in range(filler):
         at = (3.0 * (k % 200), 40.0 + 3.0 * (k // 200), 0.0)
-        s.sphere(1.0, 100.0, 0.5, at)
-        s.sphere(1.0, 100.0, 0.5, (at[0] + 0.99, at[1], 0.0))
+        s.box((1.0, 1.0, 1.0), 100.0, 0.5, at)
+        s.box((1.0, 1.0, 1.0), 100.0, 0.5, (at[0] + 1.0 - 1e-8, at[1], 0.0))
     return s
 
 
@@ -93,8 +94,8 @@ def random_pairs(scenes, abi, count, filler, seed=5):
             s.box(rng.uniform(0.1, 2.0, 3), 100.0, 0.5, at + side * rng.normal(0.0, 0.6, 3), quat=tuple(q))
     for k in range(filler):
         at = (3.0 * (k % 200), 40.0 + 3.0 * (k // 200), 0.0)
-        s.sphere(1.0, 100.0, 0.5, at)
-        s.sphere(1.0, 100.0, 0.5, (at[0] + 0.99, at[1], 0.0))
+        s.box((1.0, 1.0, 1.0), 100.0, 0.5, at)
+        s.box((1.0, 1.0, 1.0), 100.0, 0.5, (at[0] + 1.0 - 1e-8, at[1], 0.0))
     return s
 
 
