@@ -945,12 +945,16 @@ __device__ __forceinline__ D3 gshfl(D3 v, int src) {
 __device__ __forceinline__ D3 pick3(bool c, D3 a, D3 b) { return D3{c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z}; }
 
 // The lane of the group with the largest v among those with `on`, the first
-// on ties (-1: none). Compared as integers: a double compare is an FP64 warp
-// instruction. (v + 0 makes -0 equal to +0.)
+// on ties (-1: none), as a loop of `v > best` over them finds it: a NaN that
+// comes first stays, a later one is passed over. Compared as integers: a double
+// compare is an FP64 warp instruction. (v + 0 makes -0 equal to +0.)
 __device__ __forceinline__ int group_argmax(double v, bool on) {
   long long key = __double_as_longlong(v + 0.0);
+  const bool nan = (key & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+  const unsigned mine = 0xffffu << (threadIdx.x & (32 - kGroup));
+  const unsigned all = __ballot_sync(0xffffffffu, on) & mine, nans = __ballot_sync(0xffffffffu, on && nan);
   key ^= (key >> 63) & 0x7fffffffffffffffLL;
-  int at = on ? (int)(threadIdx.x & (kGroup - 1)) : kGroup;
+  int at = on && !nan ? (int)(threadIdx.x & (kGroup - 1)) : kGroup;
 #pragma unroll
   for (int m = kGroup / 2; m > 0; m >>= 1) {
     const long long ok = __shfl_xor_sync(0xffffffffu, key, m, kGroup);
@@ -959,6 +963,8 @@ __device__ __forceinline__ int group_argmax(double v, bool on) {
     key = take ? ok : key;
     at = take ? oa : at;
   }
+  const int first = __ffs(all) - 1;
+  if (first >= 0 && ((nans >> first) & 1u)) return first & (kGroup - 1);
   return at < kGroup ? at : -1;
 }
 
@@ -1173,10 +1179,9 @@ __device__ void write_materials_group(const World &w, int c, int ia, int ib, con
       const double mdSq = dist_sq(gshfl(mid, src), oldMid);
       const uint32_t feat = __shfl_sync(0xffffffffu, own ? nc.feature : 0u, src, kGroup);
       const bool ok = pass && i < num && !((used >> gl) & 1u) && !(mdSq > m.psq);
-      const unsigned okMask = ballot(ok), sameMask = ballot(ok && oldFeat == feat), nanMask = ballot(ok && mdSq != mdSq);
-      const int nearest = group_argmax(-mdSq, ok), first = __ffs(okMask) - 1;
-      int j = sameMask ? __ffs(sameMask) - 1 : nearest;
-      if (!sameMask && okMask && ((nanMask >> first) & 1u)) j = first;  // (nothing is less than NaN)
+      const unsigned sameMask = ballot(ok && oldFeat == feat);
+      const int nearest = group_argmax(-mdSq, ok);
+      const int j = sameMask ? __ffs(sameMask) - 1 : nearest;
       if (j >= 0) used |= 1u << j;
       if (own && slot == i) match = j;
     }
