@@ -781,6 +781,51 @@ __device__ __forceinline__ void push_exact(const World &w, int c) {
   w.g.npExact[push_slot(&w.ctl->npCount[2])] = c;
 }
 
+// Lists of up to kGroupMax box pairs take sixteen lanes a pair, longer ones a
+// pair a thread: that keeps every sub-partition's FP64 pipe busy either way,
+// and then needs about half the warp instructions (narrow phase of a batch with
+// 10,257 such pairs: 0.70 ms on lanes, 0.72 by threads; of a crushed pyramid
+// with 37,825: 1.24 and 0.93).
+// Under the materials model every box pair is in the list, and in a scene at
+// rest nearly all of them touch and take the same path: a warp of 32 pairs
+// then hardly diverges, and threads are ahead from 4,500 pairs (boxes
+// aligned) or 5,900 (turned about the vertical) on. 13,514 aligned pairs: 463 us
+// on lanes, 193 by threads; 7,442 turned ones: 256 and 212. Where the pairs are
+// of several kinds it is the other way round up to kGroupMax (a landing pile's
+// 8,544: 133 us on lanes, 263 by threads; a landed one's 10,903: 334 and 364), so
+// long lists count the pairs that no face separates (2 us).
+constexpr int kGroupMax = 16384, kGroupMaxTouching = 6144;
+__device__ __forceinline__ int pairs_per_warp(int n, int touching) {
+  return n > kGroupMax || (n > kGroupMaxTouching && touching >= n - n / 4) ? 32 : 2;
+}
+
+// Whether no face axis of two boxes separates them by more than the skin, in
+// f32 and as good as that is: only what pairs_per_warp counts.
+__device__ __forceinline__ bool faces_touch(const World &w, int ia, int ib, float skin) {
+  const float4 qa = w.b.quat[ia], qb = w.b.quat[ib];
+  const D4 pa = w.b.pos[ia], pb = w.b.pos[ib], sa = w.b.size[ia], sb = w.b.size[ib];
+  const V3<float> d{(float)(pb.x - pa.x), (float)(pb.y - pa.y), (float)(pb.z - pa.z)};
+  const float ha[3] = {0.5f * (float)sa.x, 0.5f * (float)sa.y, 0.5f * (float)sa.z};
+  const float hb[3] = {0.5f * (float)sb.x, 0.5f * (float)sb.y, 0.5f * (float)sb.z};
+  // B's centre and axes in A's frame
+  const Q4<float> inv{-qa.x, -qa.y, -qa.z, qa.w}, q{qb.x, qb.y, qb.z, qb.w};
+  const V3<float> c = qrotate(inv, d);
+  const V3<float> bx[3] = {qrotate(inv, qrotate(q, V3<float>{1, 0, 0})), qrotate(inv, qrotate(q, V3<float>{0, 1, 0})),
+                           qrotate(inv, qrotate(q, V3<float>{0, 0, 1}))};
+  const float ca[3] = {c.x, c.y, c.z};
+  bool touch = true;
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const float b[3] = {i == 0 ? bx[0].x : i == 1 ? bx[0].y : bx[0].z, i == 0 ? bx[1].x : i == 1 ? bx[1].y : bx[1].z,
+                        i == 0 ? bx[2].x : i == 1 ? bx[2].y : bx[2].z};
+    touch = touch && fabsf(ca[i]) <= ha[i] + hb[0] * fabsf(b[0]) + hb[1] * fabsf(b[1]) + hb[2] * fabsf(b[2]) + skin;
+    const V3<float> n = bx[i];
+    touch = touch && fabsf(c.x * n.x + c.y * n.y + c.z * n.z) <=
+                         hb[i] + ha[0] * fabsf(n.x) + ha[1] * fabsf(n.y) + ha[2] * fabsf(n.z) + skin;
+  }
+  return touch;
+}
+
 // The face axis among `mask` (bits 0-5: faces of A, then of B) with the
 // largest exact separation, the first on ties: the f64 expressions of
 // testAxis (collide.js:291-324) for just those axes.
@@ -846,8 +891,10 @@ __global__ void __launch_bounds__(256) classify_kernel(World w) {
     }
     // pairs with a contact skin (speculative contacts: the f32 certification
     // covers the skin-free tests) go to the exact collider
-    if (pair_skin(w, ia, ib) != 0.0) {
+    const double skin = pair_skin(w, ia, ib);
+    if (skin != 0.0) {
       push_exact(w, c);
+      if (total > kGroupMaxTouching && faces_touch(w, ia, ib, (float)skin)) push_slot(&w.ctl->npTouching);
       continue;
     }
     bool refIsA = true;
@@ -1216,13 +1263,8 @@ __device__ __noinline__ void exact_pair(const World &w, int c) {
 
 // 4. Sphere pairs and undecided box pairs: the whole f64 collider. Sphere pairs
 //    a thread each (a short chain: in halves of warps of their own, as the box
-//    pairs, they made it 113 us for 88 in a pile of 1,777 boxes and spheres). Lists of up to
-//    kGroupMax box pairs on sixteen lanes a pair; longer ones keep every
-//    sub-partition's FP64 pipe busy either way, and a pair a thread then needs
-//    about half the warp instructions (narrow phase of a batch with 10,257 such
-//    pairs: 0.70 ms on lanes, 0.72 by threads; of a crushed pyramid with 37,825:
-//    1.24 and 0.93).
-constexpr int kGroupMax = 16384;
+//    pairs, they made it 113 us for 88 in a pile of 1,777 boxes and spheres), box
+//    pairs on sixteen lanes or a thread each (pairs_per_warp).
 struct GroupShared {
   D3 poly[geo::kPolyCap];
 };
@@ -1271,7 +1313,7 @@ __global__ void __launch_bounds__(128) collide_kernel(const __grid_constant__ Wo
   const int lane = threadIdx.x & 31;
   const int nFace = w.ctl->npCount[0], nEdge = w.ctl->npCount[1], nExact = w.ctl->npCount[2];
   const int nSphere = w.ctl->npCount[4];
-  const int per = nExact > kGroupMax ? 32 : 2;
+  const int per = pairs_per_warp(nExact, w.ctl->npTouching);
   const int uExact = (nExact + per - 1) / per, uFace = (nFace + 31) / 32, uEdge = (nEdge + 31) / 32;
   const int uSphere = (nSphere + 31) / 32, units = uExact + uFace + uSphere + uEdge, warps = gridDim.x * (blockDim.x >> 5);
   const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -1315,7 +1357,7 @@ __global__ void __launch_bounds__(128) late_kernel(const __grid_constant__ World
   const int total = w.ctl->npCount[3], lane = threadIdx.x & 31;
   const int *last = w.g.npExact + w.g.candCap - 1;
   const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (blockDim.x >> 5);
-  const int per = total > kGroupMax ? 32 : 2;
+  const int per = pairs_per_warp(total, 0);
   for (int u = warp; u * per < total; u += warps) {
     if (per == 2) {
       const int t = u * 2 + lane / kGroup;
