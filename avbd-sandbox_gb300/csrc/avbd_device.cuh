@@ -97,7 +97,7 @@ struct Control {
   int gridEntries;  // grid entries handed out this step
   unsigned colorArrivals;  // arrivals at the colouring's grid barrier this step
   int npCount[5];      // narrow-phase work lists: face, edge, exact, late (face pairs that need the exact collider), sphere
-  int npTouching;      // exact list's pairs with a contact skin that no face separates (counted in long lists)
+  int npApart;         // exact list's pairs with a contact skin that a face separates (counted in long lists)
   int npNext;          // the next unit of the lists
   int prevCandidates;  // candidates (= manifold slots) of the previous step
   int colorBad;        // this step's uploaded colouring has a conflict

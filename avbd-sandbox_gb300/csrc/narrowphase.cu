@@ -786,17 +786,21 @@ __device__ __forceinline__ void push_exact(const World &w, int c) {
 // and then needs about half the warp instructions (narrow phase of a batch with
 // 10,257 such pairs: 0.70 ms on lanes, 0.72 by threads; of a crushed pyramid
 // with 37,825: 1.24 and 0.93).
-// Under the materials model every box pair is in the list, and in a scene at
-// rest nearly all of them touch and take the same path: a warp of 32 pairs
-// then hardly diverges, and threads are ahead from 4,500 pairs (boxes
-// aligned) or 5,900 (turned about the vertical) on. 13,514 aligned pairs: 463 us
-// on lanes, 193 by threads; 7,442 turned ones: 256 and 212. Where the pairs are
-// of several kinds it is the other way round up to kGroupMax (a landing pile's
-// 8,544: 133 us on lanes, 263 by threads; a landed one's 10,903: 334 and 364), so
-// long lists count the pairs that no face separates (2 us).
-constexpr int kGroupMax = 16384, kGroupMaxTouching = 6144;
-__device__ __forceinline__ int pairs_per_warp(int n, int touching) {
-  return n > kGroupMax || (n > kGroupMaxTouching && touching >= n - n / 4) ? 32 : 2;
+// In a scene at rest nearly all pairs touch, and take the same path: every box
+// pair is in the list under the materials model, and boxes aligned with one
+// another are undecided under both. A warp of 32 pairs then hardly diverges,
+// and threads are ahead from some 6,000 pairs on (materials: 4,500, 5,900 with
+// the boxes turned about the vertical). 13,514 aligned pairs, materials: 463 us on
+// lanes, 193 by threads; 12,706, plain: 247 and 142. Where the pairs are of
+// several kinds it is the other way round up to kGroupMax (materials, a landing
+// pile's 8,544: 133 us on lanes, 263 by threads; plain, a crushed pyramid's 7,649:
+// 300 and 606). So the line is kGroupMaxAlike when the box pairs that stand
+// `apart` are at most a third as many as the list: those decided without it, and
+// those in it (pairs with a skin) that a face separates, which long lists count
+// (2 us).
+constexpr int kGroupMax = 16384, kGroupMaxAlike = 6144;
+__device__ __forceinline__ int pairs_per_warp(int n, int apart) {
+  return n > kGroupMax || (n > kGroupMaxAlike && apart <= n / 3) ? 32 : 2;
 }
 
 // Whether no face axis of two boxes separates them by more than the skin, in
@@ -894,7 +898,7 @@ __global__ void __launch_bounds__(256) classify_kernel(World w) {
     const double skin = pair_skin(w, ia, ib);
     if (skin != 0.0) {
       push_exact(w, c);
-      if (total > kGroupMaxTouching && faces_touch(w, ia, ib, (float)skin)) push_slot(&w.ctl->npTouching);
+      if (total > kGroupMaxAlike && !faces_touch(w, ia, ib, (float)skin)) push_slot(&w.ctl->npApart);
       continue;
     }
     bool refIsA = true;
@@ -1313,7 +1317,7 @@ __global__ void __launch_bounds__(128) collide_kernel(const __grid_constant__ Wo
   const int lane = threadIdx.x & 31;
   const int nFace = w.ctl->npCount[0], nEdge = w.ctl->npCount[1], nExact = w.ctl->npCount[2];
   const int nSphere = w.ctl->npCount[4];
-  const int per = pairs_per_warp(nExact, w.ctl->npTouching);
+  const int per = pairs_per_warp(nExact, w.ctl->numCandidates - nSphere - nExact + w.ctl->npApart);
   const int uExact = (nExact + per - 1) / per, uFace = (nFace + 31) / 32, uEdge = (nEdge + 31) / 32;
   const int uSphere = (nSphere + 31) / 32, units = uExact + uFace + uSphere + uEdge, warps = gridDim.x * (blockDim.x >> 5);
   const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -1357,7 +1361,7 @@ __global__ void __launch_bounds__(128) late_kernel(const __grid_constant__ World
   const int total = w.ctl->npCount[3], lane = threadIdx.x & 31;
   const int *last = w.g.npExact + w.g.candCap - 1;
   const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (blockDim.x >> 5);
-  const int per = pairs_per_warp(total, 0);
+  const int per = total > kGroupMax ? 32 : 2;
   for (int u = warp; u * per < total; u += warps) {
     if (per == 2) {
       const int t = u * 2 + lane / kGroup;
