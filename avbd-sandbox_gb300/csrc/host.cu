@@ -1320,25 +1320,32 @@ int avbd_read_state(avbd_ctx *ctx, avbd_world *out) {
   cudaStream_t st = ctx->stream;
   avbd_joint_soa &J = out->joints;
   avbd_spring_soa &SP = out->springs;
-  auto joints_out = [&](const float4 *kl, const float4 *ka, const D4 *ll, const D4 *la, const int *js) {
-    for (int j = 0; j < ctx->nj; j++) {
-      const float kv[6] = {kl[j].x, kl[j].y, kl[j].z, ka[j].x, ka[j].y, ka[j].z};
-      const double lv[6] = {ll[j].x, ll[j].y, ll[j].z, la[j].x, la[j].y, la[j].z};
-      for (int k = 0; k < 3; k++) {
-        if (J.penalty_lin) J.penalty_lin[j * 3 + k] = kv[k];
-        if (J.penalty_ang) J.penalty_ang[j * 3 + k] = kv[3 + k];
-        if (J.lambda_lin) J.lambda_lin[j * 3 + k] = lv[k];
-        if (J.lambda_ang) J.lambda_ang[j * 3 + k] = lv[3 + k];
-      }
-      if (J.broken) J.broken[j] = (js[j] & kBroken) ? 1 : 0;
+  // an array after the other (a read of 10,000 joints 216 us with all of a
+  // joint's values at a time, 189 so; 2,000 in the pinned copy 62 and 56)
+  auto rows_out = [](double *o, const auto *v, int count) {
+    if (!o) return;
+    for (int j = 0; j < count; j++) {
+      o[j * 3] = v[j].x;
+      o[j * 3 + 1] = v[j].y;
+      o[j * 3 + 2] = v[j].z;
     }
   };
+  auto broken_out = [](int32_t *o, const int *state, int count) {
+    if (!o) return;
+    for (int j = 0; j < count; j++) o[j] = (state[j] & kBroken) ? 1 : 0;
+  };
+  auto joints_out = [&](const float4 *kl, const float4 *ka, const D4 *ll, const D4 *la, const int *js) {
+    rows_out(J.penalty_lin, kl, ctx->nj);
+    rows_out(J.penalty_ang, ka, ctx->nj);
+    rows_out(J.lambda_lin, ll, ctx->nj);
+    rows_out(J.lambda_ang, la, ctx->nj);
+    broken_out(J.broken, js, ctx->nj);
+  };
   auto springs_out = [&](const float *pen, const double *peak, const int *ss) {
-    for (int s = 0; s < ctx->ns; s++) {
-      if (SP.penalty) SP.penalty[s] = pen[s];
-      if (SP.peak_strain) SP.peak_strain[s] = peak[s];
-      if (SP.broken) SP.broken[s] = (ss[s] & kBroken) ? 1 : 0;
-    }
+    if (SP.penalty)
+      for (int s = 0; s < ctx->ns; s++) SP.penalty[s] = pen[s];
+    if (SP.peak_strain) std::memcpy(SP.peak_strain, peak, ctx->ns * sizeof(double));
+    broken_out(SP.broken, ss, ctx->ns);
   };
   if (ctx->small.d64) {
     // queued behind the steps, so that one wait covers both; steps skipped for
