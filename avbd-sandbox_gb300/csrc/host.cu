@@ -1042,7 +1042,7 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
   std::vector<int2> jb(ctx->nj), sb(ctx->ns);
   std::vector<D4> jrA(ctx->nj), jrB(ctx->nj), jst(ctx->nj), srA(ctx->ns), srB(ctx->ns), sprm(ctx->ns);
   std::vector<float4> jrAf(ctx->nj), jrBf(ctx->nj), srAf(ctx->ns), srBf(ctx->ns);
-  std::vector<std::vector<std::pair<uint32_t, int>>> refs(n);  // reference, the other body
+  std::vector<int> cStart(n + 1, 0);  // the bodies' counts first, at cStart[i + 1]
   std::vector<float4> jstF(ctx->nj);
   for (int j = 0; j < ctx->nj; j++) {
     const int a = J.body_a[j], b = J.body_b[j];
@@ -1059,8 +1059,8 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
     const double sz = (a >= 0 ? B.size[a * 3 + 2] : 0) + B.size[b * 3 + 2];
     jst[j] = mkd4(J.stiffness_lin[j], J.stiffness_ang[j], J.fracture[j], sx * sx + sy * sy + sz * sz);
     jstF[j] = make_float4(std::isinf(jst[j].x) ? 1.f : 0.f, std::isinf(jst[j].y) ? 1.f : 0.f, (float)jst[j].w, 0.f);
-    if (a >= 0) refs[a].push_back({make_ref(kRefJoint, j, 0), b});
-    refs[b].push_back({make_ref(kRefJoint, j, 1), a});
+    if (a >= 0) cStart[a + 1]++;
+    cStart[b + 1]++;
   }
   for (int s = 0; s < ctx->ns; s++) {
     const int a = SP.body_a[s], b = SP.body_b[s];
@@ -1073,20 +1073,25 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
     srAf[s] = make_float4((float)srA[s].x, (float)srA[s].y, (float)srA[s].z, 0);
     srBf[s] = make_float4((float)srB[s].x, (float)srB[s].y, (float)srB[s].z, 0);
     sprm[s] = mkd4(SP.stiffness[s], SP.rest[s], SP.tear_strain ? SP.tear_strain[s] : INFINITY, 0);
-    refs[a].push_back({make_ref(kRefSpring, s, 0), b});
-    refs[b].push_back({make_ref(kRefSpring, s, 1), a});
+    cStart[a + 1]++;
+    cStart[b + 1]++;
   }
-  std::vector<int> cStart(n + 1, 0);
-  std::vector<uint32_t> cRef;
-  std::vector<int> cOther;
-  for (int i = 0; i < n; i++) {
-    cStart[i] = (int)cRef.size();
-    for (const auto &r : refs[i]) {
-      cRef.push_back(r.first);
-      cOther.push_back(r.second < 0 ? -1 : r.second);
+  // each body's references (joints, then springs, in their order) and the other
+  // bodies, counted and then placed (a list per body made a pack of 100 x 100
+  // bonded bricks 0.7 ms longer)
+  for (int i = 0; i < n; i++) cStart[i + 1] += cStart[i];
+  std::vector<uint32_t> cRef(cStart[n]);
+  std::vector<int> cOther(cStart[n]), cAt(cStart.begin(), cStart.end() - 1);
+  auto place = [&](uint32_t type, int k, int a, int b) {
+    for (int side = 0; side < 2; side++) {
+      const int self = side ? b : a;
+      if (self < 0) continue;
+      cRef[cAt[self]] = make_ref(type, k, side);
+      cOther[cAt[self]++] = std::max(side ? a : b, -1);
     }
-  }
-  cStart[n] = (int)cRef.size();
+  };
+  for (int j = 0; j < ctx->nj; j++) place(kRefJoint, j, jb[j].x, jb[j].y);
+  for (int s = 0; s < ctx->ns; s++) place(kRefSpring, s, sb[s].x, sb[s].y);
 
   // capacities: one grid insertion per regular body
   long long insertions = 0;
