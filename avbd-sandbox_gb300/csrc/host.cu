@@ -769,6 +769,7 @@ std::vector<std::pair<void *, size_t>> mutable_regions(avbd_ctx *ctx, int keep) 
       {pm.basis2, m * sizeof(float4)}, {pm.basisD, m * 9 * sizeof(double)}, {pm.feat, m * K * sizeof(uint32_t)},
       {pm.rA, m * K * sizeof(float4)}, {pm.rB, m * K * sizeof(float4)}, {pm.cA, m * K * sizeof(float4)},
       {pm.cB, m * K * sizeof(float4)}, {pm.cK, m * K * sizeof(float4)}, {pm.cL, m * K * sizeof(float4)},
+      {pm.cX, m * K * sizeof(float)},
       {w.ctl, sizeof(Control)}};
   return r;
 }
