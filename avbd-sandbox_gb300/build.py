@@ -18,20 +18,14 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libavbd_gb300.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-# object: source, flags
 UNITS = {
-    "narrowphase": ("narrowphase.cu", ["--fmad=false"]),
-    "broadphase": ("broadphase.cu", ["--fmad=false"]),
-    "solver": ("solver.cu", []),
-    "host": ("host.cu", []),
-    "tangent": ("tangent.cu", ["--fmad=false"]),
-    "repack": ("repack.cu", []),
+    "narrowphase.cu": ["--fmad=false"],
+    "broadphase.cu": ["--fmad=false"],
+    "solver.cu": [],
+    "host.cu": [],
+    "tangent.cu": ["--fmad=false"],
+    "repack.cu": [],
 }
-# the solve's instances: contact extensions, joints and springs, FP64 bodies
-for _name, _has in {"solve_plain": (0, 0, 0), "solve_forces": (0, 1, 0), "solve_forces_fp64": (0, 1, 1),
-                    "solve_materials": (1, 0, 0), "solve_materials_forces": (1, 1, 0),
-                    "solve_materials_forces_fp64": (1, 1, 1)}.items():
-    UNITS[_name] = ("solve.cu", [f"-DSOLVE_INSTANCE={_name}"] + [f"-DSOLVE_{k}={v}" for k, v in zip(("E", "J", "F64"), _has)])
 
 
 def nvcc():
@@ -50,13 +44,13 @@ def _stale(out, deps):
 
 def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
-    headers = [os.path.join(CSRC, h) for h in ("avbd_device.cuh", "collider.cuh", "dual.cuh", "solve.cuh")]
+    headers = [os.path.join(CSRC, h) for h in ("avbd_device.cuh", "collider.cuh", "dual.cuh")]
     headers.append(os.path.join(HERE, "..", "include", "avbd_cuda.h"))
     objs = []
     jobs = []
-    for unit, (source, extra) in UNITS.items():
-        src = os.path.join(CSRC, source)
-        obj = os.path.join(BUILD, unit + ".o")
+    for unit, extra in UNITS.items():
+        src = os.path.join(CSRC, unit)
+        obj = os.path.join(BUILD, unit.replace(".cu", ".o"))
         objs.append(obj)
         if force or _stale(obj, [src] + headers):
             cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-rdc=false",
