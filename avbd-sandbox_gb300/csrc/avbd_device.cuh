@@ -451,7 +451,7 @@ void launch_prepare(const World &w, cudaStream_t st, int smCount);
 cudaError_t launch_coloring(const World &w, cudaStream_t st, int blocks);
 int coloring_grid(int n, int smCount);  // blocks of the cooperative colouring launch
 cudaError_t launch_solve(const World &w, int lanesPerBody, int blocksPerSm, cudaStream_t st, int smCount);
-int solve_max_blocks_per_sm(int lanesPerBody);
+int solve_max_blocks_per_sm(const World &w);
 void launch_commit(const World &w, cudaStream_t st, int smCount);
 void launch_stats(const World &w, double *out3, cudaStream_t st, int smCount);
 cudaError_t launch_joint_anchor(const World &w, int joint, double x, double y, double z, cudaStream_t st);

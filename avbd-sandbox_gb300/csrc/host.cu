@@ -1262,7 +1262,7 @@ int avbd_pack(avbd_ctx *ctx, const avbd_world *world) {
     return rc;
   CK(launch_set_grab(w, -1, nullptr, nullptr, 0.0, ctx->stream));  // nothing grabbed
   // launch shape of the persistent solve
-  const int maxPerSm = solve_max_blocks_per_sm(ctx->lanes);
+  const int maxPerSm = solve_max_blocks_per_sm(w);
   ctx->autoLanes = P.lanes_per_body <= 0;
   ctx->lanes = P.lanes_per_body > 0 ? P.lanes_per_body : 32;
   ctx->nDyn = 0;

@@ -2773,11 +2773,16 @@ static const void *solve_instance(bool wave, bool ext, bool joints, bool fp64) {
                                                                  : solve_instance<false, false, false>(wave);
 }
 
-int solve_max_blocks_per_sm(int lanesPerBody) {
-  (void)lanesPerBody;
+static const void *solve_instance(const World &w, bool wave) {
+  return solve_instance(wave, w.p.contactModel != 0, w.g.hasConstraints != 0, w.p.mayFp64 != 0);
+}
+
+// Of the two kernels that this world's steps can launch (either schedule): each
+// is loaded when it is first asked about (0.05 ms each).
+int solve_max_blocks_per_sm(const World &w) {
   int best = 1 << 30;
-  for (int k = 0; k < 12; k++) {
-    const void *f = solve_instance(k & 1, k & 2, k / 4 >= 1, k / 4 == 2);
+  for (int wave = 0; wave < 2; wave++) {
+    const void *f = solve_instance(w, wave != 0);
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem);
     int a = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f, kSolveBlock, kSolveSmem);
