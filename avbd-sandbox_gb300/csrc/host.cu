@@ -332,7 +332,8 @@ __global__ void state_check_kernel(const double *pos, int n, int *bad) {
 // some 8 us each. Write / read in us, with the copies and with the kernel:
 // 64 bodies 35 / 53 and 17 / 12, with 63 joints 73 / 101 and 20 / 14; 2,048
 // bodies 50 / 58 and 28 / 32; 4,096 bodies 76 / 57 and 46 / 54; 8,192 bodies
-// 80 / 61 and 82 / 104, more than one block should move.
+// 80 / 61 and 82 / 104. The line lies below the crossing, which is past 4,096
+// bodies and was not measured with joints or springs.
 constexpr int kSmallBodies = 2048;
 
 size_t small_state_bytes(size_t n, size_t nj, size_t ns) {
@@ -628,8 +629,8 @@ int enqueue_step(avbd_ctx *ctx) {
 }
 
 // Own kernels of one step: broad phase 6 (+1 with large bodies), narrow phase
-// 4, prepare 5 (+1 with joints or springs), colouring 1 (+2 with an
-// uploaded colouring), solve 1, commit 1.
+// 3, prepare 5, or 3 below kAdjAlone bodies (+1 with joints or springs),
+// colouring 1 (+2 with an uploaded colouring), solve 1, commit 1.
 int step_kernels(const avbd_ctx *ctx) {
   const int broad = 6 + (ctx->numLarge > 0 ? 1 : 0);
   const int prepare = (ctx->n < kAdjAlone ? 3 : 5) + (ctx->nj + ctx->ns > 0 ? 1 : 0);

@@ -1,10 +1,11 @@
 // narrowphase.cu - contact generation, manifold merge and warm start.
 //
-// One thread per candidate pair. The geometry runs in IEEE f64 with the
-// reference's operation order and NO fused multiply-add (this translation
-// unit is compiled with --fmad=false), so that from identical inputs the
-// contact count, feature IDs and SAT/clipping decisions equal the reference
-// engine's bit for bit:
+// One thread per candidate pair; box pairs that the f32 test below leaves
+// undecided take sixteen lanes each in lists that are not too long
+// (pairs_per_warp). The geometry runs in IEEE f64 with the reference's operation
+// order and NO fused multiply-add (this translation unit is compiled with
+// --fmad=false), so that from identical inputs the contact count, feature IDs
+// and SAT/clipping decisions equal the reference engine's bit for bit:
 //   collide.js:612-685 box-box 15-axis SAT, face clipping (:403-472),
 //                      edge contact (:475-493)
 //   collide.js:496-520 sphere-sphere, :526-600 sphere-OBB

@@ -1342,8 +1342,9 @@ __device__ __forceinline__ int round_up_groups(int g) { return (g + kGroupsPerWa
 
 // Force e of the body whose list starts at e0, from shared memory when the
 // block has read it there (force by force from memory, the walk took ~4 us of
-// a phase; with the one-word grid barrier, six steps of 16 x 16 bonded bricks
-// 30.4 -> 30.0 ms).
+// a phase of ~75; the time of a call did not change measurably with it and the
+// one-word grid barrier: six steps of 16 x 16 bonded bricks 30.8 and 30.3 ms,
+// where runs of one side differ by 2.7 %).
 __device__ __forceinline__ uint32_t force_ref(const TWorld &w, const BodySmem &sm, int e0, int e) {
   return e - e0 < kWalk ? sm.ref[e - e0] : w.fRef[e];
 }
